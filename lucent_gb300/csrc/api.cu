@@ -3,6 +3,7 @@
 #include <cstring>
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -34,13 +35,91 @@ lucent_status cuda_fail(cudaError_t e, const char* what) {
   return fail(LUCENT_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// The pool of the current device for the memory of single calls and of BVH
+// handles: cudaMalloc and cudaFree of a build's buffers cost as much as a small
+// build (the last cudaFree of a 2 MiB block alone some 180 us). Stream-ordered,
+// so threads and streams share it safely; it holds at most 1 GiB between calls
+// (the driver takes back what is free beyond that), and gives what is free
+// back when an ordinary allocation fails or a renderer is trimmed. `stream`:
+// the pool's own, for allocations that outlive a call.
+struct Pool {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;
+};
+static Pool device_pool() {
+  static std::mutex lock;
+  static Pool pools[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return {};
+  std::lock_guard<std::mutex> hold(lock);
+  Pool& P = pools[dev];
+  if (!P.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    Pool made;
+    if (cudaStreamCreateWithFlags(&made.stream, cudaStreamNonBlocking) != cudaSuccess) return {};
+    if (cudaMemPoolCreate(&made.pool, &props) != cudaSuccess) {
+      cudaStreamDestroy(made.stream);
+      return {};
+    }
+    uint64_t keep = 1ull << 30;
+    cudaMemPoolSetAttribute(made.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    P = made;
+  }
+  return P;
+}
+
+void trim_temporaries() {
+  if (cudaMemPool_t p = device_pool().pool) cudaMemPoolTrimTo(p, 0);
+}
+
+static lucent_status pool_alloc(void** ptr, size_t bytes, const Pool& P, cudaStream_t s) {
+  *ptr = nullptr;
+  if (!P.pool) return cuda_fail(cudaGetLastError(), "memory pool");
+  cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, P.pool, s);
+  if (e == cudaErrorMemoryAllocation) {  // once more without what the pool holds
+    cudaGetLastError();
+    trim_temporaries();
+    e = cudaMallocFromPoolAsync(ptr, bytes, P.pool, s);
+  }
+  if (e == cudaSuccess) return LUCENT_OK;
+  *ptr = nullptr;
+  return cuda_fail(e, "cudaMallocFromPoolAsync");
+}
+
+lucent_status TempBuffer::reserve(size_t bytes, cudaStream_t s) {
+  release();
+  stream = s;
+  return pool_alloc(&ptr, bytes < 256 ? 256 : bytes, device_pool(), s);
+}
+
+void TempBuffer::release() {
+  if (ptr) cudaFreeAsync(ptr, stream);
+  ptr = nullptr;
+}
+
 lucent_status DeviceBuffer::reserve(size_t bytes) {
   if (bytes <= cap) return LUCENT_OK;
-  if (ptr) cudaFree(ptr);
-  ptr = nullptr;
-  cap = 0;
-  size_t want = bytes < 256 ? 256 : bytes;
+  release();
+  const size_t want = bytes < 256 ? 256 : bytes;
+  if (pooled) {  // allocated on the pool's stream and waited for: usable on any stream
+    const Pool P = device_pool();
+    if (lucent_status st = pool_alloc(&ptr, want, P, P.stream)) return st;
+    if (cudaError_t e = cudaStreamSynchronize(P.stream); e != cudaSuccess) {
+      ptr = nullptr;
+      return cuda_fail(e, "pool allocation");
+    }
+    cap = want;
+    return LUCENT_OK;
+  }
   cudaError_t e = cudaMalloc(&ptr, want);
+  if (e == cudaErrorMemoryAllocation) {  // once more without what the pool holds
+    cudaGetLastError();
+    trim_temporaries();
+    e = cudaMalloc(&ptr, want);
+  }
   if (e != cudaSuccess) {
     ptr = nullptr;
     return cuda_fail(e, "cudaMalloc");
@@ -50,7 +129,12 @@ lucent_status DeviceBuffer::reserve(size_t bytes) {
 }
 
 void DeviceBuffer::release() {
-  if (ptr) cudaFree(ptr);
+  if (ptr && pooled) {
+    cudaDeviceSynchronize();  // as cudaFree does: no stream still uses it
+    if (const Pool P = device_pool(); P.stream) cudaFreeAsync(ptr, P.stream);
+  } else if (ptr) {
+    cudaFree(ptr);
+  }
   ptr = nullptr;
   cap = 0;
 }
@@ -63,7 +147,7 @@ struct lucent_bvh {
   // 64-entry stack take the all-binary64 path, which reproduces the overflow.
   uint32_t depth = 0;
   int mode = LUCENT_TRAVERSE_WIDE;
-  DeviceBuffer nodes, tris, scratch, stage;
+  DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch, stage;
   DeviceBuffer wide;  // four-wide view of `nodes` (LUCENT_TRAVERSE_WIDE), built on first use
 };
 
@@ -198,8 +282,8 @@ lucent_status lucent_bvh_build(const float* positions, uint64_t n_floats, const 
   for (uint64_t i = 0; i < n_floats; i++)
     if (!std::isfinite(positions[i])) return fail(LUCENT_ERR_UNSUPPORTED, "positions[%llu] is not finite", (unsigned long long)i);
   cudaStream_t s = (cudaStream_t)stream;
-  DeviceBuffer pos;
-  lucent_status st = pos.reserve(n_floats * 4 + 4);
+  TempBuffer pos;
+  lucent_status st = pos.reserve(n_floats * 4 + 4, s);
   if (st) return st;
   cudaError_t e = cudaMemcpyAsync(pos.ptr, positions, n_floats * 4, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) {

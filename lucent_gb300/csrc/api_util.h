@@ -15,9 +15,20 @@ void clear_error();
 struct DeviceBuffer {
   void* ptr = nullptr;
   size_t cap = 0;
+  bool pooled = false;  // from the pool (TempBuffer) instead of cudaMalloc
   lucent_status reserve(size_t bytes);
   void release();
 };
+
+// Device memory of one call, from a stream-ordered pool that keeps what is
+// freed for the next: released on the stream it was reserved on.
+struct TempBuffer {
+  void* ptr = nullptr;
+  cudaStream_t stream = nullptr;
+  lucent_status reserve(size_t bytes, cudaStream_t s);
+  void release();
+};
+void trim_temporaries();  // gives the pool's free memory back
 
 }  // namespace lucent
 

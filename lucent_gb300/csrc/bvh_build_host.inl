@@ -34,14 +34,12 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
 
   const uint32_t small_max = 2048;
   const uint32_t cap = n;
-  // Scratch: prim bounds, orders, partition positions, node records, lists.
-  DeviceBuffer b_lo, b_hi, b_cz, b_tri, b_tmp, b_P, b_Q, b_recs, b_ctr, b_small, b_bigA, b_bigB, b_info, b_chunks,
-      b_first, b_part, b_bins, b_cnt;
-  auto release_all = [&]() {
-    for (DeviceBuffer* b : {&b_lo, &b_hi, &b_cz, &b_tri, &b_tmp, &b_P, &b_Q, &b_recs, &b_ctr, &b_small, &b_bigA,
-                            &b_bigB, &b_info, &b_chunks, &b_first, &b_part, &b_bins, &b_cnt})
-      b->release();
-  };
+  // Scratch, one allocation: prim bounds, orders, partition positions, node
+  // records, lists, and the big-node levels' chunks and partial results (at
+  // most n / 2049 big nodes of a chunk per 4096 triangles and a ragged one).
+  const uint32_t big_cap = n / (small_max + 1) + 1, chunk_cap = n / kChunk + big_cap;
+  TempBuffer scratch;
+  auto release_all = [&]() { scratch.release(); };
   lucent_status st = LUCENT_OK;
 #define BB_TRY(x)      \
   do {                 \
@@ -60,18 +58,28 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     }                                         \
   } while (0)
   const uint32_t nrec = 2 * n - 1;
-  BB_TRY(b_lo.reserve((size_t)n * 16));
-  BB_TRY(b_hi.reserve((size_t)n * 16));
-  BB_TRY(b_cz.reserve((size_t)n * 4));
-  BB_TRY(b_tri.reserve((size_t)n * 4));
-  BB_TRY(b_tmp.reserve((size_t)n * 4));
-  BB_TRY(b_P.reserve((size_t)n * 4));
-  BB_TRY(b_Q.reserve((size_t)n * 4));
-  BB_TRY(b_recs.reserve((size_t)nrec * sizeof(NodeRec)));
-  BB_TRY(b_ctr.reserve(64));
-  BB_TRY(b_small.reserve((size_t)cap * sizeof(Task)));
-  BB_TRY(b_bigA.reserve((size_t)cap * sizeof(Task)));
-  BB_TRY(b_bigB.reserve((size_t)cap * sizeof(Task)));
+  struct Part {
+    size_t bytes;
+    void* ptr;
+  };
+  Part b_lo{(size_t)n * 16}, b_hi{(size_t)n * 16}, b_cz{(size_t)n * 4}, b_tri{(size_t)n * 4}, b_tmp{(size_t)n * 4},
+      b_P{(size_t)n * 4}, b_Q{(size_t)n * 4}, b_recs{(size_t)nrec * sizeof(NodeRec)}, b_ctr{64},
+      b_small{(size_t)cap * sizeof(Task)}, b_bigA{(size_t)cap * sizeof(Task)}, b_bigB{(size_t)cap * sizeof(Task)},
+      b_info{(size_t)big_cap * sizeof(BigInfo)}, b_chunks{(size_t)chunk_cap * sizeof(Chunk)},
+      b_first{((size_t)big_cap + 1) * 4}, b_part{(size_t)chunk_cap * 12 * 4},
+      b_bins{(size_t)chunk_cap * 3 * bins * 7 * 4}, b_cnt{(size_t)chunk_cap * 2 * 4};
+  {
+    Part* all[] = {&b_lo, &b_hi, &b_cz, &b_tri, &b_tmp, &b_P, &b_Q, &b_recs, &b_ctr, &b_small, &b_bigA,
+                   &b_bigB, &b_info, &b_chunks, &b_first, &b_part, &b_bins, &b_cnt};
+    size_t total = 0;
+    for (Part* p : all) total += (p->bytes + 255) & ~(size_t)255;
+    BB_TRY(scratch.reserve(total, s));
+    char* at = (char*)scratch.ptr;
+    for (Part* p : all) {
+      p->ptr = at;
+      at += (p->bytes + 255) & ~(size_t)255;
+    }
+  }
 
   uint32_t* ctr = (uint32_t*)b_ctr.ptr;  // [0] rec_count [1] small_count [2] big_next_count [3] err
   Ctx cx;
@@ -127,12 +135,10 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     }
     first_h[nbig] = (uint32_t)chunks_h.size();
     const uint32_t nch = (uint32_t)chunks_h.size();
-    BB_TRY(b_chunks.reserve(nch * sizeof(Chunk)));
-    BB_TRY(b_first.reserve((nbig + 1) * 4));
-    BB_TRY(b_part.reserve((size_t)nch * 12 * 4));
-    BB_TRY(b_bins.reserve((size_t)nch * 3 * bins * 7 * 4));
-    BB_TRY(b_cnt.reserve((size_t)nch * 2 * 4));
-    BB_TRY(b_info.reserve((size_t)nbig * sizeof(BigInfo)));
+    if (nbig > big_cap || nch > chunk_cap) {
+      release_all();
+      return fail(LUCENT_ERR_DEVICE, "task list overflow");
+    }
     BB_CUDA(cudaMemcpyAsync(b_chunks.ptr, chunks_h.data(), nch * sizeof(Chunk), cudaMemcpyHostToDevice, s), "chunks");
     BB_CUDA(cudaMemcpyAsync(b_first.ptr, first_h.data(), (nbig + 1) * 4, cudaMemcpyHostToDevice, s), "chunk index");
     BB_CUDA(cudaMemsetAsync(cx.big_next_count, 0, 4, s), "reset next");
@@ -242,8 +248,8 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     bounds[3 + k] = recs[0].hi[k];
   }
   if (nodes_dev || tris_dev) {
-    DeviceBuffer ref;
-    BB_TRY(ref.reserve((size_t)nr * 32));
+    TempBuffer ref;
+    BB_TRY(ref.reserve((size_t)nr * 32, s));
     cudaError_t e = cudaMemcpyAsync(ref.ptr, nodes_ref.data(), (size_t)nr * 32, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && nodes_dev) {
       st = nodes_dev->reserve((size_t)nr * sizeof(Node));

@@ -1184,6 +1184,7 @@ lucent_status lucent_renderer_trim(lucent_renderer* r) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return cuda_fail(e, "synchronize");
   for (WaveSet& w : r->set) w.release_paths();
+  trim_temporaries();
   return LUCENT_OK;
 }
 
