@@ -148,8 +148,18 @@ struct lucent_bvh {
   uint32_t depth = 0;
   int mode = LUCENT_TRAVERSE_WIDE;
   DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch, stage;
-  DeviceBuffer wide;  // four-wide view of `nodes` (LUCENT_TRAVERSE_WIDE), built on first use
+  float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // the root's box
+  NearTree near;       // nearest-first view (LUCENT_TRAVERSE_WIDE, where usable), built on first use
+  bool near_tried = false;
+  DeviceBuffer wide{nullptr, 0, true};  // four-wide view of `nodes` (LUCENT_TRAVERSE_WIDE otherwise), built on first use
 };
+
+static void set_root(lucent_bvh* b, const float* nodes) {
+  for (int k = 0; k < 3; k++) {
+    b->lo[k] = nodes[k];
+    b->hi[k] = nodes[4 + k];
+  }
+}
 
 extern "C" {
 
@@ -235,6 +245,7 @@ lucent_status lucent_bvh_create(const float* nodes, uint32_t node_count, const u
   e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cleanup(cuda_fail(e, "bvh upload kernels"));
+  set_root(b, nodes);
   cleanup(LUCENT_OK);
   *out = b;
   return LUCENT_OK;
@@ -264,6 +275,7 @@ static lucent_status build_common(const float* pos_d, uint32_t n, const lucent_b
     b->node_count = nc;
     b->tri_count = n;
     b->depth = tree_depth(nodes.data(), nc, n);
+    set_root(b, nodes.data());
     *handle_out = b;
   }
   return LUCENT_OK;
@@ -312,6 +324,8 @@ void lucent_bvh_destroy(lucent_bvh* b) {
   b->tris.release();
   b->scratch.release();
   b->stage.release();
+  b->wide.release();
+  b->near.release();
   delete b;
 }
 
@@ -354,17 +368,14 @@ static lucent_status check_tmin(double t_min, double t_max) {
   return LUCENT_OK;
 }
 
-// Scratch layout: [err word][queue length][work counter][pad..][queue: n u32]
-static lucent_status prepare_scratch(lucent_bvh* b, uint32_t n, cudaStream_t s, unsigned** err, uint32_t** qlen,
-                                     uint32_t** queue, uint32_t** work = nullptr) {
-  lucent_status st = b->scratch.reserve(256 + (size_t)n * 4);
+// Scratch layout: 8 counter words (launch_closest; the first is the error
+// word), then 2 n words of ray queues from byte 256.
+static lucent_status prepare_scratch(lucent_bvh* b, uint32_t n, cudaStream_t s, uint32_t** ctr, uint32_t** queue) {
+  lucent_status st = b->scratch.reserve(256 + (size_t)n * 8);
   if (st) return st;
-  char* base = (char*)b->scratch.ptr;
-  *err = (unsigned*)base;
-  *qlen = (uint32_t*)(base + 4);
-  if (work) *work = (uint32_t*)(base + 8);
-  *queue = (uint32_t*)(base + 256);
-  cudaError_t e = cudaMemsetAsync(base, 0, 12, s);
+  *ctr = (uint32_t*)b->scratch.ptr;
+  *queue = (uint32_t*)((char*)b->scratch.ptr + 256);
+  cudaError_t e = cudaMemsetAsync(b->scratch.ptr, 0, 32, s);
   if (e != cudaSuccess) return cuda_fail(e, "memset scratch");
   return LUCENT_OK;
 }
@@ -377,16 +388,28 @@ lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, ui
   lucent_status st = check_tmin(t_min, t_max);
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned* err;
-  uint32_t *qlen, *queue, *work;
-  if ((st = prepare_scratch(b, n, s, &err, &qlen, &queue, &work))) return st;
+  uint32_t *ctr, *queue;
+  if ((st = prepare_scratch(b, n, s, &ctr, &queue))) return st;
   if (n == 0) return LUCENT_OK;
   if (b->tri_count == 0) {  // bvh.ts:274: an empty BVH never hits
     cudaError_t e = cudaMemsetAsync(prim_d, 0xff, (size_t)n * 4, s);
     return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "memset");
   }
   const Node* wide = nullptr;
-  if (b->mode == LUCENT_TRAVERSE_WIDE) {
+  if (b->mode == LUCENT_TRAVERSE_WIDE && !b->near_tried) {
+    // Building the view waits for its verdict, which a capture cannot: the
+    // captured call then takes the four-wide view.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(s, &cap);
+    if (cap == cudaStreamCaptureStatusNone) {
+      if ((st = build_near_view((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, b->tri_count,
+                                b->lo, b->hi, b->near, s)))
+        return st;
+      b->near_tried = true;
+    }
+  }
+  const bool near = b->mode == LUCENT_TRAVERSE_WIDE && b->near.usable;
+  if (b->mode == LUCENT_TRAVERSE_WIDE && !(near && b->near.wide_range)) {
     if (!b->wide.ptr) {
       if ((st = b->wide.reserve((size_t)b->node_count * 4 * sizeof(Node)))) return st;
       launch_wide_view((const Node*)b->nodes.ptr, b->node_count, (Node*)b->wide.ptr, s);
@@ -394,8 +417,8 @@ lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, ui
     wide = (const Node*)b->wide.ptr;
   }
   launch_closest((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, rays_d, n, t_min, t_max, prim_d, t_d, u_d,
-                 v_d, queue, qlen, work, err, b->mode == LUCENT_TRAVERSE_EXACT || b->depth + 2 > kTsStack,
-                 b->mode == LUCENT_TRAVERSE_FAST, s, wide);
+                 v_d, queue, ctr, b->mode == LUCENT_TRAVERSE_EXACT || b->depth + 2 > kTsStack, b->mode == LUCENT_TRAVERSE_FAST, s,
+                 wide, near ? &b->near : nullptr);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "closest-hit launch");
 }
@@ -467,9 +490,8 @@ lucent_status lucent_bvh_intersect_f64(lucent_bvh* b, const double* rays, uint32
   cudaStream_t s = (cudaStream_t)stream;
   const size_t rb = (size_t)n * 48, ob = (size_t)n * 8;
   if ((st = b->stage.reserve(rb + 4 * ob + 64))) return st;
-  unsigned *err;
-  uint32_t *qlen, *queue;
-  if ((st = prepare_scratch(b, 0, s, &err, &qlen, &queue))) return st;
+  uint32_t *ctr, *queue;
+  if ((st = prepare_scratch(b, 0, s, &ctr, &queue))) return st;
   char* base = (char*)b->stage.ptr;
   double* rays_d = (double*)base;
   int32_t* prim_d = (int32_t*)(base + rb);
@@ -479,7 +501,7 @@ lucent_status lucent_bvh_intersect_f64(lucent_bvh* b, const double* rays, uint32
   cudaError_t e = cudaMemcpyAsync(rays_d, rays, rb, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return cuda_fail(e, "upload rays");
   launch_closest_d((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, rays_d, n, t_min, t_max, prim_d, t_d, u_d,
-                   v_d, err, s);
+                   v_d, ctr, s);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(prim_out, prim_d, (size_t)n * 4, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(t_out, t_d, ob, cudaMemcpyDeviceToHost, s);

@@ -2,7 +2,7 @@
 // rays as 6 floats (or doubles) each, results per ray, hit ids equal to the
 // reference's intersectBVH (src/math/bvh.ts:265-320).
 #include "internal.h"
-#include "traverse_wide.cuh"
+#include "traverse_near.cuh"
 
 namespace lucent {
 
@@ -30,6 +30,8 @@ struct ApiPolicy {
   // Lanes of a wide-kernel warp that wait before it fetches new rays
   // (measured on 10^6 random rays into a 65,536-triangle soup: 4 over 1, 8, 16).
   static constexpr int kRefillMin = 4;
+    static constexpr int kNearThreads = 128, kNearBlocks = 8, kNearRefill = 4;
+  __device__ Node leaf_box(const TravArgs& A, int, int slot) const { return load_node(A.nodes, __ldg(A.leaf_of + slot)); }
   __device__ bool alpha(int, int, uint32_t, float, float) const { return true; }
   __device__ AlphaAnswer alpha_fast(int, int, uint32_t) const { return kAlphaBlock; }
   __device__ bool alpha_any() const { return false; }
@@ -165,32 +167,52 @@ void launch_unpack(const Node* nodes, uint32_t count, const float4* tris, uint32
 
 void launch_closest(const Node* nodes, uint32_t node_count, const float4* tris, const float* rays_d, uint32_t n,
                     double tMin, double tMax, int32_t* prim, float* t, float* u, float* v, uint32_t* queue,
-                    uint32_t* queue_len, uint32_t* work, unsigned* err, bool exact_only, bool top_levels,
-                    cudaStream_t s, const Node* wide) {
+                    uint32_t* ctr, bool exact_only, bool top_levels, cudaStream_t s, const Node* wide,
+                    const NearTree* near) {
   if (n == 0) return;
   const ApiPolicy P{rays_d, n, tris, prim, t, u, v, tMin};
-  TravArgs A{nodes, node_count, tris, tMin, tMax, queue, queue_len, work, err, nullptr, top_levels ? 1 : 0};
+  using Listed = Queued<ApiPolicy>;
+  TravArgs A{nodes, node_count, tris, tMin, tMax, queue, ctr + 1, ctr + 2, ctr, nullptr, top_levels ? 1 : 0};
   if (exact_only) {
     TravArgs E = A;
     E.queue = nullptr;
     k_closest_exact_t<ApiPolicy><<<grid_for(n, 128), 128, 0, s>>>(E, P);
     return;
   }
-  static int blocks = 0, wide_blocks = 0;
-  if (!blocks) {
-    blocks = persistent_blocks((const void*)k_closest_fast_t<ApiPolicy>, ApiPolicy::kThreads);
-    wide_blocks = persistent_blocks((const void*)k_closest_wide_t<ApiPolicy>, ApiPolicy::kThreads);
-  }
+  static const int blocks = persistent_blocks((const void*)k_closest_fast_t<ApiPolicy>, ApiPolicy::kThreads);
+  static const int wide_blocks = persistent_blocks((const void*)k_closest_wide_t<ApiPolicy>, ApiPolicy::kThreads);
+  static const int near_blocks = persistent_blocks((const void*)k_closest_near_t<ApiPolicy>, ApiPolicy::kNearThreads);
   const int want = (int)((n + ApiPolicy::kThreads - 1) / ApiPolicy::kThreads);
-  if (wide) {
-    A.wide = wide;
+  if (near) {
+    TravArgs N = A;
+    N.near = {(const Node*)near->records.ptr, tris, 0, near->bound, near->far};
+    N.leaf_of = (const uint32_t*)near->leaf_of.ptr;
+    k_closest_near_t<ApiPolicy><<<near_blocks, ApiPolicy::kNearThreads, 0, s>>>(N, P);
+    // The rays it hands on, in the reference's order: over the four-wide view
+    // where they may be many (`wide` is then given), else over the binary nodes.
     A.top_scenes = 0;
-    k_closest_wide_t<ApiPolicy><<<want < wide_blocks ? want : wide_blocks, ApiPolicy::kThreads, 0, s>>>(A, P);
+    A.work = ctr + 3;
+    A.wide = wide;
+    const Listed L{P, queue, ctr + 1};
+    if (wide) {
+      A.queue = queue + n;
+      A.queue_len = ctr + 4;
+      k_closest_wide_t<Listed><<<want < wide_blocks ? want : wide_blocks, ApiPolicy::kThreads, 0, s>>>(A, L);
+      k_closest_exact_t<Listed><<<grid_for(n < 4096 ? n : 4096, 128), 128, 0, s>>>(A, L);
+    } else {
+      k_closest_fast_t<Listed, true><<<want < blocks ? want : blocks, ApiPolicy::kThreads, 0, s>>>(A, L);
+    }
   } else {
-    k_closest_fast_t<ApiPolicy><<<want < blocks ? want : blocks, ApiPolicy::kThreads, top_smem_bytes(A.top_scenes), s>>>(A, P);
+    if (wide) {
+      A.wide = wide;
+      A.top_scenes = 0;
+      k_closest_wide_t<ApiPolicy><<<want < wide_blocks ? want : wide_blocks, ApiPolicy::kThreads, 0, s>>>(A, P);
+    } else {
+      k_closest_fast_t<ApiPolicy><<<want < blocks ? want : blocks, ApiPolicy::kThreads, top_smem_bytes(A.top_scenes), s>>>(A, P);
+    }
+    // Slow path over the rays the fast kernel queued (length read on the device).
+    k_closest_exact_t<ApiPolicy><<<grid_for(n < 4096 ? n : 4096, 128), 128, 0, s>>>(A, P);
   }
-  // Slow path over the rays the fast kernel queued (length read on the device).
-  k_closest_exact_t<ApiPolicy><<<grid_for(n < 4096 ? n : 4096, 128), 128, 0, s>>>(A, P);
   k_refine_api<<<grid_for(n, 256), 256, 0, s>>>(P);
 }
 

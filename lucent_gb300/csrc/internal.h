@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/lucent.h"
+#include "api_util.h"
 #include "common.cuh"
 
 namespace lucent {
@@ -17,16 +18,37 @@ void launch_gather_tris(const float* pos_d, const uint32_t* idx_d, uint32_t tri_
                         cudaStream_t s);
 void launch_unpack(const Node* nodes, uint32_t count, const float4* tris, uint32_t tri_count, float* ref_d,
                    uint32_t* idx_d, cudaStream_t s);
+// `ctr`: 8 zeroed words (error word, queue lengths, ray counters); `queue`: n words, 2 n with `near`.
+struct NearTree;
 void launch_closest(const Node* nodes, uint32_t node_count, const float4* tris, const float* rays_d, uint32_t n, double tMin,
-                    double tMax, int32_t* prim, float* t, float* u, float* v, uint32_t* queue, uint32_t* queue_len,
-                    uint32_t* work, unsigned* err, bool exact_only, bool top_levels, cudaStream_t s,
-                    const Node* wide = nullptr);
+                    double tMax, int32_t* prim, float* t, float* u, float* v, uint32_t* queue, uint32_t* ctr,
+                    bool exact_only, bool top_levels, cudaStream_t s, const Node* wide = nullptr,
+                    const NearTree* near = nullptr);
 // Four-wide view of a binary node array (traverse_wide.cuh): 4 records per node.
 void launch_wide_view(const Node* nodes, uint32_t node_count, Node* wide, cudaStream_t s);
 void launch_closest_d(const Node* nodes, uint32_t node_count, const float4* tris, const double* rays_d, uint32_t n, double tMin,
                       double tMax, int32_t* prim, double* t, double* u, double* v, unsigned* err, cudaStream_t s);
 
-struct DeviceBuffer;
+// Nearest-first view of a tree (traverse_near.cuh, near_build.cu): records,
+// each slot's leaf, the centre of the tree with the radius within which ray
+// origins may lie, and how the box growth for farther origins rises with their
+// distance. Not usable (and empty) for trees the argument does not
+// cover. `tris`: slot order, 3 float4 each; lo, hi: the root's box.
+struct NearTree {
+  DeviceBuffer records{nullptr, 0, true}, leaf_of{nullptr, 0, true};
+  float4 bound = {0.f, 0.f, 0.f, 0.f};  // centre, radius
+  float2 far = {0.f, 0.f};              // from this distance on, growth per unit of distance
+  bool wide_range = false;              // the radius is 64 diagonals or more
+  bool usable = false;
+  void release() {
+    records.release();
+    leaf_of.release();
+    usable = false;
+  }
+};
+lucent_status build_near_view(const Node* nodes, uint32_t n_nodes, const float4* tris, uint32_t n_tris,
+                              const float lo[3], const float hi[3], NearTree& out, cudaStream_t s);
+
 // Texture arrays (texture.cu): decode tables (512: sRGB byte -> linear, then
 // byte / 255) and sRGB code-value midpoints (255), the shared layer size
 // (renderer.ts:316-322), and the resampling of each referenced image into its

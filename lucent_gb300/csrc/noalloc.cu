@@ -107,14 +107,12 @@ extern "C" lucent_status lucent_bvh_intersect_noalloc(const float* nodes_d, uint
   lucent_status st = noalloc_scratch(&base);
   if (st) return st;
   char* b = (char*)base;
-  unsigned* err = (unsigned*)b;
-  uint32_t* qlen = (uint32_t*)(b + 4);
-  uint32_t* work = (uint32_t*)(b + 8);
-  uint32_t* bad = (uint32_t*)(b + 12);
+  unsigned* err = (unsigned*)b;  // the launch's counter words start here
+  uint32_t* bad = (uint32_t*)(b + 32);
   uint32_t* queue = (uint32_t*)(b + kNoAllocHeader);
   // The array keeps the previous call's contents: the counters must start at
   // zero and the first-bad-record slot at its maximum.
-  e = cudaMemsetAsync(b, 0, 12, s);
+  e = cudaMemsetAsync(b, 0, 32, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0xff, 4, s);
   if (e != cudaSuccess) return cuda_fail(e, "clear no-allocation scratch");
   const uint32_t m = node_count > tri_count ? node_count : tri_count;
@@ -122,16 +120,16 @@ extern "C" lucent_status lucent_bvh_intersect_noalloc(const float* nodes_d, uint
                                                 err, bad);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  unsigned word[4] = {0, 0, 0, 0};
+  unsigned word[9] = {0};
   if (e == cudaSuccess) e = cudaMemcpy(word, b, sizeof word, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "no-allocation tree check");
   if (word[0] & kErrTree) {
-    if (word[3] < node_count) return fail(LUCENT_ERR_INVALID, "malformed BVH: node %u", word[3]);
+    if (word[8] < node_count) return fail(LUCENT_ERR_INVALID, "malformed BVH: node %u", word[8]);
     return fail(LUCENT_ERR_INVALID, "malformed BVH: triangle slot %u has a source index out of range",
-                word[3] - node_count);
+                word[8] - node_count);
   }
   launch_closest((const Node*)nodes_d, node_count, (const float4*)tris_d, rays_d, n, t_min, t_max, prim_d, t_d, u_d,
-                 v_d, queue, qlen, work, err, false, true, s);
+                 v_d, queue, (uint32_t*)err, false, true, s);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaMemcpy(word, err, sizeof word[0], cudaMemcpyDeviceToHost);

@@ -22,7 +22,7 @@
 #include "render_internal.h"
 #include "shade.cuh"
 #include "traverse.cuh"
-#include "traverse_wide.cuh"
+#include "traverse_near.cuh"
 
 namespace lucent {
 
@@ -50,6 +50,9 @@ struct PathClosestMulti {
   // stalls the warp on the atomic and the new rays' loads (path tracing's
   // short rays: 24 measured best of 1, 4, 8, 16, 24, 32).
   static constexpr int kRefillMin = 24;
+    // Nearest-first closest hit (box frame): 128 x 8 blocks 2.68 ms, x 7 2.75, x 6 and 256 x 3
+  // slower by 3 to 5 %; refills at 24 lanes 3.27 ms (before the batched expansions), 16 3.41, 8 3.73.
+  static constexpr int kNearThreads = 128, kNearBlocks = 8, kNearRefill = 24;
   __device__ uint32_t count() const { return *cnt; }
   __device__ uint32_t path(uint32_t k) const { return __float_as_uint(rays[2 * (size_t)k].w); }
   __device__ void ray(uint32_t k, float3& o, float3& d) const {
@@ -61,6 +64,15 @@ struct PathClosestMulti {
   __device__ BvhView scene_bvh(int sc) const {
     const SceneDev& S = recs[sc].scene;
     return {S.nodes, S.geo, S.node_count, sc, S.wide};
+  }
+  __device__ NearView near_view(uint32_t k) const { return scene_near(__float_as_int(rays[2 * (size_t)k + 1].w)); }
+  __device__ NearView scene_near(int sc) const {
+    const SceneDev& S = recs[sc].scene;
+    return {S.near, S.geo, sc, S.near_bound, S.near_far};
+  }
+  __device__ Node leaf_box(const TravArgs&, int sc, int slot) const {
+    const SceneDev& S = recs[sc].scene;
+    return load_node(S.nodes, __ldg(S.leaf_of + slot));
   }
   __device__ uint32_t key(uint32_t k) const { return __float_as_uint(ro[path(k)].w); }
   __device__ bool alpha_any() const { return any_alpha != 0; }
@@ -99,6 +111,15 @@ struct PathShadowMulti {
   __device__ BvhView scene_bvh(int sc) const {
     const SceneDev& S = recs[sc].scene;
     return {S.nodes, S.geo, S.node_count, sc, S.wide};
+  }
+  __device__ NearView near_view(uint32_t k) const { return scene_near(__ldg(sid + queue[k] / 3)); }
+  __device__ NearView scene_near(int sc) const {
+    const SceneDev& S = recs[sc].scene;
+    return {S.near, S.geo, sc, S.near_bound, S.near_far};
+  }
+  __device__ Node leaf_box(const TravArgs&, int sc, int slot) const {
+    const SceneDev& S = recs[sc].scene;
+    return load_node(S.nodes, __ldg(S.leaf_of + slot));
   }
   __device__ float tmax32(uint32_t k) const { return so[k].w; }
   __device__ uint32_t key(uint32_t k) const { return __float_as_uint(sd[k].w); }
@@ -956,6 +977,7 @@ __global__ void k_zero_counters(uint32_t* ctr, int nxt) {
     ctr[kCtrShadow] = 0;
     ctr[kCtrWork] = 0;
     ctr[kCtrSlow] = 0;
+    ctr[kCtrRestWork] = 0;
     ctr[kCtrWork2] = 0;
     ctr[kCtrSlow2] = 0;
     ctr[kCtrTex] = 0;
@@ -969,6 +991,7 @@ __global__ void k_zero_closest_counters(uint32_t* ctr) {
   if (threadIdx.x == 0) {
     ctr[kCtrWork] = 0;
     ctr[kCtrSlow] = 0;
+    ctr[kCtrRestWork] = 0;
   }
 }
 __global__ void k_zero_shade_counters(uint32_t* ctr, int nxt) {
@@ -1171,22 +1194,53 @@ static int aux_blocks() {
   return n;
 }
 
-// Closest hit of a bounce: over the scenes' four-wide BVH views, or the
-// binary nodes with the top levels staged in shared memory. Hits are the same.
-static void launch_closest_multi(int wide, int blocks, int top, const TravArgs& A, const PathClosestMulti& pc,
-                                 cudaStream_t s) {
-  if (wide)
-    k_closest_wide_t<PathClosestMulti><<<blocks, PathClosestMulti::kThreads, 0, s>>>(A, pc);
-  else
-    k_closest_fast_t<PathClosestMulti><<<blocks, PathClosestMulti::kThreads, top_smem_bytes(top), s>>>(A, pc);
+// Grids of the traversal kernels: all resident blocks.
+struct TraversalGrids {
+  int fast, wide, near, any;
+};
+static const TraversalGrids& traversal_grids() {
+  static const TraversalGrids g{
+      persistent_blocks((const void*)k_closest_fast_t<PathClosestMulti>, PathClosestMulti::kThreads),
+      persistent_blocks((const void*)k_closest_wide_t<PathClosestMulti>, PathClosestMulti::kThreads),
+      persistent_blocks((const void*)k_closest_near_t<PathClosestMulti>, PathClosestMulti::kNearThreads),
+      persistent_blocks((const void*)k_anyhit_near_t<PathShadowMulti>, kAnyThreads)};
+  return g;
 }
 
-static void launch_shadow_multi(int wide, int blocks, int top, const TravArgs& A, const PathShadowMulti& ps,
+// Closest hit of a bounce: nearest first, then the rays that could not be
+// proven in the reference's order; or all rays in that order, over the scenes'
+// four-wide BVH views or the binary nodes with the top levels staged in shared
+// memory, then those outside the binary32 bounds. Hits are the same.
+static void launch_closest_multi(const MultiLaunch& M, const Paths& P, const TravArgs& A, const PathClosestMulti& pc,
+                                 cudaStream_t s) {
+  const TraversalGrids& G = traversal_grids();
+  const int own = M.trace_blocks;
+  if (M.near) {
+    k_closest_near_t<PathClosestMulti><<<own > 0 ? own : G.near, PathClosestMulti::kNearThreads, 0, s>>>(A, pc);
+    TravArgs R = A;
+    R.work = P.ctr + kCtrRestWork;
+    using Listed = Queued<PathClosestMulti>;
+    k_closest_wide_t<Listed, true><<<own > 0 ? own : G.wide, PathClosestMulti::kThreads, 0, s>>>(R, Listed{pc, A.queue, A.queue_len});
+    return;
+  }
+  if (M.wide)
+    k_closest_wide_t<PathClosestMulti><<<own > 0 ? own : G.wide, PathClosestMulti::kThreads, 0, s>>>(A, pc);
+  else
+    k_closest_fast_t<PathClosestMulti><<<own > 0 ? own : G.fast, PathClosestMulti::kThreads, top_smem_bytes(A.top_scenes), s>>>(A, pc);
+  k_closest_exact_t<PathClosestMulti><<<64, 128, 0, s>>>(A, pc);
+}
+
+// Any hit of a bounce's shadow rays, in the same three forms.
+static void launch_shadow_multi(const MultiLaunch& M, int blocks, const TravArgs& A, const PathShadowMulti& ps,
                                 cudaStream_t s) {
-  if (wide)
+  const TraversalGrids& G = traversal_grids();
+  if (M.near)
+    k_anyhit_near_t<PathShadowMulti><<<G.any, kAnyThreads, 0, s>>>(A, ps);
+  else if (M.wide)
     k_anyhit_wide_t<PathShadowMulti><<<blocks, 256, 0, s>>>(A, ps);
   else
-    k_anyhit_fast_t<PathShadowMulti><<<blocks, 256, top_smem_bytes(top), s>>>(A, ps);
+    k_anyhit_fast_t<PathShadowMulti><<<blocks, 256, top_smem_bytes(A.top_scenes), s>>>(A, ps);
+  k_anyhit_exact_t<PathShadowMulti><<<64, 128, 0, s>>>(A, ps);
 }
 
 int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, bool accumulate) {
@@ -1198,13 +1252,7 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
   k_camera_multi<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, M.recs, M.path_base, M.n, M.sid, M.S);
   nl++;
   E.mark(kPhCamera, s);
-  static int max_closest = 0, max_wide = 0, max_shade = 0;
-  if (!max_closest) {
-    max_closest = persistent_blocks((const void*)k_closest_fast_t<PathClosestMulti>, PathClosestMulti::kThreads);
-    max_wide = persistent_blocks((const void*)k_closest_wide_t<PathClosestMulti>, PathClosestMulti::kThreads);
-    max_shade = persistent_blocks((const void*)k_shade_t<SceneTable>, 128);
-  }
-  const int closest_blocks = M.trace_blocks > 0 ? M.trace_blocks : M.wide ? max_wide : max_closest;
+  static const int max_shade = persistent_blocks((const void*)k_shade_t<SceneTable>, 128);
   const int shade_blocks = M.shade_blocks > 0 ? M.shade_blocks : max_shade;
   const int aux = M.shade_blocks > 0 ? M.shade_blocks : aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
@@ -1221,8 +1269,7 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
     PathClosestMulti pc{P.ctr + kCtrQ0 + cur, sorted ? P.sray : P.nray, P.ro, P.hit, M.recs, M.any_alpha};
     TravArgs A{nullptr, 0, nullptr, 1e-6, 1e30, P.slow, P.ctr + kCtrSlow, P.ctr + kCtrWork, P.ctr + kCtrErr,
                M.trav_stats, top};
-    launch_closest_multi(M.wide, closest_blocks, top, A, pc, s);
-    k_closest_exact_t<PathClosestMulti><<<64, 128, 0, s>>>(A, pc);
+    launch_closest_multi(M, P, A, pc, s);
     nl += 2;
     const bool capture = M.cap && (M.cap_mask >> b & 1u);
     const uint32_t region = capture ? 2u * (uint32_t)__builtin_popcount(M.cap_mask & ((1u << b) - 1u)) : 0u;
@@ -1255,8 +1302,7 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
     PathShadowMulti ps{P.ctr + kCtrShadow, P.qs, P.sh_o, P.sh_d, P.sh_c, M.recs, M.sid, M.any_alpha};
     TravArgs B{nullptr, 0, nullptr, 1e-6, 1e30, P.slow2, P.ctr + kCtrSlow2, P.ctr + kCtrWork2, P.ctr + kCtrErr,
                nullptr, top};
-    launch_shadow_multi(M.wide, aux * 2, top, B, ps, t);
-    k_anyhit_exact_t<PathShadowMulti><<<64, 128, 0, t>>>(B, ps);
+    launch_shadow_multi(M, aux * 2, B, ps, t);
     nl += 2;
     if (capture)
       k_capture_shadow<<<aux, 256, 0, t>>>(P.ctr + kCtrShadow, P.qs, P.sh_o, P.sh_d, P.sh_c,
@@ -1308,13 +1354,7 @@ int accumulate_wave(const MultiLaunch& M, cudaStream_t s) {
 // then propagating dl through every vertex.
 void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t s) {
   const SceneRec* rec = M.recs;
-  static int binary_blocks = 0, wide_blocks = 0, shade_blocks = 0;
-  if (!binary_blocks) {
-    binary_blocks = persistent_blocks((const void*)k_closest_fast_t<PathClosestMulti>, PathClosestMulti::kThreads);
-    wide_blocks = persistent_blocks((const void*)k_closest_wide_t<PathClosestMulti>, PathClosestMulti::kThreads);
-    shade_blocks = persistent_blocks((const void*)k_shade_t<SceneTable, true>, 128);
-  }
-  const int closest_blocks = M.wide ? wide_blocks : binary_blocks;
+  static const int shade_blocks = persistent_blocks((const void*)k_shade_t<SceneTable, true>, 128);
   const int aux = aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
   for (int pass = 0; pass < 2; pass++) {
@@ -1332,8 +1372,7 @@ void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t
       PathClosestMulti pc{P.ctr + kCtrQ0 + cur, sorted ? P.sray : P.nray, P.ro, P.hit, M.recs, M.any_alpha};
       TravArgs TA{nullptr, 0, nullptr, 1e-6, 1e30, P.slow, P.ctr + kCtrSlow, P.ctr + kCtrWork, P.ctr + kCtrErr,
                   nullptr, top};
-      launch_closest_multi(M.wide, closest_blocks, top, TA, pc, s);
-      k_closest_exact_t<PathClosestMulti><<<64, 128, 0, s>>>(TA, pc);
+      launch_closest_multi(M, P, TA, pc, s);
       if (forked) {  // the previous bounce's resolve (lrem, radiance) precedes this shade
         cudaStreamWaitEvent(s, M.ev_join, 0);
         k_zero_shade_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
@@ -1349,8 +1388,7 @@ void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t
       PathShadowMulti ps{P.ctr + kCtrShadow, P.qs, P.sh_o, P.sh_d, P.sh_c, M.recs, M.sid, M.any_alpha};
       TravArgs TB{nullptr, 0, nullptr, 1e-6, 1e30, P.slow2, P.ctr + kCtrSlow2, P.ctr + kCtrWork2, P.ctr + kCtrErr,
                   nullptr, top};
-      launch_shadow_multi(M.wide, aux * 2, top, TB, ps, t);
-      k_anyhit_exact_t<PathShadowMulti><<<64, 128, 0, t>>>(TB, ps);
+      launch_shadow_multi(M, aux * 2, TB, ps, t);
       Paths Pr = P;  // resolve walks the pre-sort queue, in path order
       if (sorted) Pr.q[cur] = P.sort_tmp;
       if (pass == 1)  // the primal replay resolves in its next shade and in k_seed_lrem

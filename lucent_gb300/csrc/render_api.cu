@@ -304,7 +304,7 @@ static void wave_key(const MultiLaunch& M, uint64_t key[4]) {
   key[1] = (uint64_t)M.total_pixels | ((uint64_t)(uint32_t)M.trace_blocks << 32) ^ ((uint64_t)M.sort_classes << 48);
   key[2] = ((uint64_t)(uintptr_t)M.paths.rec) ^ ((uint64_t)M.max_bounces << 48) ^ ((uint64_t)M.shade_blocks << 56);
   key[3] = ((uint64_t)(uintptr_t)M.recs) ^ ((uint64_t)(uintptr_t)M.path_base << 20) ^ ((uint64_t)M.any_alpha << 59) ^
-           ((uint64_t)(M.side != nullptr) << 57) ^ ((uint64_t)M.wide << 58) ^ ((uint64_t)M.any_tex << 60) ^ ((uint64_t)M.sort_rays << 61) ^
+           ((uint64_t)M.near << 56) ^ ((uint64_t)(M.side != nullptr) << 57) ^ ((uint64_t)M.wide << 58) ^ ((uint64_t)M.any_tex << 60) ^ ((uint64_t)M.sort_rays << 61) ^
            ((uint64_t)M.top_levels << 62) ^
            ((uint64_t)(M.trav_stats != nullptr) << 63);
 }
@@ -314,6 +314,7 @@ struct lucent_renderer {
   // scene
   DeviceBuffer nodes, geo, attr, mats, spheres, sph_mat, sph_light, lights;
   DeviceBuffer wide;  // four-wide view of `nodes` (traverse_wide.cuh)
+  NearTree near;      // nearest-first view (traverse_near.cuh)
   // A view (lucent_renderer_create_view) renders `src`'s scene: the scene
   // fields below are read from src; n_views counts the views of this one.
   lucent_renderer* src = nullptr;
@@ -523,7 +524,8 @@ static SceneRec scene_rec(const lucent_renderer* r) {
              (const int*)o->sph_light.ptr, (int)o->sphere_count, (const float4*)o->lights.ptr, (int)o->light_count,
              r->ground_enabled ? o->ground_material : -1, r->ground_height, o->any_alpha,
              (const uchar4*)o->color_maps.ptr, (const uchar4*)o->data_maps.ptr, (const float*)o->texel_lut.ptr,
-             o->tex_size, (const Node*)o->wide.ptr};
+             o->tex_size, (const Node*)o->wide.ptr, (const Node*)o->near.records.ptr,
+             (const uint32_t*)o->near.leaf_of.ptr, o->near.bound, o->near.far};
   R.light = r->light;
   R.cam = r->cam;
   R.accum = {(float4*)r->color.ptr, (half4*)r->albedo.ptr, (half4*)r->normal.ptr, (float*)r->history.ptr};
@@ -606,6 +608,7 @@ static lucent_status single_launch(lucent_renderer* r, WaveSet& w, uint32_t S, u
   M.sort_rays = r->sort_rays;
   M.top_levels = r->top_levels;
   M.wide = r->wide_bvh;
+  M.near = r->wide_bvh && scene_owner(r)->near.usable;
   M.sort_classes = 1;
   M.any_tex = scene_owner(r)->tex_size > 0;
   if (r->cap_mask) {
@@ -679,6 +682,7 @@ void lucent_renderer_destroy(lucent_renderer* r) {
                           &r->history, &r->den_a, &r->den_b, &r->guide0, &r->guide1, &r->disp, &r->adj_dl, &r->adj_path, &r->adj_grad, &r->prev,
                           &r->color_maps, &r->data_maps, &r->texel_lut})
     b->release();
+  r->near.release();
   for (WaveSet& w : r->set) w.destroy();
   if (r->ev0) cudaEventDestroy(r->ev0);
   if (r->ev1) cudaEventDestroy(r->ev1);
@@ -822,7 +826,10 @@ lucent_status lucent_renderer_load_scene(lucent_renderer* r, const lucent_scene_
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cleanup(cuda_fail(e, "scene upload"));
-  if ((st = load_textures(r, d, s))) return cleanup(st);
+  if ((st = load_textures(r, d, s)) ||
+      (st = build_near_view((const Node*)r->nodes.ptr, nc, (const float4*)r->geo.ptr, n, ref.data(), ref.data() + 4,
+                            r->near, s)))
+    return cleanup(st);
   r->node_count = nc;
   r->tri_count = n;
   r->material_count = M;
@@ -1549,7 +1556,7 @@ lucent_status lucent_batch_trace(lucent_batch* b, uint32_t samples, void* stream
   // group: samples_per_wave, or as many as fit in max_wave_paths (at least one).
   const int k = b->opt.scenes_per_wave ? (int)std::min<uint32_t>(b->opt.scenes_per_wave, (uint32_t)n) : n;
   struct Group {
-    int i0, i1, max_bounces, any_alpha, any_tex, classes;
+    int i0, i1, max_bounces, any_alpha, any_tex, classes, near;
     uint64_t pixels;
     uint32_t S, full, tail;
     size_t base;  // offset of the group's bases (full waves, then the tail wave) in b->bases, in words
@@ -1568,7 +1575,7 @@ lucent_status lucent_batch_trace(lucent_batch* b, uint32_t samples, void* stream
     }
   };
   for (int i0 = 0; i0 < n; i0 += k) {
-    Group G{i0, std::min(n, i0 + k), 0, 0, 0, 0, 0, 0, 0, 0, hb.size()};
+    Group G{i0, std::min(n, i0 + k), 0, 0, 0, 0, 1, 0, 0, 0, 0, hb.size()};
     std::vector<const Node*> bvhs;  // ray-sort classes: scenes sharing a BVH (views) sort together
     for (int i = G.i0; i < G.i1; i++) {
       const Node* nodes = recs[i].scene.nodes;
@@ -1580,6 +1587,7 @@ lucent_status lucent_batch_trace(lucent_batch* b, uint32_t samples, void* stream
       G.max_bounces = std::max(G.max_bounces, (int)b->rs[i]->max_bounces);
       G.any_alpha |= scene_owner(b->rs[i])->any_alpha;
       G.any_tex |= scene_owner(b->rs[i])->tex_size > 0;
+      G.near &= scene_owner(b->rs[i])->near.usable;
     }
     G.classes = (int)bvhs.size();
     uint64_t S = b->opt.samples_per_wave ? b->opt.samples_per_wave
@@ -1631,6 +1639,7 @@ lucent_status lucent_batch_trace(lucent_batch* b, uint32_t samples, void* stream
     M.max_bounces = G.max_bounces;
     M.any_alpha = G.any_alpha;
     M.any_tex = G.any_tex;
+    M.near = M.wide && G.near;
     M.total_pixels = (uint32_t)G.pixels;
     M.sort_classes = G.classes;
     for (uint32_t w = 0; w < G.full + (G.tail ? 1u : 0u); w++) {

@@ -12,9 +12,10 @@ enum : int {
   kCtrShadow = 2,       // shadow-queue length
   kCtrWork = 3,         // closest-hit persistent ray counter
   kCtrSlow = 4,         // closest-hit slow-path queue length
-  kCtrWork2 = 5,        // any-hit work counter (unused by the grid-stride kernel)
+  kCtrWork2 = 5,        // any-hit persistent ray counter (nearest-first kernel)
   kCtrSlow2 = 6,        // any-hit slow-path queue length
   kCtrErr = 7,          // device error word
+  kCtrRestWork = 13,    // persistent ray counter of the launch over the nearest-first kernel's queue
   kCtrTex = 12,         // textured-hit queue length (paths left to the TEX shade instantiation)
   kCtrStatClosest = 8,  // u64: closest-hit rays traced (words 8-9)
   kCtrStatShadow = 10,  // u64: shadow rays traced (words 10-11)
@@ -114,7 +115,8 @@ struct MultiLaunch {
   int sort_rays;                   // after bounces 0 and 1, sort the rays by BVH class, direction and origin cell
   int top_levels;                  // stage the top BVH levels of (up to 8) scenes in shared memory
   int any_tex;                     // some scene has texture maps: launch the TEX shade instantiation
-  int wide;                        // closest hit over the scenes' four-wide BVH views
+  int wide;                        // traversal over the scenes' four-wide BVH views
+  int near;                        // nearest-first traversal (every scene's view is usable, and wide is set)
   int sort_classes;                // distinct SceneRec::sort_class values (>= 1)
   // Ray capture (lucent_renderer_capture_rays; parity tests): for every
   // bounce b in cap_mask, the bounce's closest-hit rays with their hits and

@@ -152,6 +152,12 @@ struct SceneDev {
   const float* texel_lut;
   int tex_size;
   const Node* wide;  // four-wide view of `nodes` (traverse_wide.cuh) or nullptr
+  // Nearest-first view (traverse_near.cuh): records (nullptr: not usable), each
+  // slot's leaf, the ray origins it is proven for (NearTree).
+  const Node* near;
+  const uint32_t* leaf_of;
+  float4 near_bound;
+  float2 near_far;
 };
 
 // transformUV (scene.glsl:95-97): rows of a 2x3 affine map.

@@ -32,6 +32,9 @@
 //                                                 to compute later, with the warp converged
 //   void hit(uint32_t k, int slot, double t, double u, double v)   a hit with its binary64 values
 //   void miss(uint32_t k); void fail(uint32_t k)
+//   NearView near_view(uint32_t k) const          (nearest-first, kMultiScene) the k-th ray's view
+//   Node leaf_box(const TravArgs&, int scene, int slot) const   (nearest-first) the box of a slot's leaf
+//   static constexpr int kNearThreads, kNearBlocks, kNearRefill   (nearest-first closest hit) block shape, refill
 //   float tmax32(uint32_t k) const                (any hit) the ray's tMax, a binary32 value
 //   void shadow(uint32_t k, bool occluded)        (any hit)
 #pragma once
@@ -68,6 +71,16 @@ static __device__ __noinline__ bool slab_f64_culled(float4 mn, float4 mx, float3
   return ts_slab_culled(mn, mx, {o.x, o.y, o.z}, inv_exact(d), tMax);
 }
 
+// The tree one ray of a nearest-first launch traverses (traverse_near.cuh):
+// records, triangles, scene, and the ray origins it is proven for (NearTree).
+struct NearView {
+  const Node* nodes;
+  const float4* tris;
+  int scene;
+  float4 bound;
+  float2 far;
+};
+
 struct TravArgs {
   const Node* nodes;
   uint32_t node_limit;
@@ -85,8 +98,10 @@ struct TravArgs {
   int top_scenes = 0;
   // Four-wide view of `nodes` (traverse_wide.cuh) for the wide kernels.
   const Node* wide = nullptr;
+  // Nearest-first view and each slot's leaf (single-scene launches).
+  NearView near{};
+  const uint32_t* leaf_of = nullptr;
 };
-
 
 __device__ __forceinline__ void count_stat(const TravArgs& A, int k) {
   if (A.stats) atomicAdd(A.stats + k, 1ull);
@@ -108,6 +123,26 @@ __device__ __forceinline__ BvhView bvh_of(const TravArgs& A, const Pol& P, uint3
   else
     return {A.nodes, A.tris, A.node_limit, 0};
 }
+
+// A policy over the rays listed in a queue (nullptr: all of them): what the
+// nearest-first kernel hands to the kernels that follow the reference's order.
+template <class Pol>
+struct Queued : Pol {
+  const uint32_t* list;
+  const uint32_t* len;
+  __device__ uint32_t at(uint32_t k) const { return list ? list[k] : k; }
+  __device__ uint32_t count() const { return list ? *len : Pol::count(); }
+  __device__ void ray(uint32_t k, float3& o, float3& d) const { Pol::ray(at(k), o, d); }
+  __device__ uint32_t key(uint32_t k) const { return Pol::key(at(k)); }
+  __device__ BvhView bvh(uint32_t k) const {
+    if constexpr (Pol::kMultiScene) return Pol::bvh(at(k));
+    else return {};
+  }
+  __device__ void finish(uint32_t k, int slot) const { Pol::finish(at(k), slot); }
+  __device__ void hit(uint32_t k, int slot, double t, double u, double v) const { Pol::hit(at(k), slot, t, u, v); }
+  __device__ void miss(uint32_t k) const { Pol::miss(at(k)); }
+  __device__ void fail(uint32_t k) const { Pol::fail(at(k)); }
+};
 
 // Top BVH levels in shared memory. The top kTopDepth + 1 levels of a tree
 // (63 nodes, 2016 bytes) are copied at block start in breadth-first order,
@@ -209,21 +244,30 @@ __device__ bool trace_exact(const TravArgs& A, const Pol& P, const BvhView& bv, 
 }
 
 template <class Pol>
+__device__ __forceinline__ void closest_exact_ray(const TravArgs& A, const Pol& P, uint32_t k) {
+  float3 o, d;
+  P.ray(k, o, d);
+  int slot;
+  double t = 0, u = 0, v = 0;
+  if (!trace_exact(A, P, bvh_of(A, P, k), {o.x, o.y, o.z}, {d.x, d.y, d.z}, P.key(k), slot, t, u, v))
+    P.fail(k);
+  else if (slot < 0)
+    P.miss(k);
+  else
+    P.hit(k, slot, t, u, v);
+}
+
+template <class Pol>
 __global__ void k_closest_exact_t(TravArgs A, Pol P) {
   const uint32_t limit = A.queue ? *A.queue_len : P.count();
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < limit; q += gridDim.x * blockDim.x) {
-    const uint32_t k = A.queue ? A.queue[q] : q;
-    float3 o, d;
-    P.ray(k, o, d);
-    int slot;
-    double t = 0, u = 0, v = 0;
-    if (!trace_exact(A, P, bvh_of(A, P, k), {o.x, o.y, o.z}, {d.x, d.y, d.z}, P.key(k), slot, t, u, v))
-      P.fail(k);
-    else if (slot < 0)
-      P.miss(k);
-    else
-      P.hit(k, slot, t, u, v);
-  }
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < limit; q += gridDim.x * blockDim.x)
+    closest_exact_ray(A, P, A.queue ? A.queue[q] : q);
+}
+
+// Out of line, for a kernel that traces such rays where it meets them.
+template <class Pol>
+static __device__ __noinline__ void closest_exact_here(const TravArgs& A, const Pol& P, uint32_t k) {
+  closest_exact_ray(A, P, k);
 }
 
 // Fast path: persistent warps, one ray per lane; lanes refill from A.work as
@@ -238,8 +282,13 @@ __global__ void k_closest_exact_t(TravArgs A, Pol P) {
 // thread sets the resident warps per SM. Deep traversals of long rays (the
 // BVH API) gain from 28 warps at 72 registers; the renderer's short rays
 // lose more to the extra spills and keep 24 warps at 80 (measured).
-template <class Pol>
-__global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks) k_closest_fast_t(TravArgs A, Pol P) {
+//
+// `Rest`: the launch over the few rays that the nearest-first kernel hands on;
+// rays for the all-binary64 path are then traced in place, where a launch of
+// their own would cost more than they do.
+template <class Pol, bool Rest = false>
+__global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks)
+    k_closest_fast_t(const __grid_constant__ TravArgs A, const __grid_constant__ Pol P) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -285,7 +334,8 @@ __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks) k_closest_fast
           float3 o, d;
           P.ray(ri, o, d);
           if (!safe_ray(o, d)) {
-            A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+            if constexpr (Rest) closest_exact_here(A, P, ri);
+            else A.queue[atomicAdd(A.queue_len, 1u)] = ri;
           } else {
             r = make_ray32(o, d);
             key = use_alpha ? P.key(ri) : 0u;  // read only where alpha tests use it
@@ -422,7 +472,8 @@ __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks) k_closest_fast
       }
       have_cur = false;
       if (defer) {  // a textured alpha test: the binary64 kernel traces this ray
-        A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+        if constexpr (Rest) closest_exact_here(A, P, ri);
+        else A.queue[atomicAdd(A.queue_len, 1u)] = ri;
         active = false;
         continue;
       }

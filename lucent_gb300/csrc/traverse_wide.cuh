@@ -128,8 +128,10 @@ static __device__ __noinline__ Closest closest_exact(Closest s, float3 o, float3
 // whose own slab test the binary32 bounds leave open (`cond`), which is
 // visited and decided in binary64 only if one of its triangles is not
 // certainly rejected (otherwise the leaf changes nothing either way).
-template <class Pol>
-__global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks) k_closest_wide_t(TravArgs A, Pol P) {
+// `Rest` as in k_closest_fast_t.
+template <class Pol, bool Rest = false>
+__global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks)
+    k_closest_wide_t(const __grid_constant__ TravArgs A, const __grid_constant__ Pol P) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -166,7 +168,8 @@ __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks) k_closest_wide
           float3 o, d;
           P.ray(ri, o, d);
           if (!safe_ray(o, d)) {
-            A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+            if constexpr (Rest) closest_exact_here(A, P, ri);
+            else A.queue[atomicAdd(A.queue_len, 1u)] = ri;
           } else {
             r = make_ray32(o, d);
             key = use_alpha ? P.key(ri) : 0u;  // read only where alpha tests use it
@@ -285,7 +288,8 @@ __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks) k_closest_wide
       }
       have_cur = false;
       if (defer) {  // a textured alpha test: the binary64 kernel traces this ray
-        A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+        if constexpr (Rest) closest_exact_here(A, P, ri);
+        else A.queue[atomicAdd(A.queue_len, 1u)] = ri;
         active = false;
         continue;
       }
