@@ -256,26 +256,29 @@ static lucent_status build_common(const float* pos_d, uint32_t n, const lucent_b
                                   lucent_bvh** handle_out) {
   const int max_leaf = opts ? (int)opts->max_leaf_size : 4;  // bvh.ts:33 defaults
   const int bins = opts ? (int)opts->bins : 12;
-  std::vector<float> nodes;
-  std::vector<uint32_t> tri;
-  double bounds[6];
   lucent_bvh* b = handle_out ? new lucent_bvh() : nullptr;
-  lucent_status st = gpu_build_bvh(pos_d, n, max_leaf, bins, s, nodes, tri, bounds, b ? &b->nodes : nullptr,
-                                   b ? &b->tris : nullptr);
+  BuildOut out;
+  if (b) {
+    out.nodes = &b->nodes;
+    out.tris = &b->tris;
+  }
+  out.nodes_host = nodes_out;
+  out.tri_host = tri_out;
+  lucent_status st = gpu_build_bvh(pos_d, n, max_leaf, bins, s, out);
   if (st) {
     lucent_bvh_destroy(b);
     return st;
   }
-  const uint32_t nc = (uint32_t)(nodes.size() / 8);
-  if (nodes_out) memcpy(nodes_out, nodes.data(), nodes.size() * 4);
-  if (node_count_out) *node_count_out = nc;
-  if (tri_out && n) memcpy(tri_out, tri.data(), (size_t)n * 4);
-  if (bounds_out) memcpy(bounds_out, bounds, sizeof bounds);
+  if (node_count_out) *node_count_out = out.node_count;
+  if (bounds_out) memcpy(bounds_out, out.bounds, sizeof out.bounds);
   if (b) {
-    b->node_count = nc;
+    b->node_count = out.node_count;
     b->tri_count = n;
-    b->depth = tree_depth(nodes.data(), nc, n);
-    set_root(b, nodes.data());
+    b->depth = out.depth;
+    for (int k = 0; k < 3; k++) {
+      b->lo[k] = (float)out.bounds[k];
+      b->hi[k] = (float)out.bounds[3 + k];
+    }
     *handle_out = b;
   }
   return LUCENT_OK;

@@ -1,278 +1,183 @@
 // Host orchestration of the GPU BVH builder (included by bvh_build.cu).
-#include <vector>
+#include <algorithm>
 
 #include "api_util.h"
 
 namespace lucent {
 
-// Builds the BVH of `n` triangles at `pos_d` (device, 9 floats each).
-// Outputs the reference's node array and triIndices on the host, the bounds,
-// and (optionally) the device traversal layout: Node array + slot-order
-// triangles for a lucent_bvh handle.
-lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bins, cudaStream_t s,
-                            std::vector<float>& nodes_ref, std::vector<uint32_t>& tri_out, double bounds[6],
-                            DeviceBuffer* nodes_dev, DeviceBuffer* tris_dev) {
+// Builds the BVH of `n` triangles at `pos_d` (device, 9 floats each); `out`
+// says what is wanted. Before this form (a launch per step and level with the
+// host reading each level's nodes, one warp walking each small node out of L2,
+// the tree renumbered on the host): 2,503 triangles 0.75 ms, 300,000 8.7 ms,
+// 2,000,000 42 ms.
+lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bins, cudaStream_t s, BuildOut& out) {
   using namespace build;
   if (bins < 2 || bins > kMaxBins) return fail(LUCENT_ERR_UNSUPPORTED, "bins must be in [2, %d]", kMaxBins);
   if (max_leaf < 1) return fail(LUCENT_ERR_INVALID, "maxLeafSize must be >= 1");
   if (n > (1u << 23)) return fail(LUCENT_ERR_UNSUPPORTED, "%u triangles; the limit is 2^23", n);
-  tri_out.assign(n, 0);
+  lucent_status st = LUCENT_OK;
   if (n == 0) {  // bvh.ts:143-147
-    nodes_ref.assign(8, 0.f);
-    for (int k = 0; k < 6; k++) bounds[k] = 0;
-    if (nodes_dev) {
-      lucent_status st = nodes_dev->reserve(sizeof(Node));
-      if (st) return st;
-      cudaMemsetAsync(nodes_dev->ptr, 0, sizeof(Node), s);
+    for (int k = 0; k < 6; k++) out.bounds[k] = 0;
+    for (int k = 0; k < 8 && out.nodes_host; k++) out.nodes_host[k] = 0.f;
+    out.node_count = 1;
+    out.depth = 0;
+    if (out.nodes) {
+      if ((st = out.nodes->reserve(sizeof(Node)))) return st;
+      cudaError_t e = cudaMemsetAsync(out.nodes->ptr, 0, sizeof(Node), s);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+      if (e != cudaSuccess) return cuda_fail(e, "empty BVH");
     }
-    if (tris_dev) {
-      lucent_status st = tris_dev->reserve(48);
-      if (st) return st;
-    }
+    if (out.tris && (st = out.tris->reserve(48))) return st;
+    if (out.order && (st = out.order->reserve(16))) return st;
     return LUCENT_OK;
   }
 
-  const uint32_t small_max = 2048;
-  const uint32_t cap = n;
-  // Scratch, one allocation: prim bounds, orders, partition positions, node
-  // records, lists, and the big-node levels' chunks and partial results (at
-  // most n / 2049 big nodes of a chunk per 4096 triangles and a ragged one).
-  const uint32_t big_cap = n / (small_max + 1) + 1, chunk_cap = n / kChunk + big_cap;
-  TempBuffer scratch;
-  auto release_all = [&]() { scratch.release(); };
-  lucent_status st = LUCENT_OK;
-#define BB_TRY(x)      \
-  do {                 \
-    st = (x);          \
-    if (st) {          \
-      release_all();   \
-      return st;       \
-    }                  \
-  } while (0)
-#define BB_CUDA(x, what)                      \
-  do {                                        \
-    cudaError_t e_ = (x);                     \
-    if (e_ != cudaSuccess) {                  \
-      release_all();                          \
-      return cuda_fail(e_, what);             \
-    }                                         \
-  } while (0)
-  const uint32_t nrec = 2 * n - 1;
+  // Scratch, one allocation. Big nodes hold more than kSub triangles, so a
+  // level has at most n / (kSub + 1) of them, each with one ragged chunk.
+  const uint32_t nrec = 2 * n - 1, big_cap = n / (kSub + 1) + 1, chunk_cap = n / kChunk + big_cap;
+  const size_t words = (size_t)3 * bins * 7;
   struct Part {
     size_t bytes;
     void* ptr;
   };
-  Part b_lo{(size_t)n * 16}, b_hi{(size_t)n * 16}, b_cz{(size_t)n * 4}, b_tri{(size_t)n * 4}, b_tmp{(size_t)n * 4},
-      b_P{(size_t)n * 4}, b_Q{(size_t)n * 4}, b_recs{(size_t)nrec * sizeof(NodeRec)}, b_ctr{64},
-      b_small{(size_t)cap * sizeof(Task)}, b_bigA{(size_t)cap * sizeof(Task)}, b_bigB{(size_t)cap * sizeof(Task)},
-      b_info{(size_t)big_cap * sizeof(BigInfo)}, b_chunks{(size_t)chunk_cap * sizeof(Chunk)},
-      b_first{((size_t)big_cap + 1) * 4}, b_part{(size_t)chunk_cap * 12 * 4},
-      b_bins{(size_t)chunk_cap * 3 * bins * 7 * 4}, b_cnt{(size_t)chunk_cap * 2 * 4};
+  Part b_lo{(size_t)n * 16}, b_hi{(size_t)n * 16}, b_cz{(size_t)n * 4}, b_tri0{(size_t)n * 4}, b_tri1{(size_t)n * 4},
+      b_tri2{(size_t)n * 4}, b_P{(size_t)n * 4}, b_Q{(size_t)n * 4}, b_recs{(size_t)nrec * 32},
+      b_parent{(size_t)nrec * 4}, b_arrived{(size_t)nrec * 4}, b_inner{(size_t)nrec * 4}, b_height{(size_t)nrec * 4},
+      b_ctr{kCtrBuild * 4}, b_small{(size_t)n * sizeof(Task)}, b_bins{big_cap * words * 4},
+      b_bits{(size_t)chunk_cap * kChunk / 8}, b_count{(size_t)chunk_cap * sizeof(uint2)};
+  Part b_big[2], b_box[2], b_chunk[2];
+  TempBuffer scratch, ref;
   {
-    Part* all[] = {&b_lo, &b_hi, &b_cz, &b_tri, &b_tmp, &b_P, &b_Q, &b_recs, &b_ctr, &b_small, &b_bigA,
-                   &b_bigB, &b_info, &b_chunks, &b_first, &b_part, &b_bins, &b_cnt};
+    for (int k = 0; k < 2; k++) {
+      b_big[k].bytes = (size_t)big_cap * sizeof(Big);
+      b_box[k].bytes = (size_t)big_cap * 48;
+      b_chunk[k].bytes = (size_t)chunk_cap * sizeof(Chunk);
+    }
+    Part* all[] = {&b_lo, &b_hi, &b_cz, &b_tri0, &b_tri1, &b_tri2, &b_P, &b_Q, &b_recs, &b_parent, &b_arrived, &b_inner,
+                   &b_height, &b_ctr, &b_small, &b_bins, &b_bits, &b_count, &b_big[0], &b_big[1], &b_box[0], &b_box[1],
+                   &b_chunk[0], &b_chunk[1]};
     size_t total = 0;
     for (Part* p : all) total += (p->bytes + 255) & ~(size_t)255;
-    BB_TRY(scratch.reserve(total, s));
+    if ((st = scratch.reserve(total, s))) return st;
     char* at = (char*)scratch.ptr;
     for (Part* p : all) {
       p->ptr = at;
       at += (p->bytes + 255) & ~(size_t)255;
     }
   }
+  auto done = [&](lucent_status code) {
+    ref.release();
+    scratch.release();
+    return code;
+  };
+#define BB_CUDA(x, what)                                      \
+  do {                                                        \
+    cudaError_t e_ = (x);                                     \
+    if (e_ != cudaSuccess) return done(cuda_fail(e_, what));  \
+  } while (0)
 
-  uint32_t* ctr = (uint32_t*)b_ctr.ptr;  // [0] rec_count [1] small_count [2] big_next_count [3] err
   Ctx cx;
   cx.p = {(const float4*)b_lo.ptr, (const float4*)b_hi.ptr, (const float*)b_cz.ptr};
-  cx.tri = (uint32_t*)b_tri.ptr;
-  cx.tmp = (uint32_t*)b_tmp.ptr;
+  cx.tri[0] = (uint32_t*)b_tri0.ptr;
+  cx.tri[1] = (uint32_t*)b_tri1.ptr;
+  cx.tri[2] = (uint32_t*)b_tri2.ptr;
+  cx.recs = (float4*)b_recs.ptr;
+  cx.parent = (uint32_t*)b_parent.ptr;
+  cx.ctr = (uint32_t*)b_ctr.ptr;
+  cx.small = (Task*)b_small.ptr;
+  for (int k = 0; k < 2; k++) {
+    cx.big[k] = (Big*)b_big[k].ptr;
+    cx.box[k] = (unsigned*)b_box[k].ptr;
+    cx.chunk[k] = (Chunk*)b_chunk[k].ptr;
+  }
+  cx.bins = (unsigned*)b_bins.ptr;
+  cx.bits = (unsigned*)b_bits.ptr;
+  cx.count = (uint2*)b_count.ptr;
   cx.P = (int32_t*)b_P.ptr;
   cx.Q = (int32_t*)b_Q.ptr;
-  cx.recs = (NodeRec*)b_recs.ptr;
-  cx.rec_count = ctr;
-  cx.small = (Task*)b_small.ptr;
-  cx.small_count = ctr + 1;
-  cx.big_next_count = ctr + 2;
-  cx.err = ctr + 3;
-  cx.cap = cap;
+  cx.n = n;
+  cx.big_cap = big_cap;
+  cx.chunk_cap = chunk_cap;
   cx.rec_cap = nrec;
   cx.max_leaf = max_leaf;
-  cx.bins = bins;
+  cx.nbins = bins;
 
-  bb_prim_bounds(pos_d, n, (float4*)b_lo.ptr, (float4*)b_hi.ptr, (float*)b_cz.ptr, cx.tri, s);
-  const Task root = {0, n, 0, 0};
-  uint32_t init[4] = {1, 0, 0, 0};
-  Task* big_cur = (Task*)b_bigA.ptr;
-  Task* big_nxt = (Task*)b_bigB.ptr;
-  uint32_t nbig = 0;
-  if (n <= small_max) {
-    init[1] = 1;
-    BB_CUDA(cudaMemcpyAsync(cx.small, &root, sizeof(Task), cudaMemcpyHostToDevice, s), "upload root");
+  BB_CUDA(cudaMemsetAsync(cx.ctr, 0, kCtrBuild * 4, s), "clear counters");
+  BB_CUDA(cudaMemsetAsync(cx.recs, 0xff, (size_t)nrec * 32, s), "clear nodes");
+  BB_CUDA(cudaMemsetAsync(cx.parent, 0, (char*)b_height.ptr + b_height.bytes - (char*)b_parent.ptr, s), "clear tree");
+  k_init<<<1, 32, 0, s>>>(cx);
+  k_prim_bounds<<<std::min<uint32_t>((n + 255) / 256, 152 * 8), 256, 0, s>>>(pos_d, cx, (float4*)b_lo.ptr,
+                                                                             (float4*)b_hi.ptr, (float*)b_cz.ptr);
+  uint32_t got[kCtrBuild] = {0};
+  int p = 0;
+  if (n > kSub) {
+    k_clear_bins<<<std::min<uint32_t>((uint32_t)(big_cap * words + 255) / 256, 152 * 8), 256, 0, s>>>(cx.bins, big_cap * words);
+    // Two levels more than halving would take, then a few at a time until no
+    // big node is left; a level of no nodes costs five empty launches.
+    int levels = 3;
+    while ((n >> (levels - 2)) > (uint32_t)kSub) levels++;
+    for (int total = 0;; levels = 3) {
+      if ((total += levels) > 8192) return done(fail(LUCENT_ERR_DEVICE, "BVH build did not converge"));
+      for (int k = 0; k < levels; k++, p ^= 1) {
+        k_big_bins<<<chunk_cap, 256, words * 4, s>>>(cx, p);
+        k_big_sah<<<(big_cap + 3) / 4, 128, 4 * words * 4, s>>>(cx, p);
+        k_big_count<<<chunk_cap, 256, 0, s>>>(cx, p);
+        k_big_place<<<chunk_cap, 256, 0, s>>>(cx, p);
+        k_big_move<<<chunk_cap, 256, 0, s>>>(cx, p);
+      }
+      BB_CUDA(cudaMemcpyAsync(got, cx.ctr, sizeof got, cudaMemcpyDeviceToHost, s), "read counters");
+      BB_CUDA(cudaStreamSynchronize(s), "big levels");
+      if (got[kErrW]) return done(fail(LUCENT_ERR_DEVICE, "BVH build raised device error 0x%x", got[kErrW]));
+      if (got[kNBig + p] == 0) break;
+    }
   } else {
-    nbig = 1;
-    BB_CUDA(cudaMemcpyAsync(big_cur, &root, sizeof(Task), cudaMemcpyHostToDevice, s), "upload root");
+    got[kNSmall] = 1;
   }
-  BB_CUDA(cudaMemcpyAsync(ctr, init, sizeof init, cudaMemcpyHostToDevice, s), "init counters");
-
-  std::vector<Task> tasks_h;
-  std::vector<Chunk> chunks_h;
-  std::vector<uint32_t> first_h;
-  int guard = 0;
-  while (nbig > 0) {
-    if (++guard > 4096) {
-      release_all();
-      return fail(LUCENT_ERR_DEVICE, "BVH build did not converge");
-    }
-    tasks_h.resize(nbig);
-    BB_CUDA(cudaMemcpyAsync(tasks_h.data(), big_cur, nbig * sizeof(Task), cudaMemcpyDeviceToHost, s), "read tasks");
-    BB_CUDA(cudaStreamSynchronize(s), "sync tasks");
-    chunks_h.clear();
-    first_h.assign(nbig + 1, 0);
-    for (uint32_t t = 0; t < nbig; t++) {
-      first_h[t] = (uint32_t)chunks_h.size();
-      for (uint32_t b = tasks_h[t].start; b < tasks_h[t].end; b += kChunk)
-        chunks_h.push_back({t, b, std::min(tasks_h[t].end, b + (uint32_t)kChunk), 0});
-    }
-    first_h[nbig] = (uint32_t)chunks_h.size();
-    const uint32_t nch = (uint32_t)chunks_h.size();
-    if (nbig > big_cap || nch > chunk_cap) {
-      release_all();
-      return fail(LUCENT_ERR_DEVICE, "task list overflow");
-    }
-    BB_CUDA(cudaMemcpyAsync(b_chunks.ptr, chunks_h.data(), nch * sizeof(Chunk), cudaMemcpyHostToDevice, s), "chunks");
-    BB_CUDA(cudaMemcpyAsync(b_first.ptr, first_h.data(), (nbig + 1) * 4, cudaMemcpyHostToDevice, s), "chunk index");
-    BB_CUDA(cudaMemsetAsync(cx.big_next_count, 0, 4, s), "reset next");
-    cx.big_next = big_nxt;
-    const Chunk* ch = (const Chunk*)b_chunks.ptr;
-    const uint32_t* fi = (const uint32_t*)b_first.ptr;
-    BigInfo* info = (BigInfo*)b_info.ptr;
-    k_big_measure<<<nch, 256, 0, s>>>(cx, ch, (float*)b_part.ptr);
-    k_big_setup<<<(nbig * 32 + 127) / 128, 128, 0, s>>>(cx, big_cur, nbig, fi, (const float*)b_part.ptr, info);
-    k_big_bins<<<nch, 256, 0, s>>>(cx, ch, info, (unsigned*)b_bins.ptr);
-    k_big_sah<<<(nbig + 3) / 4, 128, 0, s>>>(cx, big_cur, nbig, fi, (const unsigned*)b_bins.ptr, info);
-    k_big_count<<<nch, 256, 0, s>>>(cx, ch, big_cur, info, (uint32_t*)b_cnt.ptr);
-    k_big_scan<<<(nbig + 127) / 128, 128, 0, s>>>(big_cur, nbig, fi, (uint32_t*)b_cnt.ptr, info, cx.err);
-    k_big_place<<<nch, 256, 0, s>>>(cx, ch, big_cur, info, (const uint32_t*)b_cnt.ptr, 0);
-    k_big_place<<<nch, 256, 0, s>>>(cx, ch, big_cur, info, (const uint32_t*)b_cnt.ptr, 1);
-    k_big_copyback<<<nch, 256, 0, s>>>(cx, ch, info);
-    k_big_finish<<<(nbig + 127) / 128, 128, 0, s>>>(cx, big_cur, nbig, info, small_max);
-    BB_CUDA(cudaGetLastError(), "big-node kernels");
-    BB_CUDA(cudaMemcpyAsync(&nbig, cx.big_next_count, 4, cudaMemcpyDeviceToHost, s), "read next count");
-    BB_CUDA(cudaStreamSynchronize(s), "sync level");
-    if (nbig > cap) {
-      release_all();
-      return fail(LUCENT_ERR_DEVICE, "task list overflow");
-    }
-    std::swap(big_cur, big_nxt);
-  }
-  // Small nodes level by level: the tasks of a level are processed by one
-  // warp each, their children form the next level. Two task lists alternate
-  // (the small list and a big-node list, free by now) with their counts in
-  // ctr[1] and ctr[2]; the host checks for an empty level every 8 levels.
-  {
-    Task* lv[2] = {cx.small, big_nxt};
-    uint32_t* lc[2] = {cx.small_count, cx.big_next_count};
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int g = 8 * (sms > 0 ? sms : 152);
-    int cur = 0;
-    for (int level = 0;; level++) {
-      if (level >= 4096) {
-        release_all();
-        return fail(LUCENT_ERR_DEVICE, "BVH build did not converge");
-      }
-      if (level % 8 == 0) {  // any task left in the current level?
-        uint32_t left = 0;
-        BB_CUDA(cudaMemcpyAsync(&left, lc[cur], 4, cudaMemcpyDeviceToHost, s), "read small count");
-        BB_CUDA(cudaStreamSynchronize(s), "sync small count");
-        if (left == 0) break;
-      }
-      BB_CUDA(cudaMemsetAsync(lc[cur ^ 1], 0, 4, s), "reset small count");
-      k_small_level<<<g, 128, 0, s>>>(cx, lv[cur], lc[cur], lv[cur ^ 1], lc[cur ^ 1]);
-      BB_CUDA(cudaGetLastError(), "small-level kernel");
-      cur ^= 1;
-    }
-  }
-  uint32_t ctr_h[4];
-  BB_CUDA(cudaMemcpyAsync(ctr_h, ctr, sizeof ctr_h, cudaMemcpyDeviceToHost, s), "read counters");
+  if (got[kNSmall] > n) return done(fail(LUCENT_ERR_DEVICE, "task list overflow"));
+  // Subtrees that all run at once take 16 warps each, as the launch lasts as
+  // long as one of them (2,503 triangles, whole build: 367 us against 416 with
+  // 8; 82,000: 651 against 703); more of them 8 (2,000,000: 3.80 ms against
+  // 3.94). Subtrees of 512 or 2,048 triangles measured slower at both ends.
+  const int threads = got[kNSmall] <= 3 * 152 ? kSubThreads : kSubThreads / 2;
+  const size_t smem = sub_bytes(bins, threads);
+  BB_CUDA(cudaFuncSetAttribute((const void*)k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+          "shared memory of the subtree kernel");
+  if (got[kNSmall]) k_subtree<<<got[kNSmall], threads, smem, s>>>(cx);
+  const int g = (int)((nrec + 127) / 128);
+  uint32_t* inner = (uint32_t*)b_inner.ptr;
+  uint32_t* height = (uint32_t*)b_height.ptr;
+  k_tree_counts<<<g, 128, 0, s>>>(cx, (uint32_t*)b_arrived.ptr, inner, height, nrec);
+  uint32_t root[2];
+  float box[8];
+  BB_CUDA(cudaMemcpyAsync(got, cx.ctr, sizeof got, cudaMemcpyDeviceToHost, s), "read counters");
+  BB_CUDA(cudaMemcpyAsync(&root[0], inner, 4, cudaMemcpyDeviceToHost, s), "read node count");
+  BB_CUDA(cudaMemcpyAsync(&root[1], height, 4, cudaMemcpyDeviceToHost, s), "read depth");
+  BB_CUDA(cudaMemcpyAsync(box, cx.recs, 32, cudaMemcpyDeviceToHost, s), "read root");
   BB_CUDA(cudaStreamSynchronize(s), "build");
-  if (ctr_h[3]) {
-    release_all();
-    return fail(LUCENT_ERR_DEVICE, "BVH build raised device error 0x%x", ctr_h[3]);
-  }
-  const uint32_t nr = ctr_h[0];
-  if (nr > nrec || (nr & 1) == 0) {
-    release_all();
-    return fail(LUCENT_ERR_DEVICE, "BVH build produced %u nodes", nr);
-  }
-  std::vector<NodeRec> recs(nr);
-  BB_CUDA(cudaMemcpyAsync(recs.data(), cx.recs, nr * sizeof(NodeRec), cudaMemcpyDeviceToHost, s), "read nodes");
-  BB_CUDA(cudaMemcpyAsync(tri_out.data(), cx.tri, (size_t)n * 4, cudaMemcpyDeviceToHost, s), "read triIndices");
-  BB_CUDA(cudaStreamSynchronize(s), "read results");
-
-  // Inner-node counts bottom-up (children always have larger temporary ids),
-  // then DFS-preorder ranks top-down: left = parent + 1, right = parent + 1 +
-  // inner nodes of the left subtree; children of rank k get ids 2k+1, 2k+2.
-  std::vector<uint32_t> ic(nr, 0), rank(nr, 0), fid(nr, 0);
-  for (uint32_t x = 0; x < nr; x++) {  // children are allocated after their parent, in pairs
-    const NodeRec& r = recs[x];
-    if (r.left >= 0 && (r.left <= (int32_t)x || r.right != r.left + 1 || (uint32_t)r.right >= nr)) {
-      release_all();
-      return fail(LUCENT_ERR_DEVICE, "BVH build produced a malformed node %u", x);
-    }
-  }
-  for (int64_t x = (int64_t)nr - 1; x >= 0; x--)
-    if (recs[x].left >= 0) ic[x] = 1 + ic[recs[x].left] + ic[recs[x].right];
-  nodes_ref.assign((size_t)nr * 8, 0.f);
-  for (uint32_t x = 0; x < nr; x++) {
-    const NodeRec& r = recs[x];
-    float* o = nodes_ref.data() + (size_t)fid[x] * 8;
-    o[0] = r.lo[0], o[1] = r.lo[1], o[2] = r.lo[2];
-    o[4] = r.hi[0], o[5] = r.hi[1], o[6] = r.hi[2];
-    if (r.left >= 0) {
-      const uint32_t k = rank[x];
-      rank[r.left] = k + 1;
-      rank[r.right] = k + 1 + ic[r.left];
-      fid[r.left] = 2 * k + 1;
-      fid[r.right] = 2 * k + 2;
-      o[3] = (float)(2 * k + 1);
-      o[7] = 0.f;
-    } else {
-      o[3] = (float)r.first;
-      o[7] = (float)r.count;
-    }
-  }
+  if (got[kErrW]) return done(fail(LUCENT_ERR_DEVICE, "BVH build raised device error 0x%x", got[kErrW]));
+  const uint32_t nr = 2 * root[0] + 1;
+  if (nr > nrec) return done(fail(LUCENT_ERR_DEVICE, "BVH build produced %u nodes", nr));
+  out.node_count = nr;
+  out.depth = root[1];
   for (int k = 0; k < 3; k++) {  // bvh.ts:245-251: measure(0, triCount) = the root's box
-    bounds[k] = recs[0].lo[k];
-    bounds[3 + k] = recs[0].hi[k];
+    out.bounds[k] = box[k];
+    out.bounds[3 + k] = box[4 + k];
   }
-  if (nodes_dev || tris_dev) {
-    TempBuffer ref;
-    BB_TRY(ref.reserve((size_t)nr * 32, s));
-    cudaError_t e = cudaMemcpyAsync(ref.ptr, nodes_ref.data(), (size_t)nr * 32, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && nodes_dev) {
-      st = nodes_dev->reserve((size_t)nr * sizeof(Node));
-      if (!st) launch_pack_nodes((const float*)ref.ptr, nr, (Node*)nodes_dev->ptr, s);
-    }
-    if (e == cudaSuccess && !st && tris_dev) {
-      st = tris_dev->reserve((size_t)n * 48);
-      if (!st) launch_gather_tris(pos_d, cx.tri, n, (float4*)tris_dev->ptr, s);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    ref.release();
-    if (e != cudaSuccess) {
-      release_all();
-      return cuda_fail(e, "pack built BVH");
-    }
-    if (st) {
-      release_all();
-      return st;
-    }
-  }
-  release_all();
-  return LUCENT_OK;
-#undef BB_TRY
+  if ((out.nodes && (st = out.nodes->reserve((size_t)nr * sizeof(Node)))) ||
+      (out.tris && (st = out.tris->reserve((size_t)n * 48))) || (out.order && (st = out.order->reserve((size_t)n * 4))) ||
+      (out.nodes_host && (st = ref.reserve((size_t)nr * 32, s))))
+    return done(st);
+  k_tree_emit<<<g, 128, 0, s>>>(cx, inner, nrec, out.nodes ? (float4*)out.nodes->ptr : nullptr, (float4*)ref.ptr);
+  if (out.tris) launch_gather_tris(pos_d, cx.tri[2], n, (float4*)out.tris->ptr, s);
+  if (out.order)
+    BB_CUDA(cudaMemcpyAsync(out.order->ptr, cx.tri[2], (size_t)n * 4, cudaMemcpyDeviceToDevice, s), "copy order");
+  BB_CUDA(cudaGetLastError(), "build kernels");
+  if (out.nodes_host)
+    BB_CUDA(cudaMemcpyAsync(out.nodes_host, ref.ptr, (size_t)nr * 32, cudaMemcpyDeviceToHost, s), "read nodes");
+  if (out.tri_host)
+    BB_CUDA(cudaMemcpyAsync(out.tri_host, cx.tri[2], (size_t)n * 4, cudaMemcpyDeviceToHost, s), "read triIndices");
+  BB_CUDA(cudaStreamSynchronize(s), "pack built BVH");
+  return done(LUCENT_OK);
 #undef BB_CUDA
 }
 

@@ -63,8 +63,18 @@ lucent_status build_texture_layers(const uint8_t* const* images, const uint32_t*
 void env_grid(uint32_t w, uint32_t h, uint32_t max_w, uint32_t& gw, uint32_t& gh);
 lucent_status gpu_env_sampler(const float* rgb_d, uint32_t w, uint32_t h, uint32_t max_w, uint32_t& gw, uint32_t& gh,
                               float4* table_d, double& total, cudaStream_t s);
-lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bins, cudaStream_t s,
-                            std::vector<float>& nodes_ref, std::vector<uint32_t>& tri_out, double bounds[6],
-                            DeviceBuffer* nodes_dev, DeviceBuffer* tris_dev);
+// What a build returns: node count, depth and bounds always; the device layout
+// (Node array, slot-order triangles, triIndices) and the reference's arrays on
+// the host (8 floats a node, n indices) where given.
+struct BuildOut {
+  DeviceBuffer* nodes = nullptr;
+  DeviceBuffer* tris = nullptr;
+  DeviceBuffer* order = nullptr;
+  float* nodes_host = nullptr;
+  uint32_t* tri_host = nullptr;
+  uint32_t node_count = 0, depth = 0;
+  double bounds[6] = {0, 0, 0, 0, 0, 0};
+};
+lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bins, cudaStream_t s, BuildOut& out);
 
 }  // namespace lucent

@@ -774,31 +774,38 @@ lucent_status lucent_renderer_load_scene(lucent_renderer* r, const lucent_scene_
   if (d->uvs && (st = upload(uvs, d->uvs, (size_t)n * 24))) return cleanup(st);
   if (d->tri_light && (st = upload(lgt, d->tri_light, (size_t)n * 4))) return cleanup(st);
   if (d->tri_alpha && (st = upload(alp, d->tri_alpha, (size_t)n))) return cleanup(st);
-  std::vector<float> ref;
-  std::vector<uint32_t> tri;
-  double bounds[6];
+  uint32_t nc, depth;
+  float root[6];
   if (d->bvh_nodes) {
-    ref.assign(d->bvh_nodes, d->bvh_nodes + (size_t)d->bvh_node_count * 8);
-    tri.assign(d->bvh_tri_indices, d->bvh_tri_indices + n);
+    nc = d->bvh_node_count;
+    depth = tree_depth(d->bvh_nodes, nc, n);
+    for (int k = 0; k < 3; k++) {
+      root[k] = d->bvh_nodes[k];
+      root[3 + k] = d->bvh_nodes[4 + k];
+    }
     DeviceBuffer rb;
-    if ((st = upload(rb, ref.data(), ref.size() * 4)) || (st = r->nodes.reserve((size_t)d->bvh_node_count * 32))) {
+    if ((st = upload(rb, d->bvh_nodes, (size_t)nc * 32)) || (st = r->nodes.reserve((size_t)nc * 32)) ||
+        (st = upload(idx, d->bvh_tri_indices, (size_t)n * 4))) {
       rb.release();
       return cleanup(st);
     }
-    launch_pack_nodes((const float*)rb.ptr, d->bvh_node_count, (Node*)r->nodes.ptr, s);
+    launch_pack_nodes((const float*)rb.ptr, nc, (Node*)r->nodes.ptr, s);
     cudaStreamSynchronize(s);
     rb.release();
   } else {
-    if ((st = gpu_build_bvh((const float*)pos.ptr, n, 4, 12, s, ref, tri, bounds, &r->nodes, nullptr)))
-      return cleanup(st);
+    BuildOut out;
+    out.nodes = &r->nodes;
+    out.order = &idx;
+    if ((st = gpu_build_bvh((const float*)pos.ptr, n, 4, 12, s, out))) return cleanup(st);
+    nc = out.node_count;
+    depth = out.depth;
+    for (int k = 0; k < 6; k++) root[k] = (float)out.bounds[k];
   }
-  const uint32_t nc = (uint32_t)(ref.size() / 8);
-  if (tree_depth(ref.data(), nc, n) + 2 > kTsStack)
+  if (depth + 2 > kTsStack)
     return cleanup(fail(LUCENT_ERR_UNSUPPORTED, "BVH deeper than the reference's 64-entry traversal stack"));
   if ((st = r->wide.reserve((size_t)nc * 4 * sizeof(Node)))) return cleanup(st);
   launch_wide_view((const Node*)r->nodes.ptr, nc, (Node*)r->wide.ptr, s);
-  if ((st = upload(idx, tri.data(), (size_t)n * 4)) || (st = r->geo.reserve((size_t)(n ? n : 1) * 48)) ||
-      (st = r->attr.reserve((size_t)(n ? n : 1) * 64)))
+  if ((st = r->geo.reserve((size_t)(n ? n : 1) * 48)) || (st = r->attr.reserve((size_t)(n ? n : 1) * 64)))
     return cleanup(st);
   if (n)
     k_pack_scene<<<grid_for(n, 256), 256, 0, s>>>((const float*)pos.ptr, (const float*)nrm.ptr,
@@ -827,7 +834,7 @@ lucent_status lucent_renderer_load_scene(lucent_renderer* r, const lucent_scene_
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cleanup(cuda_fail(e, "scene upload"));
   if ((st = load_textures(r, d, s)) ||
-      (st = build_near_view((const Node*)r->nodes.ptr, nc, (const float4*)r->geo.ptr, n, ref.data(), ref.data() + 4,
+      (st = build_near_view((const Node*)r->nodes.ptr, nc, (const float4*)r->geo.ptr, n, root, root + 3,
                             r->near, s)))
     return cleanup(st);
   r->node_count = nc;
