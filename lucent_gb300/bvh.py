@@ -145,7 +145,7 @@ def build_bvh(positions, max_leaf_size=4, bins=12, stream=None) -> BVH:
     if pos.size % 9:
         raise ValueError("positions length %d is not a multiple of 9" % pos.size)  # bvh.ts:55-57
     n = pos.size // 9
-    nodes = np.zeros(max(1, 2 * n - 1) * NODE_STRIDE, np.float32)
+    nodes = np.empty(max(1, 2 * n - 1) * NODE_STRIDE, np.float32)  # room for the most nodes; only those built are touched
     tri = np.zeros(max(n, 1), np.uint32)
     cnt = C.c_uint32()
     bounds = np.zeros(6, np.float64)
@@ -155,7 +155,7 @@ def build_bvh(positions, max_leaf_size=4, bins=12, stream=None) -> BVH:
                                      C.byref(cnt), N.ptr(tri, C.c_uint32), N.ptr(bounds, C.c_double), C.byref(h),
                                      stream))
     nc = cnt.value
-    b = BVH(nodes[: nc * NODE_STRIDE].copy(), nc, tri[:n].copy(), AABB(bounds[:3], bounds[3:]))
+    b = BVH(nodes[: nc * NODE_STRIDE], nc, tri[:n], AABB(bounds[:3], bounds[3:]))
     b._device = _wrap_handle(h, nc, n)
     return b
 

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
+#include <stdint.h>
 
 #include "../../include/lucent.h"
 
@@ -10,6 +11,9 @@ namespace lucent {
 lucent_status fail(lucent_status code, const char* fmt, ...);
 lucent_status cuda_fail(cudaError_t e, const char* what);
 void clear_error();
+
+// Index of the first infinity or NaN in v[0 .. n - 1], or n.
+uint64_t first_not_finite(const float* v, uint64_t n);
 
 // A growable device allocation owned by a handle.
 struct DeviceBuffer {

@@ -5,6 +5,14 @@
 
 namespace lucent {
 
+// Writes to every page of a host buffer that a copy from the device is about to
+// fill: a copy into pages that were never touched faults them one by one from
+// the device's side (6 MB into a fresh allocation: 6 ms; touched first, 0.2).
+static void touch_pages(void* p, size_t bytes) {
+  for (size_t i = 0; i < bytes; i += 4096) ((volatile char*)p)[i] = 0;
+  if (bytes) ((volatile char*)p)[bytes - 1] = 0;
+}
+
 // Builds the BVH of `n` triangles at `pos_d` (device, 9 floats each); `out`
 // says what is wanted. Before this form (a launch per step and level with the
 // host reading each level's nodes, one warp walking each small node out of L2,
@@ -172,6 +180,8 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
   if (out.order)
     BB_CUDA(cudaMemcpyAsync(out.order->ptr, cx.tri[2], (size_t)n * 4, cudaMemcpyDeviceToDevice, s), "copy order");
   BB_CUDA(cudaGetLastError(), "build kernels");
+  if (out.nodes_host) touch_pages(out.nodes_host, (size_t)nr * 32);
+  if (out.tri_host) touch_pages(out.tri_host, (size_t)n * 4);
   if (out.nodes_host)
     BB_CUDA(cudaMemcpyAsync(out.nodes_host, ref.ptr, (size_t)nr * 32, cudaMemcpyDeviceToHost, s), "read nodes");
   if (out.tri_host)

@@ -754,8 +754,8 @@ lucent_status lucent_renderer_load_scene(lucent_renderer* r, const lucent_scene_
       return fail(LUCENT_ERR_INVALID, "sphere %u has light %d", i, d->sphere_lights[i]);
   }
   if (d->ground_material >= (int32_t)M) return fail(LUCENT_ERR_INVALID, "ground material %d", d->ground_material);
-  for (uint64_t i = 0; i < (uint64_t)n * 9; i++)
-    if (!std::isfinite(d->positions[i])) return fail(LUCENT_ERR_UNSUPPORTED, "positions[%llu] is not finite", (unsigned long long)i);
+  if (const uint64_t i = first_not_finite(d->positions, (uint64_t)n * 9); i < (uint64_t)n * 9)
+    return fail(LUCENT_ERR_UNSUPPORTED, "positions[%llu] is not finite", (unsigned long long)i);
   if (d->bvh_nodes) {
     if (!d->bvh_tri_indices) return fail(LUCENT_ERR_INVALID, "prebuilt BVH without triIndices");
     lucent_status st = validate_bvh(d->bvh_nodes, d->bvh_node_count, d->bvh_tri_indices, n);
