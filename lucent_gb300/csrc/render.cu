@@ -425,16 +425,31 @@ static __device__ __forceinline__ float4 hit_values(const float4* __restrict__ g
 // textured-hit queue untouched, so untextured shading carries none of the
 // texture code; the TEX launch then shades exactly those paths. Which
 // instantiation shades a hit depends on the hit alone, never on the launch,
-// so a scene renders the same alone and in a batch. Four blocks of 128 per
-// SM: 128 registers a thread, no spills (measured faster than five blocks
-// at 96 registers with spills, and than six).
+// so a scene renders the same alone and in a batch.
+//
+// Bound by instruction fetch: warps that drift apart over the kernel's code
+// evict one another's instructions (ncu at bounce 1 of the box frame, without
+// waiting: 5.4 warps a cycle wait for instructions, 4.1 for memory, issue
+// slots 26 % busy). So a block's warps wait for one another before each path.
+// Shade time per box frame (512 x 512 x 16) and per 1080p x 4 frame of layered,
+// glass and blended materials: 128 threads x 4 blocks an SM without waiting
+// 2.79 and 6.87 ms, with 2.42 and 5.37; 256 x 2 2.30 and 4.26; 512 x 1 2.37
+// and 3.56, 640 x 1 (96 registers) 2.42 and 3.64. Waves of 2^21 paths and more
+// take blocks of 512, smaller ones 256: half the threads of a 512-block idle
+// where it is the last of its SM (641 x 359 previews: 1.8 % slower with 512).
+// 128 registers a thread, no spills in the forward kernel.
+constexpr int kShadeThreads = 512;  // at most
+static int shade_threads(uint32_t paths) { return paths >= (1u << 21) ? kShadeThreads : kShadeThreads / 2; }
 template <class Src, bool ADJ = false, bool TEX = false>
-__global__ void __launch_bounds__(128, 4) k_shade_t(Paths P, const __grid_constant__ Src src, int cur, int bounce,
+__global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __grid_constant__ Src src, int cur, int bounce,
                                                     const __grid_constant__ AdjointDev A = AdjointDev{}) {
   const uint32_t n = TEX ? P.ctr[kCtrTex] : P.ctr[kCtrQ0 + cur];
   const uint32_t* q = P.q[cur];
   uint32_t* qn = P.q[cur ^ 1];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+  for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < n; k0 += gridDim.x * blockDim.x) {
+    __syncthreads();
+    const uint32_t k = k0 + threadIdx.x;
+    if (k >= n) continue;
     const uint32_t kq = TEX ? P.qtex[k] : k;  // position in queue `cur`, which also indexes the hits
     const uint32_t p = q[kq];
     const SceneDev& S = src.scene(p);
@@ -1252,8 +1267,10 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
   k_camera_multi<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, M.recs, M.path_base, M.n, M.sid, M.S);
   nl++;
   E.mark(kPhCamera, s);
-  static const int max_shade = persistent_blocks((const void*)k_shade_t<SceneTable>, 128);
-  const int shade_blocks = M.shade_blocks > 0 ? M.shade_blocks : max_shade;
+  static const int max_shade[2] = {persistent_blocks((const void*)k_shade_t<SceneTable>, kShadeThreads / 2),
+                                   persistent_blocks((const void*)k_shade_t<SceneTable>, kShadeThreads)};
+  const int shade_t = shade_threads(M.total_paths);
+  const int shade_blocks = M.shade_blocks > 0 ? M.shade_blocks : max_shade[shade_t == kShadeThreads];
   const int aux = M.shade_blocks > 0 ? M.shade_blocks : aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
   bool sorted = false;  // the rays of this bounce are in the sorted stream
@@ -1284,8 +1301,8 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
       k_zero_shade_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
       nl++;
     }
-    k_shade_t<SceneTable><<<shade_blocks, 128, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b);
-    if (M.any_tex) k_shade_t<SceneTable, false, true><<<shade_blocks, 128, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b);
+    k_shade_t<SceneTable><<<shade_blocks, shade_t, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b);
+    if (M.any_tex) k_shade_t<SceneTable, false, true><<<shade_blocks, shade_t, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b);
     nl += 1 + (M.any_tex != 0);
     E.mark(kPhShade, s);
     // This bounce's shadow rays do not depend on the next bounce's ray sort
@@ -1354,7 +1371,9 @@ int accumulate_wave(const MultiLaunch& M, cudaStream_t s) {
 // then propagating dl through every vertex.
 void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t s) {
   const SceneRec* rec = M.recs;
-  static const int shade_blocks = persistent_blocks((const void*)k_shade_t<SceneTable, true>, 128);
+  static const int max_shade[2] = {persistent_blocks((const void*)k_shade_t<SceneTable, true>, kShadeThreads / 2),
+                                   persistent_blocks((const void*)k_shade_t<SceneTable, true>, kShadeThreads)};
+  const int shade_t = shade_threads(M.total_paths), shade_blocks = max_shade[shade_t == kShadeThreads];
   const int aux = aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
   for (int pass = 0; pass < 2; pass++) {
@@ -1377,7 +1396,7 @@ void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t
         cudaStreamWaitEvent(s, M.ev_join, 0);
         k_zero_shade_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
       }
-      k_shade_t<SceneTable, true><<<shade_blocks, 128, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b, A);
+      k_shade_t<SceneTable, true><<<shade_blocks, shade_t, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b, A);
       const bool fork = M.side && b < M.max_bounces;
       cudaStream_t t = s;
       if (fork) {
