@@ -166,7 +166,7 @@ struct lucent_bvh {
   // 64-entry stack take the all-binary64 path, which reproduces the overflow.
   uint32_t depth = 0;
   int mode = LUCENT_TRAVERSE_WIDE;
-  DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch, stage;
+  DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch, stage{nullptr, 0, true};
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // the root's box
   NearTree near;       // nearest-first view (LUCENT_TRAVERSE_WIDE, where usable), built on first use
   bool near_tried = false;
@@ -445,6 +445,13 @@ lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, ui
   return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "closest-hit launch");
 }
 
+static lucent_status device_error(unsigned word) {
+  if (word & kErrIterations) return fail(LUCENT_ERR_DEVICE, "traversal exceeded node_count steps (malformed BVH)");
+  if (word & kErrStack)
+    return fail(LUCENT_ERR_DEVICE, "traversal needed more than 64 stack entries (BVH too deep for the reference)");
+  return fail(LUCENT_ERR_DEVICE, "device error word 0x%x", word);
+}
+
 lucent_status lucent_bvh_check(lucent_bvh* b, void* stream) {
   clear_error();
   if (!b) return fail(LUCENT_ERR_INVALID, "null bvh");
@@ -457,10 +464,7 @@ lucent_status lucent_bvh_check(lucent_bvh* b, void* stream) {
   if (e != cudaSuccess) return cuda_fail(e, "read error word");
   if (word) {
     cudaMemset(b->scratch.ptr, 0, 4);
-    if (word & kErrIterations) return fail(LUCENT_ERR_DEVICE, "traversal exceeded node_count steps (malformed BVH)");
-    if (word & kErrStack)
-      return fail(LUCENT_ERR_DEVICE, "traversal needed more than 64 stack entries (BVH too deep for the reference)");
-    return fail(LUCENT_ERR_DEVICE, "device error word 0x%x", word);
+    return device_error(word);
   }
   return LUCENT_OK;
 }
@@ -511,6 +515,35 @@ lucent_status lucent_bvh_intersect_f64(lucent_bvh* b, const double* rays, uint32
   }
   cudaStream_t s = (cudaStream_t)stream;
   const size_t rb = (size_t)n * 48, ob = (size_t)n * 8;
+  // A warp per ray while all of them run at once (18 an SM); trees the
+  // reference's stack cannot walk keep the kernel that reproduces its overflow.
+  if (n <= 18 * 152 && b->depth + 2 <= kTsStack && b->mode != LUCENT_TRAVERSE_EXACT) {
+    const bool args = n <= kPickArgs;
+    const size_t hb = (size_t)n * sizeof(PickHit);
+    if ((st = b->stage.reserve(hb + (args ? 0 : rb)))) return st;
+    PickHit* hits_d = (PickHit*)b->stage.ptr;
+    double* rays_d = (double*)((char*)b->stage.ptr + hb);
+    cudaError_t e = args ? cudaSuccess : cudaMemcpyAsync(rays_d, rays, rb, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return cuda_fail(e, "upload rays");
+    launch_pick((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, args ? rays : rays_d, !args, n,
+                t_min, t_max, hits_d, s);
+    PickHit few[kPickArgs];
+    std::vector<PickHit> many(args ? 0 : n);
+    PickHit* hits = args ? few : many.data();
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hits, hits_d, hb, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(e, "f64 closest-hit");
+    unsigned word = 0;
+    for (uint32_t i = 0; i < n; i++) {
+      prim_out[i] = hits[i].prim;
+      t_out[i] = hits[i].t;
+      u_out[i] = hits[i].u;
+      v_out[i] = hits[i].v;
+      word |= hits[i].err;
+    }
+    return word ? device_error(word) : LUCENT_OK;
+  }
   if ((st = b->stage.reserve(rb + 4 * ob + 64))) return st;
   uint32_t *ctr, *queue;
   if ((st = prepare_scratch(b, 0, s, &ctr, &queue))) return st;

@@ -77,6 +77,160 @@ __global__ void k_closest_exact_d(TravArgs A, const double* __restrict__ rays, u
   }
 }
 
+// A few binary64 rays (picks), a warp each. One thread's walk is a chain of
+// dependent loads and binary64 tests, one pick into 81,920 triangles 200 to 650
+// us a call, 1,000 rays 1.9 to 3.0 ms (here: 100 us, and 0.17 to 0.2 ms, of which
+// the tree's depth in dependent steps is the most). The warp pops up to 32 pending nodes at a time and tests their
+// children, or a leaf's triangles, a lane each. Nothing is skipped for its
+// distance, so every triangle the reference could take is met; the answer is
+// the one of least t (lowest slot among equals) if the reference reaches it:
+// it visits a leaf iff every box on the way passes with the running closest
+// c, and c > t(w) until w is tested, so it takes w if the largest entry
+// distance on the way is at most t(w), or at least below the next t (the
+// argument of traverse_near.cuh, here over any tree, as each box is tested).
+// Rays with a zero or non-finite component (whose NaN slab decisions are not
+// monotone), pending nodes beyond the list, equal least t or an undecided
+// winner take one lane's walk in the reference's order instead.
+constexpr int kPickPending = 768;
+struct PickArgs {  // rays as kernel arguments: no copy to the device
+  double r[kPickArgs * 6];
+  __device__ const double* at(uint32_t k) const { return r + 6 * k; }
+};
+struct PickArray {
+  const double* r;
+  __device__ const double* at(uint32_t k) const { return r + 6 * (size_t)k; }
+};
+struct PendingBox {
+  double entry;  // largest entry distance on the way
+  int node;
+  int pad;
+};
+
+// AABB.intersect's test (ts_slab_culled) with the entry distance it computes.
+__device__ __forceinline__ bool slab_entry(const Node& nd, const double o[3], const double inv[3], double tMax,
+                                           double& entry) {
+  const double lo[3] = {(double)nd.lo.x, (double)nd.lo.y, (double)nd.lo.z};
+  const double hi[3] = {(double)nd.hi.x, (double)nd.hi.y, (double)nd.hi.z};
+  double tmin = 0, tmax = tMax;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double a = dmul(dsub(lo[i], o[i]), inv[i]), b = dmul(dsub(hi[i], o[i]), inv[i]);
+    const double t0 = a > b ? b : a, t1 = a > b ? a : b;
+    if (t0 > tmin) tmin = t0;
+    if (t1 < tmax) tmax = t1;
+  }
+  entry = tmin;
+  return !(tmax < tmin);
+}
+
+template <class Rays>
+__global__ void __launch_bounds__(32) k_pick(TravArgs A, const __grid_constant__ Rays rays, PickHit* __restrict__ out) {
+  __shared__ PendingBox list[kPickPending];
+  const int lane = threadIdx.x;
+  const uint32_t k = blockIdx.x;
+  const double* r = rays.at(k);
+  const double o[3] = {r[0], r[1], r[2]}, d[3] = {r[3], r[4], r[5]};
+  const double inv[3] = {ddiv(1.0, d[0]), ddiv(1.0, d[1]), ddiv(1.0, d[2])};
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < 3; i++) ok = ok && isfinite(o[i]) && isfinite(d[i]) && isfinite(inv[i]) && inv[i] != 0.0;
+  const double INF64 = __longlong_as_double(0x7ff0000000000000ll);
+  double bt = INF64, bu = 0, bv = 0, be = 0, second = INF64;  // this lane's least t, its entry distance, its next t
+  int bs = 0x7fffffff;
+  uint32_t n = 0, seen = 0;
+  if (ok) {
+    const Node root = load_node(A.nodes, 0);
+    double e;
+    if (slab_entry(root, o, inv, A.tMax, e)) {
+      if (lane == 0) list[0] = {e, 0, 0};
+      n = 1;
+    }
+  }
+  __syncwarp();
+  while (ok && n > 0) {
+    const uint32_t take = min(n, 32u);
+    seen += take;
+    const bool mine = lane < (int)take;
+    PendingBox it{};
+    if (mine) it = list[n - 1 - lane];
+    n -= take;
+    __syncwarp();
+    double e0 = 0, e1 = 0;
+    bool p0 = false, p1 = false;
+    int first = 0;
+    if (mine) {
+      const Node nd = load_node(A.nodes, it.node);
+      const int cnt = node_count(nd);
+      first = node_first(nd);
+      if (cnt == 0) {
+        const Node c0 = load_node(A.nodes, first), c1 = load_node(A.nodes, first + 1);
+        p0 = slab_entry(c0, o, inv, A.tMax, e0);
+        p1 = slab_entry(c1, o, inv, A.tMax, e1);
+      }
+      for (int q = 0; q < cnt; q++) {
+        const int s = first + q;
+        double t, u, v;
+        if (!ts_triangle({o[0], o[1], o[2]}, {d[0], d[1], d[2]}, d3f(__ldg(A.tris + 3 * (size_t)s)),
+                         d3f(__ldg(A.tris + 3 * (size_t)s + 1)), d3f(__ldg(A.tris + 3 * (size_t)s + 2)), A.tMin,
+                         A.tMax, t, u, v))
+          continue;
+        if (t < bt || (t == bt && s < bs)) {
+          second = bt;
+          bt = t, bu = u, bv = v, bs = s, be = it.entry;
+        } else if (t < second) {
+          second = t;
+        }
+      }
+    }
+    const unsigned m0 = __ballot_sync(0xffffffffu, p0), m1 = __ballot_sync(0xffffffffu, p1);
+    const unsigned lt = (1u << lane) - 1u;
+    const uint32_t push = __popc(m0) + __popc(m1);
+    ok = n + push <= kPickPending && seen <= A.node_limit;  // (a tree is walked once)
+    if (ok) {
+      if (p0) list[n + __popc(m0 & lt)] = {fmax(it.entry, e0), first, 0};
+      if (p1) list[n + __popc(m0) + __popc(m1 & lt)] = {fmax(it.entry, e1), first + 1, 0};
+    }
+    n += push;
+    __syncwarp();
+  }
+  // The warp's least (t, slot), then the least t of all the others.
+  double wt = bt;
+  int ws = bs;
+  for (int off = 16; off > 0; off >>= 1) {
+    const double t = __shfl_xor_sync(0xffffffffu, wt, off);
+    const int s = __shfl_xor_sync(0xffffffffu, ws, off);
+    if (t < wt || (t == wt && s < ws)) wt = t, ws = s;
+  }
+  double next = bs == ws ? second : bt;
+  for (int off = 16; off > 0; off >>= 1) next = fmin(next, __shfl_xor_sync(0xffffffffu, next, off));
+  const bool hit = ws != 0x7fffffff, winner = hit && bs == ws;
+  const double entry = __shfl_sync(0xffffffffu, be, hit ? __ffs(__ballot_sync(0xffffffffu, winner)) - 1 : 0);
+  ok = ok && (!hit || (wt < next && (entry <= wt || entry < next)));
+  PickHit h{INF64, 0, 0, -1, 0u};
+  if (ok) {
+    if (hit ? !winner : lane != 0) return;
+    if (hit) h = {bt, bu, bv, __float_as_int(__ldg(A.tris + 3 * (size_t)bs).w), 0u};
+  } else {
+    if (lane != 0) return;
+    __shared__ unsigned err;
+    err = 0;
+    int slot;
+    TravArgs B = A;
+    B.err = &err;
+    ApiPolicy P{};
+    if (!trace_exact(B, P, bvh_of(B, P, k), {o[0], o[1], o[2]}, {d[0], d[1], d[2]}, 0, slot, h.t, h.u, h.v)) {
+      h.prim = -2;
+    } else if (slot >= 0) {
+      h.prim = __float_as_int(__ldg(A.tris + 3 * (size_t)slot).w);
+    } else {
+      h.t = INF64;
+      h.u = h.v = 0;
+    }
+    h.err = err;
+  }
+  out[k] = h;
+}
+
 // The values of the hits the traversal found (prim = -3 - slot): the
 // reference's binary64 t, u, v rounded to binary32, from double-float
 // arithmetic where its bound proves the roundings of all three, else from
@@ -218,6 +372,19 @@ void launch_closest(const Node* nodes, uint32_t node_count, const float4* tris, 
 
 void launch_wide_view(const Node* nodes, uint32_t node_count, Node* wide, cudaStream_t s) {
   launch_build_wide(nodes, node_count, wide, s);
+}
+
+void launch_pick(const Node* nodes, uint32_t node_count, const float4* tris, const double* rays, bool on_device,
+                 uint32_t n, double tMin, double tMax, PickHit* out_d, cudaStream_t s) {
+  if (n == 0) return;
+  TravArgs A{nodes, node_count, tris, tMin, tMax, nullptr, nullptr, nullptr, nullptr};
+  if (on_device) {
+    k_pick<<<n, 32, 0, s>>>(A, PickArray{rays}, out_d);
+  } else {
+    PickArgs args{};
+    for (uint32_t i = 0; i < n * 6 && i < kPickArgs * 6; i++) args.r[i] = rays[i];
+    k_pick<<<n < kPickArgs ? n : kPickArgs, 32, 0, s>>>(A, args, out_d);
+  }
 }
 
 void launch_closest_d(const Node* nodes, uint32_t node_count, const float4* tris, const double* rays_d, uint32_t n,

@@ -26,6 +26,16 @@ void launch_closest(const Node* nodes, uint32_t node_count, const float4* tris, 
                     const NearTree* near = nullptr);
 // Four-wide view of a binary node array (traverse_wide.cuh): 4 records per node.
 void launch_wide_view(const Node* nodes, uint32_t node_count, Node* wide, cudaStream_t s);
+// A few binary64 rays, a warp each (closest_hit.cu): rays in host memory (at
+// most kPickArgs, passed by value) or on the device; results and error bits per ray.
+constexpr uint32_t kPickArgs = 32;
+struct PickHit {
+  double t, u, v;
+  int32_t prim;
+  unsigned err;
+};
+void launch_pick(const Node* nodes, uint32_t node_count, const float4* tris, const double* rays, bool on_device,
+                 uint32_t n, double tMin, double tMax, PickHit* out_d, cudaStream_t s);
 void launch_closest_d(const Node* nodes, uint32_t node_count, const float4* tris, const double* rays_d, uint32_t n, double tMin,
                       double tMax, int32_t* prim, double* t, double* u, double* v, unsigned* err, cudaStream_t s);
 

@@ -63,7 +63,7 @@ __global__ void k_near_parents(const Node* __restrict__ nodes, uint32_t n_nodes,
 // lower index, so every climb ends).
 __global__ void k_near_leaves(const Node* __restrict__ nodes, uint32_t n_nodes, const float4* __restrict__ tris,
                               float diag, const uint32_t* __restrict__ parent, uint32_t* __restrict__ arrived,
-                              Node* cull, uint32_t* __restrict__ leaf_of, uint32_t* __restrict__ words) {
+                              Node* cull, uint32_t* tail, uint32_t* __restrict__ leaf_of, uint32_t* __restrict__ words) {
   uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= n_nodes) return;
   const Node nd = load_node(nodes, n);
@@ -86,11 +86,13 @@ __global__ void k_near_leaves(const Node* __restrict__ nodes, uint32_t n_nodes, 
   Node c;
   c.lo = make_float4(__fsub_rd(nd.lo.x, g), __fsub_rd(nd.lo.y, g), __fsub_rd(nd.lo.z, g),
                      __int_as_float(kNearLeaf | f << 8 | (cnt & kNearMaxLeaf)));
-  c.hi = make_float4(__fadd_ru(nd.hi.x, g), __fadd_ru(nd.hi.y, g), __fadd_ru(nd.hi.z, g), nd.hi.w);
-  while (true) {
+  c.hi = make_float4(__fadd_ru(nd.hi.x, g), __fadd_ru(nd.hi.y, g), __fadd_ru(nd.hi.z, g), __int_as_float(f));
+  uint32_t end = (uint32_t)(f + cnt);
+  while (true) {  // (hi.w and `tail`: the subtree's slots, which have to be in the order the reference visits them)
     float4* p = reinterpret_cast<float4*>(cull) + 2 * (size_t)n;
     __stcg(p, c.lo);
     __stcg(p + 1, c.hi);
+    __stcg(tail + n, end);
     const uint32_t up = parent[n];
     if (up == 0) return;
     __threadfence();
@@ -101,7 +103,9 @@ __global__ void k_near_leaves(const Node* __restrict__ nodes, uint32_t n_nodes, 
     const float4* q = reinterpret_cast<const float4*>(cull) + 2 * (size_t)first;
     const float4 al = __ldcg(q), ah = __ldcg(q + 1), bl = __ldcg(q + 2), bh = __ldcg(q + 3);
     c.lo = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __int_as_float((int)n));
-    c.hi = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), __int_as_float(0));
+    c.hi = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), ah.w);
+    end = __ldcg(tail + first + 1);
+    if (__ldcg(tail + first) > (uint32_t)__float_as_int(bh.w)) atomicOr(words + kNearBad, 1u);
   }
 }
 
@@ -163,17 +167,18 @@ lucent_status build_near_view(const Node* nodes, uint32_t n_nodes, const float4*
     return st;
   TempBuffer tmp;
   const size_t cull = (size_t)n_nodes * sizeof(Node), idx = (size_t)n_nodes * 4;
-  if ((st = tmp.reserve(cull + 2 * idx + 64, s))) return st;
+  if ((st = tmp.reserve(cull + 3 * idx + 64, s))) return st;
   char* b = (char*)tmp.ptr;
   uint32_t* parent = (uint32_t*)(b + cull);
   uint32_t* arrived = parent + n_nodes;
   uint32_t* words = arrived + n_nodes;
+  uint32_t* tail = words + 16;
   uint32_t got[kNearWords] = {1, 0, 0};
   const int g = (int)((n_nodes + 127) / 128);
   cudaError_t e = cudaMemsetAsync(parent, 0, 2 * idx + kNearWords * 4, s);
   if (e == cudaSuccess) {
     k_near_parents<<<g, 128, 0, s>>>(nodes, n_nodes, parent, words);
-    k_near_leaves<<<g, 128, 0, s>>>(nodes, n_nodes, tris, diag, parent, arrived, (Node*)b,
+    k_near_leaves<<<g, 128, 0, s>>>(nodes, n_nodes, tris, diag, parent, arrived, (Node*)b, tail,
                                     (uint32_t*)out.leaf_of.ptr, words);
     k_near_records<<<g, 128, 0, s>>>(nodes, (const Node*)b, n_nodes, (Node*)out.records.ptr);
     e = cudaGetLastError();

@@ -44,11 +44,12 @@
 // bound for |d| <= 2 and origins within two diagonals of the tree's centre; for
 // farther ones it rises linearly with the distance, and the ray's boxes are
 // grown by the largest such rise of any triangle (NearTree::far), as long as
-// that is small against a leaf. Other rays go to the ordered kernel. A tree with many leaves whose
-// growth is not small against the scene (scenes in units far above 1, where
-// 1e-12 is no bound at all), with boxes that are not nested or do not hold
-// their triangles (caller-supplied trees), or with leaves of over 255
-// triangles is not traversed this way (NearTree::usable).
+// that is small against a leaf. Other rays go to the ordered kernel. A tree
+// with many leaves whose growth is not small against the scene (scenes in units
+// far above 1, where 1e-12 is no bound at all), with boxes that are not nested
+// or do not hold their triangles or slots out of visiting order
+// (caller-supplied trees), or with leaves of over 255 triangles is not
+// traversed this way (NearTree::usable).
 //
 // A record: (min.xyz, reference), (max.xyz, unused); the reference is the
 // binary index of an inner node or kNearLeaf | first slot << 8 | count. As in
