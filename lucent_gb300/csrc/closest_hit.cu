@@ -30,7 +30,8 @@ struct ApiPolicy {
   // Lanes of a wide-kernel warp that wait before it fetches new rays
   // (measured on 10^6 random rays into a 65,536-triangle soup: 4 over 1, 8, 16).
   static constexpr int kRefillMin = 4;
-    static constexpr int kNearThreads = 128, kNearBlocks = 8, kNearRefill = 4;
+    // (7 blocks, 72 registers: the soup's 10^6 rays 1.82 ms, 1.90 at 8 blocks)
+  static constexpr int kNearThreads = 128, kNearBlocks = 7, kNearRefill = 4;
   __device__ Node leaf_box(const TravArgs& A, int, int slot) const { return load_node(A.nodes, __ldg(A.leaf_of + slot)); }
   __device__ bool alpha(int, int, uint32_t, float, float) const { return true; }
   __device__ AlphaAnswer alpha_fast(int, int, uint32_t) const { return kAlphaBlock; }

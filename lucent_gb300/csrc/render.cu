@@ -50,8 +50,8 @@ struct PathClosestMulti {
   // stalls the warp on the atomic and the new rays' loads (path tracing's
   // short rays: 24 measured best of 1, 4, 8, 16, 24, 32).
   static constexpr int kRefillMin = 24;
-    // Nearest-first closest hit (box frame): 128 x 8 blocks 2.68 ms, x 7 2.75, x 6 and 256 x 3
-  // slower by 3 to 5 %; refills at 24 lanes 3.27 ms (before the batched expansions), 16 3.41, 8 3.73.
+    // Nearest-first closest hit: 8 blocks of 128 an SM (64 registers); 7 measured the same on the box
+  // frame and 0.5 % slower over 2 M triangles, 6 and 256 x 3 3 to 5 % slower.
   static constexpr int kNearThreads = 128, kNearBlocks = 8, kNearRefill = 24;
   __device__ uint32_t count() const { return *cnt; }
   __device__ uint32_t path(uint32_t k) const { return __float_as_uint(rays[2 * (size_t)k].w); }

@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks)
   const float cmax_lo = __double2float_rd(A.tMax), cmax_hi = __double2float_ru(A.tMax);
   const double INF64 = __longlong_as_double(0x7ff0000000000000ll);
   const uint32_t n = P.count();
+  if (Rest && n == 0) return;  // mostly
   const bool use_alpha = P.alpha_any();
 
   bool active = false, exhausted = false, have_cur = false, c_exact = true;

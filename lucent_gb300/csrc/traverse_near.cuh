@@ -66,17 +66,20 @@ constexpr int kNearMaxLeaf = 255;
 constexpr float kNearWindow = 1.0000153f;      // 1 + 2^-16
 constexpr float kNearSlack = 1.0000010f;       // 1 + 2^-20
 constexpr float kNearOiPad = 2.3841858e-07f;   // 2^-22
-// Expansions a lane makes before its warp tests triangles again: lanes that
-// reach a leaf wait for the others' boxes, so both phases run with more lanes.
-// Per 512 x 512 x 16 box frame, closest hit: one expansion at a time 3.27 ms,
-// 2 2.74, 3 2.75, 4 2.75, 6 3.02, until every lane has a leaf 2.73 (but the
-// 10^6 soup rays 2.13 against 1.97 ms at 3).
-constexpr int kNearSteps = 3;
-// Any hit: block shape, expansions per turn and lanes that wait before a
-// refill. Box frame's shadow rays, one ray per thread and no refill: 2.35 ms;
-// persistent: 1.57 at (128, 7), 4 expansions, 24 lanes; 8 blocks 1.63, 10
-// 1.72; 2 expansions 1.74, 8 1.60; 8 waiting lanes 1.65, 32 1.75.
-constexpr int kAnyThreads = 128, kAnyBlocks = 7, kAnySteps = 4, kAnyRefill = 24;
+// A warp tests boxes while a quarter of its lanes have some to test, then
+// triangles (one a lane and turn) the same way, at most kNearSteps turns each;
+// lanes whose ray is finished wait until a refill's worth of them write their
+// answers and fetch rays together. Closest hit per 512 x 512 x 16 box frame and
+// per 1080p x 4 frame over 2 M triangles: one box or leaf per lane and turn
+// 3.27 and 13.4 ms; three boxes, then whole leaves, answers where they fall
+// 2.70 and 10.4; in turns 2.40 and 9.4 (turns of 4 the same; ending below 12,
+// 16 or 20 lanes up to 2 % slower; the loops unrolled 3.4 and 12.4, by their
+// spills).
+constexpr int kNearSteps = 8;
+// Any hit: one ray per thread without refill 2.35 ms of the box frame; in turns,
+// with refills at 24 lanes: 1.57 at (128, 8), 7 blocks 1.62, 6 1.63; refill at
+// 16 1.60.
+constexpr int kAnyThreads = 128, kAnyBlocks = 8, kAnySteps = 8, kAnyRefill = 24;
 // Norm-based bound of mt_classify's absolute-value evaluations: 2^-19 x 6 max|a| max|b| max|c|.
 constexpr float kMtRel6 = 6.f * kMtRel;
 
@@ -215,18 +218,18 @@ LUCENT_DEV bool near_ray_ok(float3 o, float3 d, const NearView& v, float& grow) 
 }
 
 // Closest hit: persistent warps, one ray per lane, refilled as in
-// k_closest_wide_t. An expansion tests four boxes (16 operations each instead
+// k_closest_wide_t. A turn tests four boxes (16 operations each instead
 // of the 60 of a certain decision), sorts the hits by entry distance (the two
 // low bits of the distance carry the record number) and goes on with the
 // nearest. With few rays for the grid, a warp takes only as many as spread
 // them over all warps: fewer lanes in a warp diverge less, and a launch of few
 // rays lasts as long as its slowest warp.
-// Bound by divergence and instruction issue (ncu, bounce 1 of the box frame:
-// 11.5 of 32 lanes active, issue slots 65 % busy, L1 45 %, DRAM 2 %).
-// Against the ordered wide kernel: 4,099 rays into 20,480 triangles 284 -> 94
-// us a call, 10^6 rays into the 65,536-triangle soup 3.48 -> 1.97 ms, closest
-// hit of the box frame (11.8 M rays, 82 k triangles) 4.19 -> 2.70 ms, of a
-// 1080p 4-spp frame over 2 M triangles (14.7 M rays) 25.5 -> 10.4 ms.
+// Bound by divergence, instruction issue and node latency (ncu, bounce 1: some
+// 10 of 32 lanes active, issue slots 55 to 65 % busy, L1 45 to 52 %, DRAM 10 %).
+// Against the ordered wide kernel: 4,099 rays into 20,480 triangles 284 -> 89
+// us a call, 10^6 rays into the 65,536-triangle soup 3.48 -> 1.82 ms, closest
+// hit of the box frame (11.8 M rays, 82 k triangles) 4.19 -> 2.40 ms, of a
+// 1080p 4-spp frame over 2 M triangles (14.7 M rays) 25.5 -> 9.4 ms.
 template <class Pol>
 __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest_near_t(TravArgs A, const __grid_constant__ Pol P) {
   const unsigned FULL = 0xffffffffu;
@@ -238,9 +241,9 @@ __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest
   const bool use_alpha = P.alpha_any();
   const uint32_t warps = gridDim.x * (Pol::kNearThreads / 32);
   const int lanes = (int)min(32u, (n + warps - 1) / warps);
-  const int refill = min(Pol::kNearRefill, lanes);
+  const int refill = min(Pol::kNearRefill, lanes), turn = max(1, lanes / 4);
 
-  bool active = false, exhausted = lane >= lanes;
+  bool has = false, exhausted = lane >= lanes;  // has: a ray whose answer is not written yet
   uint32_t ri = 0, key = 0;
   Ray32 r;
   NearRay nr;
@@ -250,166 +253,169 @@ __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest
   if constexpr (!Pol::kMultiScene) bv = A.near;
   WidePending stack[kWideStack];
 
-  while (true) {
-    const bool need = !active && !exhausted;
-    const unsigned m = __ballot_sync(FULL, need);
-    if (m && (__popc(m) >= refill || __ballot_sync(FULL, active) == 0)) {
-      const int leader = __ffs(m) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(A.work, (uint32_t)__popc(m));
-      base = __shfl_sync(FULL, base, leader);
-      if (need) {
-        ri = base + __popc(m & lt);
-        if (ri >= n) {
-          exhausted = true;
-        } else {
-          float3 o, d;
-          P.ray(ri, o, d);
-          if constexpr (Pol::kMultiScene) bv = P.near_view(ri);
-          float grow;
-          if (!near_ray_ok(o, d, bv, grow)) {
-            A.queue[atomicAdd(A.queue_len, 1u)] = ri;
-          } else {
-            r = make_ray32(o, d);
-            nr = make_near_ray(r, grow);
-            md6 = kMtRel6 * fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
-            key = use_alpha ? P.key(ri) : 0u;
-            count_stat(A, 0);
-            c = cmax_hi;
-            best = -1;
-            pend = -1;
-            sp = 0;
-            ref = 0;
-            active = true;
-          }
-        }
-      }
+  auto pop = [&]() {
+    while (sp > 0) {
+      const WidePending e = stack[--sp];
+      if (e.ehi <= c) return e.rec;
     }
-    if (__all_sync(FULL, exhausted)) break;
-    if (!active) continue;
-
-    auto pop = [&]() {
-      while (sp > 0) {
-        const WidePending e = stack[--sp];
-        if (e.ehi <= c) return e.rec;
-      }
-      return kNearNone;
-    };
-    auto expand = [&]() {
-      const float4* rec = reinterpret_cast<const float4*>(bv.nodes) + (size_t)ref * (2 * kWide);
-      unsigned k[kWide];
-      int rf[kWide];
-#pragma unroll
-      for (int i = 0; i < kWide; i++) {
-        const float4 bl = __ldg(rec + 2 * i), bh = __ldg(rec + 2 * i + 1);
-        float e;
-        const bool hit = near_box(nr, bl, bh, c, e);
-        k[i] = hit ? (__float_as_uint(e) & ~3u) | (unsigned)i : 0xffffffffu;
-        rf[i] = __float_as_int(bl.w);
-      }
-      auto cas = [](unsigned& x, unsigned& y) {
-        const unsigned a = min(x, y), b = max(x, y);
-        x = a;
-        y = b;
-      };
-      cas(k[0], k[1]);
-      cas(k[2], k[3]);
-      cas(k[0], k[2]);
-      cas(k[1], k[3]);
-      cas(k[1], k[2]);
-      auto ref_of = [&](unsigned key4) {
-        const int a = key4 & 1u ? rf[1] : rf[0], b = key4 & 1u ? rf[3] : rf[2];
-        return key4 & 2u ? b : a;
-      };
-#pragma unroll
-      for (int i = kWide - 1; i > 0; i--)
-        if (k[i] != 0xffffffffu) stack[sp++] = {ref_of(k[i]), __uint_as_float(k[i] & ~3u)};
-      ref = k[0] != 0xffffffffu ? ref_of(k[0]) : kNearNone;
-    };
-
-    if (ref == kNearNone) {
-      ref = pop();
-      if (ref == kNearNone) {  // finished
-        active = false;
+    return kNearNone;
+  };
+  while (true) {
+    const unsigned wait = __ballot_sync(FULL, ref == kNearNone && (has || !exhausted));
+    const bool idle = __ballot_sync(FULL, ref != kNearNone) == 0;
+    if (__popc(wait) >= refill || idle) {
+      // The answers of the lanes that wait, together.
+      if (has && ref == kNearNone) {
+        has = false;
         if (best < 0) {
           P.miss(ri);
-          continue;
-        }
-        const bool tie = pend >= 0;
-        if (tie) {
-          count_stat(A, 3);
-          const NearBest b = near_tie(r.o, r.d, bv.tris, A.tMin, best, pend);
-          best = b.slot;
-          lo = b.lo;
-        }
-        const Node box = P.leaf_box(A, bv.scene, best);
-        float ehi;
-        const float INF32 = __int_as_float(0x7f800000);
-        const SlabClass cl = classify_slab_e(r, box.lo, box.hi, INF32, INF32, ehi);
-        bool ok = cl == kPass;
-        if (cl == kAmbiguous) {
-          count_stat(A, 1);
-          ok = near_leaf_passes(box.lo, box.hi, r.o, r.d, __longlong_as_double(0x7ff0000000000000ll));
-        }
-        ok = ok && (ehi <= lo || (!tie && ehi * kNearSlack <= c && ehi <= cmax_lo));
-        if (ok) P.finish(ri, best);
-        else A.queue[atomicAdd(A.queue_len, 1u)] = ri;
-        continue;
-      }
-    }
-
-    bool full = false;
-    for (int it = 0; it < kNearSteps && ref >= 0; it++) {
-      full = sp + 3 > kWideStack;  // unreachable for trees the reference's stack can traverse
-      if (full) break;
-      expand();
-      if (ref == kNearNone) ref = pop();
-    }
-    if (ref < 0) {
-      const int first = (ref & 0x7fffffff) >> 8, cnt = ref & 255;
-      for (int q = 0; q < cnt; q++) {
-        const int slot = first + q;
-        const float4* g = bv.tris + 3 * (size_t)slot;
-        float tl, th;
-        TriClass tc = mt_classify_near(r, md6, __ldg(g), __ldg(g + 1), __ldg(g + 2), tmin_lo, tmin_hi, c, tl, th);
-        if (tc == kTriReject) continue;
-        bool exact = tc == kTriExact || !(th < cmax_lo);
-        if (use_alpha) {
-          const AlphaAnswer aa = P.alpha_fast(bv.scene, slot, key);
-          if (aa == kAlphaPass) continue;
-          exact = exact || aa == kAlphaDefer;  // a textured alpha needs the binary64 barycentrics
-        }
-        if (exact) {
-          count_stat(A, 2);
-          if (!near_exact(P, bv.scene, key, use_alpha, r.o, r.d, bv.tris, slot, A.tMin, A.tMax, tl, th)) continue;
-        }
-        if (best < 0 || th * kNearWindow < lo) {
-          best = slot;
-          pend = -1;
-          lo = tl;
-          hi = th;
-        } else if (tl > hi * kNearWindow) {
-          continue;
-        } else {  // compared at the end, unless a nearer hit makes it moot
-          if (pend >= 0) {
+        } else {
+          const bool tie = pend >= 0;
+          if (tie) {
             count_stat(A, 3);
             const NearBest b = near_tie(r.o, r.d, bv.tris, A.tMin, best, pend);
             best = b.slot;
             lo = b.lo;
-            hi = b.hi;
           }
-          pend = slot;
-          lo = fminf(lo, tl);
-          hi = fminf(hi, th);
+          const Node box = P.leaf_box(A, bv.scene, best);
+          float ehi;
+          const float INF32 = __int_as_float(0x7f800000);
+          const SlabClass cl = classify_slab_e(r, box.lo, box.hi, INF32, INF32, ehi);
+          bool ok = cl == kPass;
+          if (cl == kAmbiguous) {
+            count_stat(A, 1);
+            ok = near_leaf_passes(box.lo, box.hi, r.o, r.d, __longlong_as_double(0x7ff0000000000000ll));
+          }
+          ok = ok && (ehi <= lo || (!tie && ehi * kNearSlack <= c && ehi <= cmax_lo));
+          if (ok) P.finish(ri, best);
+          else A.queue[atomicAdd(A.queue_len, 1u)] = ri;
         }
-        c = fminf(cmax_hi, hi * kNearWindow);
       }
-      ref = kNearNone;
+      const bool need = ref == kNearNone && !exhausted;
+      const unsigned m = __ballot_sync(FULL, need);
+      if (m) {
+        const int leader = __ffs(m) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(A.work, (uint32_t)__popc(m));
+        base = __shfl_sync(FULL, base, leader);
+        if (need) {
+          ri = base + __popc(m & lt);
+          if (ri >= n) {
+            exhausted = true;
+          } else {
+            float3 o, d;
+            P.ray(ri, o, d);
+            if constexpr (Pol::kMultiScene) bv = P.near_view(ri);
+            float grow;
+            if (!near_ray_ok(o, d, bv, grow)) {
+              A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+            } else {
+              r = make_ray32(o, d);
+              nr = make_near_ray(r, grow);
+              md6 = kMtRel6 * fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+              key = use_alpha ? P.key(ri) : 0u;
+              count_stat(A, 0);
+              c = cmax_hi;
+              best = -1;
+              pend = -1;
+              sp = 0;
+              ref = 0;
+              has = true;
+            }
+          }
+        }
+      }
+      if (__ballot_sync(FULL, has) == 0 && __all_sync(FULL, exhausted)) break;
     }
-    if (full) {
-      atomicOr(A.err, kErrStack);
-      P.fail(ri);
-      active = false;
+
+    // Boxes.
+#pragma unroll 1
+    for (int it = 0; it < kNearSteps; it++) {
+      if (ref >= 0) {
+        if (sp + 3 > kWideStack) {  // unreachable for trees the reference's stack can traverse
+          atomicOr(A.err, kErrStack);
+          P.fail(ri);
+          has = false;
+          ref = kNearNone;
+        } else {
+          const float4* rec = reinterpret_cast<const float4*>(bv.nodes) + (size_t)ref * (2 * kWide);
+          unsigned k[kWide];
+          int rf[kWide];
+#pragma unroll
+          for (int i = 0; i < kWide; i++) {
+            const float4 bl = __ldg(rec + 2 * i), bh = __ldg(rec + 2 * i + 1);
+            float e;
+            const bool hit = near_box(nr, bl, bh, c, e);
+            k[i] = hit ? (__float_as_uint(e) & ~3u) | (unsigned)i : 0xffffffffu;
+            rf[i] = __float_as_int(bl.w);
+          }
+          auto cas = [](unsigned& x, unsigned& y) {
+            const unsigned a = min(x, y), b = max(x, y);
+            x = a;
+            y = b;
+          };
+          cas(k[0], k[1]);
+          cas(k[2], k[3]);
+          cas(k[0], k[2]);
+          cas(k[1], k[3]);
+          cas(k[1], k[2]);
+          auto ref_of = [&](unsigned key4) {
+            const int a = key4 & 1u ? rf[1] : rf[0], b = key4 & 1u ? rf[3] : rf[2];
+            return key4 & 2u ? b : a;
+          };
+#pragma unroll
+          for (int i = kWide - 1; i > 0; i--)
+            if (k[i] != 0xffffffffu) stack[sp++] = {ref_of(k[i]), __uint_as_float(k[i] & ~3u)};
+          ref = k[0] != 0xffffffffu ? ref_of(k[0]) : pop();
+        }
+      }
+      if (__popc(__ballot_sync(FULL, ref >= 0)) < turn) break;
+    }
+    // Triangles, one a lane and turn: the reference counts down to the next.
+#pragma unroll 1
+    for (int it = 0; it < kNearSteps; it++) {
+      if (ref < 0 && (ref & 255)) {
+        const int slot = (ref & 0x7fffffff) >> 8;
+        ref += 255;  // first + 1, count - 1
+        const float4* g = bv.tris + 3 * (size_t)slot;
+        float tl, th;
+        const TriClass tc = mt_classify_near(r, md6, __ldg(g), __ldg(g + 1), __ldg(g + 2), tmin_lo, tmin_hi, c, tl, th);
+        bool take = tc != kTriReject;
+        if (take) {
+          bool exact = tc == kTriExact || !(th < cmax_lo);
+          if (use_alpha) {
+            const AlphaAnswer aa = P.alpha_fast(bv.scene, slot, key);
+            take = aa != kAlphaPass;
+            exact = exact || aa == kAlphaDefer;  // a textured alpha needs the binary64 barycentrics
+          }
+          if (take && exact) {
+            count_stat(A, 2);
+            take = near_exact(P, bv.scene, key, use_alpha, r.o, r.d, bv.tris, slot, A.tMin, A.tMax, tl, th);
+          }
+        }
+        if (take) {
+          if (best < 0 || th * kNearWindow < lo) {
+            best = slot;
+            pend = -1;
+            lo = tl;
+            hi = th;
+          } else if (!(tl > hi * kNearWindow)) {  // compared at the end, unless a nearer hit makes it moot
+            if (pend >= 0) {
+              count_stat(A, 3);
+              const NearBest b = near_tie(r.o, r.d, bv.tris, A.tMin, best, pend);
+              best = b.slot;
+              lo = b.lo;
+              hi = b.hi;
+            }
+            pend = slot;
+            lo = fminf(lo, tl);
+            hi = fminf(hi, th);
+          }
+          c = fminf(cmax_hi, hi * kNearWindow);
+        }
+        if (!(ref & 255)) ref = pop();
+      }
+      if (__popc(__ballot_sync(FULL, ref < 0 && (ref & 255))) < turn) break;
     }
   }
 }
@@ -429,9 +435,9 @@ __global__ void __launch_bounds__(kAnyThreads, kAnyBlocks) k_anyhit_near_t(TravA
   const bool use_alpha = P.alpha_any();
   const uint32_t warps = gridDim.x * (kAnyThreads / 32);
   const int lanes = (int)min(32u, (n + warps - 1) / warps);
-  const int refill = min(kAnyRefill, lanes);
+  const int refill = min(kAnyRefill, lanes), turn = max(1, lanes / 4);
 
-  bool active = false, exhausted = lane >= lanes;
+  bool exhausted = lane >= lanes;
   uint32_t ri = 0, key = 0;
   Ray32 r;
   NearRay nr;
@@ -440,9 +446,9 @@ __global__ void __launch_bounds__(kAnyThreads, kAnyBlocks) k_anyhit_near_t(TravA
   NearView bv = A.near;
   int stack[kWideStack];
   while (true) {
-    const bool need = !active && !exhausted;
+    const bool need = ref == kNearNone && !exhausted;
     const unsigned m = __ballot_sync(FULL, need);
-    if (m && (__popc(m) >= refill || __ballot_sync(FULL, active) == 0)) {
+    if (m && (__popc(m) >= refill || __ballot_sync(FULL, ref != kNearNone) == 0)) {
       const int leader = __ffs(m) - 1;
       uint32_t base = 0;
       if (lane == leader) base = atomicAdd(A.work, (uint32_t)__popc(m));
@@ -465,57 +471,68 @@ __global__ void __launch_bounds__(kAnyThreads, kAnyBlocks) k_anyhit_near_t(TravA
             tmax = P.tmax32(ri);
             sp = 0;
             ref = 0;
-            active = true;
           }
         }
       }
     }
-    if (__all_sync(FULL, exhausted)) break;
-    if (!active) continue;
-    bool full = false, occ = false;
-    const float c = tmax * kNearSlack;
-    for (int it = 0; it < kAnySteps && ref >= 0; it++) {
-      full = sp + 3 > kWideStack;  // unreachable for trees the reference's stack can traverse
-      if (full) break;
-      const float4* rec = reinterpret_cast<const float4*>(bv.nodes) + (size_t)ref * (2 * kWide);
-      ref = kNearNone;
+    if (__all_sync(FULL, exhausted && ref == kNearNone)) break;
+#pragma unroll 1
+    for (int it = 0; it < kAnySteps; it++) {
+      if (ref >= 0) {
+        if (sp + 3 > kWideStack) {  // unreachable for trees the reference's stack can traverse
+          atomicOr(A.err, kErrStack);
+          P.shadow(ri, true);
+          ref = kNearNone;
+        } else {
+          const float4* rec = reinterpret_cast<const float4*>(bv.nodes) + (size_t)ref * (2 * kWide);
+          const float c = tmax * kNearSlack;
+          ref = kNearNone;
 #pragma unroll
-      for (int i = 0; i < kWide; i++) {
-        const float4 bl = __ldg(rec + 2 * i), bh = __ldg(rec + 2 * i + 1);
-        float e;
-        if (!near_box(nr, bl, bh, c, e)) continue;
-        if (ref != kNearNone) stack[sp++] = ref;
-        ref = __float_as_int(bl.w);
+          for (int i = 0; i < kWide; i++) {
+            const float4 bl = __ldg(rec + 2 * i), bh = __ldg(rec + 2 * i + 1);
+            float e;
+            if (!near_box(nr, bl, bh, c, e)) continue;
+            if (ref != kNearNone) stack[sp++] = ref;
+            ref = __float_as_int(bl.w);
+          }
+          if (ref == kNearNone && sp > 0) ref = stack[--sp];
+        }
       }
-      if (ref == kNearNone && sp > 0) ref = stack[--sp];
+      if (__popc(__ballot_sync(FULL, ref >= 0)) < turn) break;
     }
-    if (ref < 0 && !full) {
-      const int first = (ref & 0x7fffffff) >> 8, cnt = ref & 255;
-      for (int q = 0; q < cnt && !occ; q++) {
-        const int slot = first + q;
+#pragma unroll 1
+    for (int it = 0; it < kAnySteps; it++) {
+      if (ref < 0 && (ref & 255)) {
+        const int slot = (ref & 0x7fffffff) >> 8;
+        ref += 255;  // first + 1, count - 1
         const float4* g = bv.tris + 3 * (size_t)slot;
         float tl, th;
         const TriClass tc =
             mt_classify_near(r, md6, __ldg(g), __ldg(g + 1), __ldg(g + 2), tmin_lo, tmin_hi, tmax, tl, th);
-        if (tc == kTriReject) continue;
-        bool exact = tc == kTriExact || !(th < tmax);
-        if (use_alpha) {
-          const AlphaAnswer aa = P.alpha_fast(bv.scene, slot, key);
-          if (aa == kAlphaPass) continue;
-          exact = exact || aa == kAlphaDefer;
+        bool take = tc != kTriReject;
+        if (take) {
+          bool exact = tc == kTriExact || !(th < tmax);
+          if (use_alpha) {
+            const AlphaAnswer aa = P.alpha_fast(bv.scene, slot, key);
+            take = aa != kAlphaPass;
+            exact = exact || aa == kAlphaDefer;
+          }
+          if (take && exact)
+            take = near_exact(P, bv.scene, key, use_alpha, r.o, r.d, bv.tris, slot, A.tMin, (double)tmax, tl, th);
+          if (take) {
+            const Node box = P.leaf_box(A, bv.scene, slot);
+            const SlabClass cl = classify_slab(r, box.lo, box.hi, tmax, tmax);
+            take = cl == kPass || (cl == kAmbiguous && near_leaf_passes(box.lo, box.hi, r.o, r.d, (double)tmax));
+          }
         }
-        if (exact && !near_exact(P, bv.scene, key, use_alpha, r.o, r.d, bv.tris, slot, A.tMin, (double)tmax, tl, th))
-          continue;
-        const Node box = P.leaf_box(A, bv.scene, slot);
-        const SlabClass cl = classify_slab(r, box.lo, box.hi, tmax, tmax);
-        occ = cl == kPass || (cl == kAmbiguous && near_leaf_passes(box.lo, box.hi, r.o, r.d, (double)tmax));
+        if (take) {
+          P.shadow(ri, true);  // unoccluded rays need no answer
+          ref = kNearNone;
+        } else if (!(ref & 255)) {
+          ref = sp > 0 ? stack[--sp] : kNearNone;
+        }
       }
-      ref = sp > 0 ? stack[--sp] : kNearNone;
-    }
-    if (full) atomicOr(A.err, kErrStack);
-    if (full || occ || ref == kNearNone) {
-      P.shadow(ri, full || occ);
-      active = false;
+      if (__popc(__ballot_sync(FULL, ref < 0 && (ref & 255))) < turn) break;
     }
   }
 }

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks)
   const float cmax_lo = __double2float_rd(A.tMax), cmax_hi = __double2float_ru(A.tMax);
   const float INF32 = __int_as_float(0x7f800000);
   const uint32_t n = P.count();
+  if (Rest && n == 0) return;  // mostly
   const bool use_alpha = P.alpha_any();
 
   bool active = false, exhausted = false, have_cur = false, cond = false;
