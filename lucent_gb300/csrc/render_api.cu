@@ -1128,7 +1128,8 @@ lucent_status lucent_renderer_backward(lucent_renderer* r, uint32_t samples, uin
   if (e != cudaSuccess) return cuda_fail(e, "backward setup");
   float4* base = (float4*)r->adj_path.ptr;
   AdjointDevHost H{(const float4*)r->adj_dl.ptr, base, base + cap, base + 6 * cap, base + 12 * cap,
-                   (float*)r->adj_grad.ptr, nenv ? (float*)r->adj_grad.ptr + env_off : nullptr};
+                   (float*)r->adj_grad.ptr, nenv ? (float*)r->adj_grad.ptr + env_off : nullptr,
+                   (int)scene_owner(r)->material_count};
   for (uint32_t done = 0; done < samples; done += batch) {
     const uint32_t S = std::min(batch, samples - done);
     MultiLaunch M{};

@@ -165,6 +165,7 @@ struct AdjointDevHost {
   float4 *lrem, *gcont, *gslot, *genv;
   float* dmat;
   float* denv;  // environment texel gradients, 4 floats (RGB, pad) per texel, 16-byte aligned
+  int materials;  // of the scene: dmat holds 6 floats each
 };
 // Gradient of sum_px dl[px] . (mean of the wave's samples) with respect to
 // material parameters (6 per material) and environment texels, for a launch
