@@ -120,7 +120,8 @@ __global__ void k_near_records(const Node* __restrict__ nodes, const Node* __res
   const float inf = __int_as_float(0x7f800000);
   Node rec[kWide];
 #pragma unroll
-  for (int k = 0; k < kWide; k++) rec[k] = {make_float4(inf, inf, inf, 0.f), make_float4(-inf, -inf, -inf, 0.f)};
+  for (int k = 0; k < kWide; k++)  // unused: an inverted box, a leaf of no triangles
+    rec[k] = {make_float4(inf, inf, inf, __int_as_float(kNearNone)), make_float4(-inf, -inf, -inf, 0.f)};
   if (node_count(nd) > 0) {
     rec[0] = load_node(cull, n);
   } else {

@@ -54,7 +54,8 @@
 // A record: (min.xyz, reference), (max.xyz, unused); the reference is the
 // binary index of an inner node or kNearLeaf | first slot << 8 | count. As in
 // the four-wide view, records 4 n .. 4 n + 3 are the grandchildren of binary
-// node n, a leaf child standing in for its own.
+// node n, a leaf child standing in for its own (opening the child of largest
+// surface twice instead measured the same within 1 %).
 #pragma once
 #include "traverse_wide.cuh"
 
@@ -76,6 +77,10 @@ constexpr float kNearOiPad = 2.3841858e-07f;   // 2^-22
 // 16 or 20 lanes up to 2 % slower; the loops unrolled 3.4 and 12.4, by their
 // spills).
 constexpr int kNearSteps = 8;
+// Turns a warp takes at most between two refills; its rays are then handed to
+// the ordered kernels (which count their own steps). A tree is walked once per
+// ray, so this ends nothing sooner than a scene of many overlapping boxes.
+constexpr uint32_t kNearTurns = 1u << 20;
 // Any hit: one ray per thread without refill 2.35 ms of the box frame; in turns,
 // with refills at 24 lanes: 1.57 at (128, 8), 7 blocks 1.62, 6 1.63; refill at
 // 16 1.60.
@@ -252,6 +257,7 @@ __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest
   NearView bv{};
   if constexpr (!Pol::kMultiScene) bv = A.near;
   WidePending stack[kWideStack];
+  uint32_t turns = 0;
 
   auto pop = [&]() {
     while (sp > 0) {
@@ -263,7 +269,13 @@ __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest
   while (true) {
     const unsigned wait = __ballot_sync(FULL, ref == kNearNone && (has || !exhausted));
     const bool idle = __ballot_sync(FULL, ref != kNearNone) == 0;
+    if (++turns > kNearTurns && ref != kNearNone) {
+      A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+      has = false;
+      ref = kNearNone;
+    }
     if (__popc(wait) >= refill || idle) {
+      turns = 0;
       // The answers of the lanes that wait, together.
       if (has && ref == kNearNone) {
         has = false;
@@ -333,8 +345,7 @@ __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest
     for (int it = 0; it < kNearSteps; it++) {
       if (ref >= 0) {
         if (sp + 3 > kWideStack) {  // unreachable for trees the reference's stack can traverse
-          atomicOr(A.err, kErrStack);
-          P.fail(ri);
+          A.queue[atomicAdd(A.queue_len, 1u)] = ri;
           has = false;
           ref = kNearNone;
         } else {
@@ -445,10 +456,16 @@ __global__ void __launch_bounds__(kAnyThreads, kAnyBlocks) k_anyhit_near_t(TravA
   int sp = 0, ref = kNearNone;
   NearView bv = A.near;
   int stack[kWideStack];
+  uint32_t turns = 0;
   while (true) {
+    if (++turns > kNearTurns && ref != kNearNone) {
+      A.queue[atomicAdd(A.queue_len, 1u)] = ri;
+      ref = kNearNone;
+    }
     const bool need = ref == kNearNone && !exhausted;
     const unsigned m = __ballot_sync(FULL, need);
     if (m && (__popc(m) >= refill || __ballot_sync(FULL, ref != kNearNone) == 0)) {
+      turns = 0;
       const int leader = __ffs(m) - 1;
       uint32_t base = 0;
       if (lane == leader) base = atomicAdd(A.work, (uint32_t)__popc(m));
@@ -479,9 +496,8 @@ __global__ void __launch_bounds__(kAnyThreads, kAnyBlocks) k_anyhit_near_t(TravA
 #pragma unroll 1
     for (int it = 0; it < kAnySteps; it++) {
       if (ref >= 0) {
-        if (sp + 3 > kWideStack) {  // unreachable for trees the reference's stack can traverse
-          atomicOr(A.err, kErrStack);
-          P.shadow(ri, true);
+        if (sp + 3 > kWideStack) {  // unreachable, as above
+          A.queue[atomicAdd(A.queue_len, 1u)] = ri;
           ref = kNearNone;
         } else {
           const float4* rec = reinterpret_cast<const float4*>(bv.nodes) + (size_t)ref * (2 * kWide);
