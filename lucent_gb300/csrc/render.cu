@@ -50,7 +50,7 @@ struct PathClosestMulti {
   // stalls the warp on the atomic and the new rays' loads (path tracing's
   // short rays: 24 measured best of 1, 4, 8, 16, 24, 32).
   static constexpr int kRefillMin = 24;
-    // Nearest-first closest hit: 8 blocks of 128 an SM (64 registers); 7 measured the same on the box
+  // Nearest-first closest hit: 8 blocks of 128 an SM (64 registers); 7 measured the same on the box
   // frame and 0.5 % slower over 2 M triangles, 6 and 256 x 3 3 to 5 % slower.
   static constexpr int kNearThreads = 128, kNearBlocks = 8, kNearRefill = 24;
   __device__ uint32_t count() const { return *cnt; }
@@ -89,6 +89,13 @@ struct PathClosestMulti {
   }
   __device__ void miss(uint32_t k) const { hits[k] = make_float4(INF, 0.f, 0.f, __int_as_float(-1)); }
   __device__ void fail(uint32_t k) const { miss(k); }
+};
+
+// The same for a wave of one scene, whose view comes with the launch: no
+// lookup per ray, and its pointers in uniform registers (nearest-first only).
+struct PathClosestOne : PathClosestMulti {
+  static constexpr bool kMultiScene = false;
+  __device__ Node leaf_box(const TravArgs& A, int, int slot) const { return load_node(A.nodes, __ldg(A.leaf_of + slot)); }
 };
 
 struct PathShadowMulti {
@@ -133,6 +140,11 @@ struct PathShadowMulti {
   __device__ void shadow(uint32_t k, bool occluded) const {
     if (occluded) sh_c[queue[k]].w = 0.f;
   }
+};
+
+struct PathShadowOne : PathShadowMulti {
+  static constexpr bool kMultiScene = false;
+  __device__ Node leaf_box(const TravArgs& A, int, int slot) const { return load_node(A.nodes, __ldg(A.leaf_of + slot)); }
 };
 
 // ------------------------------------------------------------ kernels
@@ -1236,6 +1248,15 @@ static const TraversalGrids& traversal_grids() {
   return g;
 }
 
+// A with the one scene's view of a single-scene wave.
+static TravArgs one_scene(const MultiLaunch& M, TravArgs A) {
+  const SceneDev& S = M.scene;
+  A.nodes = S.nodes;
+  A.leaf_of = S.leaf_of;
+  A.near = {S.near, S.geo, 0, S.near_bound, S.near_far};
+  return A;
+}
+
 // Closest hit of a bounce: nearest first, then the rays that could not be
 // proven in the reference's order; or all rays in that order, over the scenes'
 // four-wide BVH views or the binary nodes with the top levels staged in shared
@@ -1245,7 +1266,11 @@ static void launch_closest_multi(const MultiLaunch& M, const Paths& P, const Tra
   const TraversalGrids& G = traversal_grids();
   const int own = M.trace_blocks;
   if (M.near) {
-    k_closest_near_t<PathClosestMulti><<<own > 0 ? own : G.near, PathClosestMulti::kNearThreads, 0, s>>>(A, pc);
+    const int g = own > 0 ? own : G.near;
+    if (M.n == 1)
+      k_closest_near_t<PathClosestOne><<<g, PathClosestOne::kNearThreads, 0, s>>>(one_scene(M, A), PathClosestOne{pc});
+    else
+      k_closest_near_t<PathClosestMulti><<<g, PathClosestMulti::kNearThreads, 0, s>>>(A, pc);
     TravArgs R = A;
     R.work = P.ctr + kCtrRestWork;
     using Listed = Queued<PathClosestMulti>;
@@ -1263,7 +1288,9 @@ static void launch_closest_multi(const MultiLaunch& M, const Paths& P, const Tra
 static void launch_shadow_multi(const MultiLaunch& M, int blocks, const TravArgs& A, const PathShadowMulti& ps,
                                 cudaStream_t s) {
   const TraversalGrids& G = traversal_grids();
-  if (M.near)
+  if (M.near && M.n == 1)
+    k_anyhit_near_t<PathShadowOne><<<G.any, kAnyThreads, 0, s>>>(one_scene(M, A), PathShadowOne{ps});
+  else if (M.near)
     k_anyhit_near_t<PathShadowMulti><<<G.any, kAnyThreads, 0, s>>>(A, ps);
   else if (M.wide)
     k_anyhit_wide_t<PathShadowMulti><<<blocks, 256, 0, s>>>(A, ps);

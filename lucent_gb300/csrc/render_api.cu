@@ -180,7 +180,7 @@ void sheen_lut_half(float* out) {
 struct WaveGraph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  uint64_t key[4] = {0, 0, 0, 0};
+  uint64_t key[5] = {0, 0, 0, 0, 0};
   cudaStream_t cap = nullptr;
   int launches = 0;  // kernels in the captured wave
   void drop() {
@@ -194,7 +194,7 @@ struct WaveGraph {
     if (cap) cudaStreamDestroy(cap);
     cap = nullptr;
   }
-  lucent_status run(const MultiLaunch& M, const uint64_t k[4], cudaStream_t s, bool accumulate = true) {
+  lucent_status run(const MultiLaunch& M, const uint64_t k[5], cudaStream_t s, bool accumulate = true) {
     cudaError_t e;
     if (!exec || std::memcmp(k, key, sizeof key) != 0) {
       drop();
@@ -299,7 +299,7 @@ struct WaveSet {
 };
 
 // Everything a captured wave bakes in besides the buffer contents.
-static void wave_key(const MultiLaunch& M, uint64_t key[4]) {
+static void wave_key(const MultiLaunch& M, uint64_t key[5]) {
   key[0] = (uint64_t)(uint32_t)M.S | ((uint64_t)(uint32_t)M.n << 32);
   key[1] = (uint64_t)M.total_pixels | ((uint64_t)(uint32_t)M.trace_blocks << 32) ^ ((uint64_t)M.sort_classes << 48);
   key[2] = ((uint64_t)(uintptr_t)M.paths.rec) ^ ((uint64_t)M.max_bounces << 48) ^ ((uint64_t)M.shade_blocks << 56);
@@ -307,6 +307,19 @@ static void wave_key(const MultiLaunch& M, uint64_t key[4]) {
            ((uint64_t)M.near << 56) ^ ((uint64_t)(M.side != nullptr) << 57) ^ ((uint64_t)M.wide << 58) ^ ((uint64_t)M.any_tex << 60) ^ ((uint64_t)M.sort_rays << 61) ^
            ((uint64_t)M.top_levels << 62) ^
            ((uint64_t)(M.trav_stats != nullptr) << 63);
+  key[4] = 0;
+  if (M.n == 1 && M.near) {  // the scene's view is part of the launch
+    const sh::SceneDev& S = M.scene;
+    const float f[6] = {S.near_bound.x, S.near_bound.y, S.near_bound.z, S.near_bound.w, S.near_far.x, S.near_far.y};
+    const void* ptrs[4] = {S.nodes, S.geo, S.near, S.leaf_of};
+    auto mix = [&](uint64_t v) { key[4] = (key[4] ^ v) * 0x9e3779b97f4a7c15ull + (key[4] >> 29); };
+    for (const void* p : ptrs) mix((uint64_t)(uintptr_t)p);
+    for (float x : f) {
+      uint32_t w;
+      std::memcpy(&w, &x, 4);
+      mix(w);
+    }
+  }
 }
 
 struct lucent_renderer {
@@ -600,6 +613,7 @@ static lucent_status single_launch(lucent_renderer* r, WaveSet& w, uint32_t S, u
   M.pix_base = M.path_base + 2;
   M.sid = (uint16_t*)w.sid.ptr;
   M.n = 1;
+  M.scene = rec.scene;
   M.S = (int)S;
   M.max_bounces = (int)r->max_bounces;
   M.total_paths = WH * S;
@@ -1027,7 +1041,7 @@ lucent_status lucent_renderer_trace(lucent_renderer* r, uint32_t samples, void* 
       if (w == 0) cudaEventRecord(r->ev0, X.stream);
       // The first wave ever runs uncaptured (one-time setup).
       if (w < full && r->waves > 0) {
-        uint64_t key[4];
+        uint64_t key[5];
         wave_key(M, key);
         key[0] |= 1ull << 63;  // captured without the accumulation
         if ((st = X.graph.run(M, key, X.stream, false))) return st;
@@ -1048,7 +1062,7 @@ lucent_status lucent_renderer_trace(lucent_renderer* r, uint32_t samples, void* 
     M.trav_stats = r->trav_counters ? (unsigned long long*)((uint32_t*)X.ctr.ptr + kCtrTrav) : nullptr;
     cudaEventRecord(r->ev0, s);
     PhaseEvents pe{r->pev.data(), r->ptag.data(), (int)r->pev.size(), 0};
-    uint64_t key[4];
+    uint64_t key[5];
     wave_key(M, key);
     for (uint32_t w = 0; w < full + (tail ? 1 : 0); w++) {
       if (w == full) single_tail(r, X, tail, M);
@@ -1644,6 +1658,7 @@ lucent_status lucent_batch_trace(lucent_batch* b, uint32_t samples, void* stream
     const Group& G = gs[g];
     const int ng = G.i1 - G.i0;
     M.n = ng;
+    M.scene = recs[G.i0].scene;
     M.max_bounces = G.max_bounces;
     M.any_alpha = G.any_alpha;
     M.any_tex = G.any_tex;
@@ -1675,7 +1690,7 @@ lucent_status lucent_batch_trace(lucent_batch* b, uint32_t samples, void* stream
       M.path_base = (const uint32_t*)X.base.ptr + G.base + (full ? 0 : 2 * (ng + 1));
       M.pix_base = M.path_base + (ng + 1);
       if (full && b->opt.use_graph && b->waves > 0) {  // first wave ever runs uncaptured (one-time setup inside)
-        uint64_t key[4];
+        uint64_t key[5];
         wave_key(M, key);
         key[0] |= 1ull << 63;  // captured without the accumulation
         if ((st = b->graphs[x][g].run(M, key, X.stream, false))) return st;

@@ -117,6 +117,7 @@ struct MultiLaunch {
   int any_tex;                     // some scene has texture maps: launch the TEX shade instantiation
   int wide;                        // traversal over the scenes' four-wide BVH views
   int near;                        // nearest-first traversal (every scene's view is usable, and wide is set)
+  sh::SceneDev scene;              // the scene, where n is 1
   int sort_classes;                // distinct SceneRec::sort_class values (>= 1)
   // Ray capture (lucent_renderer_capture_rays; parity tests): for every
   // bounce b in cap_mask, the bounce's closest-hit rays with their hits and
