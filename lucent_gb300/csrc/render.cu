@@ -13,10 +13,12 @@
 //   any-hit  -> shadow rays
 //   resolve  -> unoccluded NEE added in the reference's order (sun, env, light):
 //               at the start of the next shade, or in the accumulation for a
-//               path that ends (the backward replays keep a resolve kernel)
+//               path that ends
 // Accumulation replays the running mean (trace.frag:350-354) sample by
 // sample per pixel, so a batch equals S sequential draws.
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "internal.h"
 #include "render_internal.h"
@@ -258,25 +260,28 @@ __device__ __forceinline__ bool analytic_occluded(const SceneDev& S, float3 ro, 
 // Path-replay adjoint state (used by the ADJ instantiation of k_shade_t).
 // Gradients are of sum_pixels dl[pixel] . (mean radiance of the replayed
 // samples) with respect to each material's base colour (3), roughness,
-// metallic and clearcoat (dmat, 6 floats per material) and to the
-// environment texels (denv, RGB + one pad float per texel, 16-byte aligned, so
-// that a tap is one vector atomic). Sampling (directions,
+// metallic and clearcoat (dmat, 6 of 8 floats per material) and to the
+// environment texels (denv, RGB + one pad float per texel), both 16-byte
+// aligned, so that a tap is one vector atomic and a material two. Sampling (directions,
 // pdfs, MIS weights, lobe and Russian-roulette choices, the firefly clamp's
 // scale) is held fixed, as in path replay backpropagation.
 struct AdjointDev {
   const float4* dl;  // per pixel: dL/dI (rgb) / samples
-  float4* lrem;      // per path: radiance still to come (primal total minus what is accounted for)
-  float4* gcont;     // per path, 5 float4: dl_c * df_c/dtheta_p / f_c at the BSDF-sampled direction (18), material
-  float4* gslot;     // per shadow slot, 2 float4: dl . c * df/f for its light direction (6), material
-  float4* genv;      // per path: environment sample uv and scale (rgb) of its env shadow slot
+  float4* lrem;      // per path: radiance still to come (primal total minus what is accounted for); w: see k_seed_lrem
+  int* hit;          // [bounce][queue position]: triangle slot, as the primal replay met it
+  uint32_t* count;   // [bounce]: length of its queue
+  uint8_t* lit;      // [bounce][path]: bit j = next-event ray j was unoccluded
   float* dmat;
   float* denv;       // nullptr: no environment gradient
-  uint32_t WH;
+  uint32_t WH, paths;
   int primal;        // 1: the primal replay (paths only, no adjoint work)
 };
+constexpr int kBounceShift = 8;  // path flags of the primal replay: the bounce last shaded
 
-// Adds g[0..5] to dmat[mat * 6 ..] (global or shared memory), one atomic per
-// distinct material per warp.
+// Adds g[0..5] to material `mat`'s gradient, once per distinct material per
+// warp and as vectors: a scene has few materials, so what bounds this is the
+// atomics to one sector that wait for one another (a backward of 512 x 512 x 8
+// with 33 materials: 10.7 ms with six scalar atomics, 9.9 with two vectors).
 __device__ __forceinline__ void add_material_grad(float* dmat, int mat, const float g[6]) {
   const unsigned act = __activemask();
   const unsigned peers = __match_any_sync(act, mat);
@@ -288,10 +293,11 @@ __device__ __forceinline__ void add_material_grad(float* dmat, int mat, const fl
 #pragma unroll
     for (int k = 0; k < 6; k++) sum[k] += __shfl_sync(peers, g[k], src);
   }
-  if (lane == leader && mat >= 0)
-#pragma unroll
-    for (int k = 0; k < 6; k++)
-      if (sum[k] != 0.f) atomicAdd(dmat + (size_t)mat * 6 + k, sum[k]);
+  if (lane == leader && mat >= 0) {
+    float* const d = dmat + (size_t)mat * 8;
+    atomicAdd(reinterpret_cast<float4*>(d), make_float4(sum[0], sum[1], sum[2], sum[3]));
+    atomicAdd(reinterpret_cast<float2*>(d + 4), make_float2(sum[4], sum[5]));
+  }
 }
 
 // Environment texel gradient: sv_c * bilinear weight into each of 4 texels,
@@ -316,24 +322,12 @@ __device__ __forceinline__ float clamp_scale(float3 c, int bounce, float uclamp)
   return l > uclamp ? uclamp / l : 1.f;
 }
 
-// dl . (c (.) df_p / f) for p = 0..5 (zero where f is zero).
+// g_p += dl . (c (.) df_p / f) for p = 0..5 (nothing where f is zero).
 __device__ __forceinline__ void contract_grad(float3 dl, float3 c, float3 f, const float3 df[6], float g[6]) {
   const float w[3] = {f.x != 0.f ? dl.x * c.x / f.x : 0.f, f.y != 0.f ? dl.y * c.y / f.y : 0.f,
                       f.z != 0.f ? dl.z * c.z / f.z : 0.f};
 #pragma unroll
-  for (int k = 0; k < 6; k++) g[k] = w[0] * df[k].x + w[1] * df[k].y + w[2] * df[k].z;
-}
-
-// Gradient of one next-event contribution c (light direction wi) with respect
-// to the vertex's material, stored in its shadow slot until occlusion is known.
-__device__ __forceinline__ void nee_grad(const AdjointDev& A, const LightingDev& L, const Surface& s, float3 wo,
-                                         float3 wi, float3 dl, float3 c, int material, uint32_t slot) {
-  float3 df[6];
-  const float3 fg = eval_opaque_grad(L, s, wo, wi, df);
-  float g[6];
-  contract_grad(dl, c, fg, df, g);
-  A.gslot[2 * (size_t)slot] = make_float4(g[0], g[1], g[2], g[3]);
-  A.gslot[2 * (size_t)slot + 1] = make_float4(g[4], g[5], __int_as_float(material), 0.f);
+  for (int k = 0; k < 6; k++) g[k] += w[0] * df[k].x + w[1] * df[k].y + w[2] * df[k].z;
 }
 
 // Where the shade kernel finds a path's scene, lighting and settings: a
@@ -456,9 +450,11 @@ static int shade_threads(uint32_t paths) { return paths >= (1u << 21) ? kShadeTh
 template <class Src, bool ADJ = false, bool TEX = false>
 __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __grid_constant__ Src src, int cur, int bounce,
                                                     const __grid_constant__ AdjointDev A = AdjointDev{}) {
-  const uint32_t n = TEX ? P.ctr[kCtrTex] : P.ctr[kCtrQ0 + cur];
+  const bool adj = ADJ && !A.primal;
+  const uint32_t n = TEX ? P.ctr[kCtrTex] : adj ? A.count[bounce] : P.ctr[kCtrQ0 + cur];
   const uint32_t* q = P.q[cur];
   uint32_t* qn = P.q[cur ^ 1];
+  if (ADJ && !adj && blockIdx.x == 0 && threadIdx.x == 0) A.count[bounce] = n;
   for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < n; k0 += gridDim.x * blockDim.x) {
     __syncthreads();
     const uint32_t k = k0 + threadIdx.x;
@@ -476,36 +472,46 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
     const float4 tint4 = first ? first_record_field(3, rd) : P.tint[p];
     float3 thr = f3(thr4), rad = f3(first ? first_record_field(7, rd) : P.rad[p]), tint = f3(tint4);
     // The forward render and the backward's primal replay resolve the
-    // previous bounce's next-event contributions here (the adjoint replay
-    // keeps its resolve kernel, which also gathers gradients): the unoccluded
-    // ones join the radiance first, in the reference's order (sun,
-    // environment, light), as a separate resolve pass would add them.
-    unsigned emitted = 0u;
+    // previous bounce's next-event contributions here: the unoccluded ones
+    // join the radiance first, in the reference's order (sun, environment,
+    // light), as a separate resolve pass would add them.
+    unsigned emitted = 0u, lit = 0u;
     const unsigned flags = __float_as_uint(tint4.w);
-    if (!ADJ || A.primal) {
+    if (!adj) {
       const unsigned pending = flags >> kPendShift & 7u;
 #pragma unroll
       for (int j = 0; j < 3; j++) {
         if (!(pending >> j & 1u)) continue;
         const float4 c = P.sh_c[3 * (size_t)p + j];
-        if (c.w != 0.f) rad = rad + f3(c);  // unoccluded
+        if (c.w != 0.f) {  // unoccluded
+          rad = rad + f3(c);
+          if (ADJ) lit |= 1u << j;
+        }
       }
+      if (ADJ && !first) A.lit[(size_t)(bounce - 1) * A.paths + p] = (uint8_t)lit;
     }
     float bsdf_pdf = thr4.w;
     bool spec = flags & kSpecular, done = flags & kGuideDone;
-    float4 galb = first ? first_record_field(4, rd) : P.galb[p];
-    float4 gnrm = first ? first_record_field(5, rd) : P.gnrm[p];
+    float4 galb = first || ADJ ? first_record_field(4, rd) : P.galb[p];  // the backward has no guides
+    float4 gnrm = first || ADJ ? first_record_field(5, rd) : P.gnrm[p];
     uint32_t st = __float_as_uint(ro4.w);  // the path's RNG state
-    float4 hv = P.hit[kq];
+    float4 hv;
+    if (adj) hv = make_float4(INF, 0.f, 0.f, __int_as_float(A.hit[(size_t)bounce * A.paths + k]));
+    else hv = P.hit[kq];
+    if (ADJ && !adj) A.hit[(size_t)bounce * A.paths + k] = __float_as_int(hv.w);
     if (__float_as_int(hv.w) >= 0) hv = hit_values(S.geo, ro, rd, __float_as_int(hv.w));
     bool alive = false, deferred = false;
     float3 dl = f3(0.f, 0.f, 0.f), lrem = f3(0.f, 0.f, 0.f);
-    int cont_mat = -1;
-    const bool adj = ADJ && !A.primal;
+    float grad[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float cont[6];  // the gradient of what follows the BSDF-sampled direction
+    int grad_mat = -1, last = 0;
     if (adj) {
       const float4 l4 = A.lrem[p];
-      dl = l4.w == 0.f ? f3(A.dl[p % A.WH]) : f3(0.f, 0.f, 0.f);  // w != 0: the sample was dropped (NaN)
+      const unsigned w = __float_as_uint(l4.w);
+      dl = w & 1u ? f3(0.f, 0.f, 0.f) : f3(A.dl[p % A.WH]);
+      last = (int)(w >> 1);
       lrem = f3(l4);
+      lit = A.lit[(size_t)bounce * A.paths + p];
     }
 
     // traceScene (scene.glsl:192-333): spheres, ground, then the triangle hit.
@@ -535,7 +541,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
     }
     do {
       if (!tri && best_sphere < 0 && !ground) {  // miss (trace.frag:146-155)
-        if (bounce == 0) P.gpos[p] = make_float4(0.f, 0.f, 0.f, 1.f);  // no guide position: full reuse
+        if (!ADJ && bounce == 0) P.gpos[p] = make_float4(0.f, 0.f, 0.f, 1.f);  // no guide position: full reuse
         const float3 env = bounce == 0 && !L.env_background ? L.backdrop : environment(L, rd, spec, bsdf_pdf);
         rad = rad + clamp_c(thr * env, bounce, uclamp);
         if (adj) {
@@ -558,7 +564,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
       }
       // Hit record.
       const float3 pos = ro + rd * closest;
-      if (bounce == 0) P.gpos[p] = make_float4(pos.x, pos.y, pos.z, 1.f);
+      if (!ADJ && bounce == 0) P.gpos[p] = make_float4(pos.x, pos.y, pos.z, 1.f);
       float3 normal, gn;
       bool front;
       int material, light = -1;
@@ -654,7 +660,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
         if (light >= 0) break;
       }
       const bool glass = s.transmission > 0.f && rnd(st) < s.transmission;
-      if (bounce == 0) {  // trace.frag:187-193: reflections and refractions do not move with the surface
+      if (!ADJ && bounce == 0) {  // trace.frag:187-193: reflections and refractions do not move with the surface
         const float sharp = 1.f - smooth(0.1f, 0.7f, s.roughness);
         float glossy = fmaxf(sharp * mixf(0.5f, 1.f, s.metallic), s.transmission);
         glossy = fmaxf(glossy, s.clearcoat * 0.5f * (1.f - smooth(0.08f, 0.5f, s.clearcoat_roughness)));
@@ -674,10 +680,10 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
         thr = thr * weight;
         if (adj) {
           if (!refl) {  // transmission weight = base colour: d/d albedo_c of what follows = lrem_c / albedo_c
-            const float g[6] = {s.albedo.x > 0.f ? dl.x * lrem.x / s.albedo.x : 0.f,
-                                s.albedo.y > 0.f ? dl.y * lrem.y / s.albedo.y : 0.f,
-                                s.albedo.z > 0.f ? dl.z * lrem.z / s.albedo.z : 0.f, 0.f, 0.f, 0.f};
-            add_material_grad(A.dmat, material, g);
+            grad[0] = s.albedo.x > 0.f ? dl.x * lrem.x / s.albedo.x : 0.f;
+            grad[1] = s.albedo.y > 0.f ? dl.y * lrem.y / s.albedo.y : 0.f;
+            grad[2] = s.albedo.z > 0.f ? dl.z * lrem.z / s.albedo.z : 0.f;
+            grad_mat = material;
           }
         }
         if (!done) tint = tint * weight;
@@ -728,6 +734,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
             tmax = ls.dist * (1.f - 1e-4f);
             ok = ls.pdf > 0.f;
           }
+          if (adj && !(lit >> j & 1u)) continue;
           const float NdotL = dot3(n, wi);
           if (!(ok && NdotL > 0.f && dot3(gn, wi) > 0.f && !analytic_occluded(S, so, wi, tmax))) continue;
           float pb;
@@ -735,15 +742,18 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
           const float w = mis(pdf, pb);
           const float3 cu = thr * f * NdotL * le * (w / pdf);
           const float3 c = clamp_c(cu, bounce, uclamp);
-          emit_shadow(P, p, j, so, wi, tmax, st, c);
-          emitted |= 1u << j;
           if (adj) {
-            nee_grad(A, L, s, wo, wi, dl, c, material, 3 * p + j);
-            if (j == 1) {
-              const float3 sv = thr * f * (clamp_scale(cu, bounce, uclamp) * NdotL * (w / pdf) * L.env_intensity);
-              A.genv[2 * (size_t)p] = make_float4(env_uv.x, env_uv.y, sv.x, sv.y);
-              A.genv[2 * (size_t)p + 1] = make_float4(sv.z, 0.f, 0.f, 0.f);
-            }
+            lrem = lrem - c;
+            float3 df[6];
+            const float3 fg = eval_opaque_grad(L, s, wo, wi, df);
+            contract_grad(dl, c, fg, df, grad);
+            grad_mat = material;
+            if (j == 1 && A.denv)
+              add_env_grad(A, L, env_uv, dl,
+                           thr * f * (clamp_scale(cu, bounce, uclamp) * NdotL * (w / pdf) * L.env_intensity));
+          } else {
+            emit_shadow(P, p, j, so, wi, tmax, st, c);
+            emitted |= 1u << j;
           }
         }
         const BsdfSample bs = sample_opaque(L, s, wo, U);  // :255-261
@@ -753,17 +763,9 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
           const float3 fg = eval_opaque_grad(L, s, wo, bs.dir, df);
           const float w[3] = {fg.x != 0.f ? dl.x / fg.x : 0.f, fg.y != 0.f ? dl.y / fg.y : 0.f,
                               fg.z != 0.f ? dl.z / fg.z : 0.f};
-          float gc[18];
 #pragma unroll
-          for (int k = 0; k < 6; k++) gc[3 * k] = w[0] * df[k].x, gc[3 * k + 1] = w[1] * df[k].y, gc[3 * k + 2] = w[2] * df[k].z;
-          float4* o = A.gcont + 5 * (size_t)p;
-          o[0] = make_float4(gc[0], gc[1], gc[2], gc[3]);
-          o[1] = make_float4(gc[4], gc[5], gc[6], gc[7]);
-          o[2] = make_float4(gc[8], gc[9], gc[10], gc[11]);
-          o[3] = make_float4(gc[12], gc[13], gc[14], gc[15]);
-          o[4].x = gc[16];
-          o[4].y = gc[17];
-          cont_mat = material;
+          for (int k = 0; k < 6; k++)
+            cont[k] = lrem.x * (w[0] * df[k].x) + lrem.y * (w[1] * df[k].y) + lrem.z * (w[2] * df[k].z);
         }
         thr = thr * bs.weight;
         bsdf_pdf = bs.pdf;
@@ -773,34 +775,43 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
       }
       if (bounce >= 2) {  // Russian roulette (:265-269)
         const float pr = fminf(0.95f, max3(thr));
-        if (rnd(st) >= pr) {
-          cont_mat = -1;
-          break;
-        }
+        if (rnd(st) >= pr) break;
         thr = thr / pr;
       }
       alive = bounce < max_bounces;
-      if (!alive) cont_mat = -1;
+      if (adj) {
+        alive = bounce < last;
+        if (alive && !spec) {
+#pragma unroll
+          for (int k = 0; k < 6; k++) grad[k] += cont[k];
+          grad_mat = material;
+        }
+      }
     } while (false);
     if (deferred) {
       P.qtex[atomicAdd(&P.ctr[kCtrTex], 1u)] = kq;
       continue;
     }
     if (adj) {
-      A.lrem[p].x = lrem.x, A.lrem[p].y = lrem.y, A.lrem[p].z = lrem.z;
-      A.gcont[5 * (size_t)p + 4].z = __int_as_float(cont_mat);
+      add_material_grad(A.dmat, grad_mat, grad);
+      if (alive) A.lrem[p].x = lrem.x, A.lrem[p].y = lrem.y, A.lrem[p].z = lrem.z;
+    } else {
+      P.rad[p] = make_float4(rad.x, rad.y, rad.z, 0.f);
     }
-
-    P.rad[p] = make_float4(rad.x, rad.y, rad.z, 0.f);
     // Flags always (the slots this bounce left pending, for resolve), the rest if the path goes on.
-    P.tint[p] = make_float4(tint.x, tint.y, tint.z,
-                            __uint_as_float((spec ? kSpecular : 0u) | (done ? kGuideDone : 0u) | emitted << kPendShift));
-    P.galb[p] = galb;
-    P.gnrm[p] = gnrm;
+    const unsigned out = (spec ? kSpecular : 0u) | (done ? kGuideDone : 0u) | emitted << kPendShift;
+    if (ADJ) {
+      P.tint[p].w = __uint_as_float(out | (unsigned)bounce << kBounceShift);
+    } else {
+      P.tint[p] = make_float4(tint.x, tint.y, tint.z, __uint_as_float(out));
+      P.galb[p] = galb;
+      P.gnrm[p] = gnrm;
+    }
     if (alive) {
       P.ro[p] = make_float4(ro.x, ro.y, ro.z, __uint_as_float(st));
       P.rd[p] = make_float4(rd.x, rd.y, rd.z, 0.f);
       P.thr[p] = make_float4(thr.x, thr.y, thr.z, bsdf_pdf);
+      if (adj) continue;  // the queues are the primal replay's
       const uint32_t pos = atomicAdd(&P.ctr[kCtrQ0 + (cur ^ 1)], 1u);
       qn[pos] = p;
       P.nray[2 * (size_t)pos] = make_float4(ro.x, ro.y, ro.z, __uint_as_float(p));
@@ -809,86 +820,26 @@ __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __g
   }
 }
 
-// Resolve for the adjoint replay: the unoccluded next-event contributions
-// leave the path's remaining radiance and add their material (and
-// environment) gradients; what remains is the radiance that followed the
-// BSDF-sampled direction, whose gradient is lrem (.) dl (.) df/f.
-//
-// A scene has few materials, and every warp adding to their 6 words in global
-// memory made all other accesses queue behind those atomics (33 materials, 0.9
-// M paths: 542 us, 143 warps waiting for memory per instruction). Each block sums in
-// shared memory and adds its sums once (nmat > 0; up to kSharedMaterials).
-constexpr int kSharedMaterials = 1024;  // 24 KB
-__global__ void __launch_bounds__(128) k_resolve_adjoint(Paths P, const __grid_constant__ AdjointDev A,
-                                                         const SceneRec* __restrict__ rec, int cur, int nmat) {
-  extern __shared__ float sum[];
-  for (int i = threadIdx.x; i < nmat * 6; i += blockDim.x) sum[i] = 0.f;
-  __syncthreads();
-  const LightingDev& L = rec->light;
-  const uint32_t n = P.ctr[kCtrQ0 + cur];
-  const uint32_t* q = P.q[cur];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const uint32_t p = q[k];
-    float4 r = P.rad[p];
-    const float4 l4 = A.lrem[p];
-    float3 lrem = f3(l4);
-    const float3 dl = l4.w == 0.f ? f3(A.dl[p % A.WH]) : f3(0.f, 0.f, 0.f);
-    float g[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    int mat = -1;
-    const unsigned pending = __float_as_uint(P.tint[p].w) >> kPendShift & 7u;
-    for (int j = 0; j < 3; j++) {
-      const uint32_t s = 3 * p + j;
-      if (!(pending >> j & 1u)) continue;
-      const float4 c = P.sh_c[s];
-      if (c.w != 0.f) {  // unoccluded
-        r.x += c.x;
-        r.y += c.y;
-        r.z += c.z;
-        lrem = lrem - f3(c);
-        const float4 a = A.gslot[2 * (size_t)s], b = A.gslot[2 * (size_t)s + 1];
-        g[0] += a.x, g[1] += a.y, g[2] += a.z, g[3] += a.w, g[4] += b.x, g[5] += b.y;
-        mat = __float_as_int(b.z);
-        if (j == 1 && A.denv) {
-          const float4 e0 = A.genv[2 * (size_t)p], e1 = A.genv[2 * (size_t)p + 1];
-          add_env_grad(A, L, make_float2(e0.x, e0.y), dl, f3(e0.z, e0.w, e1.x));
-        }
-      }
-    }
-    const float4* gc = A.gcont + 5 * (size_t)p;
-    const int cm = __float_as_int(gc[4].z);
-    if (cm >= 0) {
-      mat = cm;
-      const float4 a = gc[0], b = gc[1], c = gc[2], d = gc[3], e = gc[4];
-      const float v[18] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w, e.x, e.y};
-#pragma unroll
-      for (int t = 0; t < 6; t++) g[t] += lrem.x * v[3 * t] + lrem.y * v[3 * t + 1] + lrem.z * v[3 * t + 2];
-    }
-    P.rad[p] = r;
-    A.lrem[p] = make_float4(lrem.x, lrem.y, lrem.z, l4.w);
-    if (nmat > 0) add_material_grad(sum, mat, g);
-    else add_material_grad(A.dmat, mat, g);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nmat * 6; i += blockDim.x)
-    if (sum[i] != 0.f) atomicAdd(A.dmat + i, sum[i]);
-}
-
 // Primal radiance of each replayed sample -> the adjoint replay's remaining
-// radiance (a dropped NaN/inf sample is flagged in w and contributes nothing).
-// The primal replay's last shaded bounce is resolved here, as the forward
-// render's accumulation resolves it.
+// radiance; w = 2 * the bounce the path ended at, + 1 for a dropped NaN/inf
+// sample, which contributes nothing. The primal replay's last shaded bounce is
+// resolved here, as the forward render's accumulation resolves it.
 __global__ void k_seed_lrem(Paths P, AdjointDev A, uint32_t total) {
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
     float4 c = P.rad[p];
-    const unsigned pending = __float_as_uint(P.tint[p].w) >> kPendShift & 7u;
+    const unsigned flags = __float_as_uint(P.tint[p].w), pending = flags >> kPendShift & 7u, last = flags >> kBounceShift;
+    unsigned lit = 0u;
     for (int j = 0; j < 3; j++) {
       if (!(pending >> j & 1u)) continue;
       const float4 e = P.sh_c[3 * (size_t)p + j];
       if (e.w == 0.f) continue;  // occluded
       c = make_float4(c.x + e.x, c.y + e.y, c.z + e.z, c.w);
+      lit |= 1u << j;
     }
+    A.lit[(size_t)last * A.paths + p] = (uint8_t)lit;
     const bool bad = isnan(c.x) || isnan(c.y) || isnan(c.z) || isinf(c.x) || isinf(c.y) || isinf(c.z);
-    A.lrem[p] = bad ? make_float4(0.f, 0.f, 0.f, 1.f) : make_float4(c.x, c.y, c.z, 0.f);
+    A.lrem[p] = bad ? make_float4(0.f, 0.f, 0.f, __uint_as_float(2u * last + 1u))
+                    : make_float4(c.x, c.y, c.z, __uint_as_float(2u * last));
   }
 }
 
@@ -1199,12 +1150,11 @@ __global__ void k_sort_scatter(Paths P, int nxt) {
   }
 }
 
-// Sorts the rays of queue `nxt` into the ray stream and the queue into the
-// free queue buffer `dst`, which becomes queue `nxt`; returns the buffer of
-// the pre-sort queue. P is the caller's copy of the path state: every wave
-// starts from the launch's own pointers, so a captured wave replays the same
-// sequence of buffer rotations.
-static uint32_t* sort_rays_into(const MultiLaunch& M, Paths& P, int nxt, int blocks, cudaStream_t s, uint32_t* dst) {
+// Sorts the rays of queue `nxt` into the ray stream and the queue into `dst`,
+// which becomes queue `nxt`; returns the buffer of the pre-sort queue. P is the
+// caller's copy of the path state: every wave starts from the launch's own
+// pointers, so a captured wave replays the same sequence of buffer rotations.
+static uint32_t* sort_rays(const MultiLaunch& M, Paths& P, int nxt, int blocks, cudaStream_t s, uint32_t* dst) {
   Paths Ps = P;
   Ps.sort_tmp = dst;
   cudaMemsetAsync(P.sort_hist, 0, (size_t)kSortBins * 4, s);
@@ -1215,15 +1165,11 @@ static uint32_t* sort_rays_into(const MultiLaunch& M, Paths& P, int nxt, int blo
   P.q[nxt] = dst;
   return pre;
 }
-// The sorted queue into sort_tmp, the pre-sort queue kept there in its place.
-static void sort_rays(const MultiLaunch& M, Paths& P, int nxt, int blocks, cudaStream_t s) {
-  P.sort_tmp = sort_rays_into(M, P, nxt, blocks, s, P.sort_tmp);
-}
 
 // ------------------------------------------------------------ one wave
-// Grid of the any-hit (twice this many blocks of 256), resolve and sort
+// Grid of the any-hit (twice this many blocks of 256) and sort
 // kernels: five 128-thread blocks per SM (measured; smaller grids slowed the
-// any-hit and resolve kernels).
+// any-hit kernel).
 static int aux_blocks() {
   static int n = 0;
   if (!n) {
@@ -1315,7 +1261,7 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
   const int aux = M.shade_blocks > 0 ? M.shade_blocks : aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
   bool sorted = false;  // the rays of this bounce are in the sorted stream
-  bool forked = false;  // the previous bounce's shadow rays and resolve run on M.side
+  bool forked = false;  // the previous bounce's shadow rays run on M.side
   for (int b = 0; b <= M.max_bounces; b++) {
     const int cur = b & 1;
     if (forked)  // the side stream still reads the other counters
@@ -1374,23 +1320,11 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
     nl++;
     if (fork) cudaEventRecord(M.ev_join, t);
     forked = fork;
-    const bool was_sorted = sorted;
     // The two largest queues; the third too in waves of 2^21 paths or more
     // (measured: it pays for its sort there, not in smaller waves).
     sorted = M.sort_rays && b < M.max_bounces && (b < 2 || (b == 2 && M.total_paths >= (1u << 21)));
     nl += sorted ? 3 : 0;  // keys, scan, scatter
-    if (sorted && was_sorted) {
-      // This bounce's pre-sort queue in sort_tmp stays as it is (the backward
-      // replays' resolve, perhaps still running on the side stream, walks it);
-      // its sorted queue buffer is free once shaded, so the next queue is
-      // sorted into that one instead, and sort_tmp becomes the next-but-one
-      // queue after the join.
-      uint32_t* busy = P.sort_tmp;
-      P.sort_tmp = sort_rays_into(M, P, cur ^ 1, aux, s, P.q[cur]);
-      P.q[cur] = busy;
-    } else if (sorted) {
-      sort_rays(M, P, cur ^ 1, aux, s);
-    }
+    if (sorted) P.sort_tmp = sort_rays(M, P, cur ^ 1, aux, s, P.sort_tmp);
   }
   E.mark(kPhResolve, s);
   if (accumulate) nl += accumulate_wave(M, s);
@@ -1409,64 +1343,68 @@ int accumulate_wave(const MultiLaunch& M, cudaStream_t s) {
 // Replays the wave's samples twice with the adjoint instantiation of the
 // shade kernel (one instantiation, so both replays make identical choices):
 // first with the adjoint work off to recover each sample's primal radiance,
-// then propagating dl through every vertex.
+// then propagating dl through every vertex. What the second replay needs of
+// the rays is a triangle and three bits a vertex, so the first one writes them
+// down beside its queues (9 bytes a path and bounce) and the second traces
+// nothing; knowing which next-event rays arrive, its shade adds their
+// gradients at once. 512 x 512 x 8, 33
+// materials: 12.8 ms with both replays tracing and a pass that resolves, 9.9 so.
+// The second replay's shade waits for instructions most (bounce 1: 4.9 of 13.5
+// warps, issue slots 29 % busy).
 void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t s) {
-  const SceneRec* rec = M.recs;
-  const int nmat = H.materials <= kSharedMaterials ? H.materials : 0;
   static const int max_shade[2] = {persistent_blocks((const void*)k_shade_t<SceneTable, true>, kShadeThreads / 2),
                                    persistent_blocks((const void*)k_shade_t<SceneTable, true>, kShadeThreads)};
   const int shade_t = shade_threads(M.total_paths), shade_blocks = max_shade[shade_t == kShadeThreads];
   const int aux = aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
-  for (int pass = 0; pass < 2; pass++) {
-    const AdjointDev A{H.dl, H.lrem, H.gcont, H.gslot, H.genv, H.dmat, H.denv, M.total_pixels, pass == 0 ? 1 : 0};
-    Paths P = M.paths;     // queue buffers swap with the sort buffer below
-    bool sorted = false;  // as in render_wave_multi: the rays of bounces 1 and 2 are sorted
-    bool forked = false;  // as in render_wave_multi: shadow rays and resolve on M.side
-    k_camera_multi<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, M.recs, M.path_base, M.n, M.sid, M.S);
-    for (int b = 0; b <= M.max_bounces; b++) {
-      const int cur = b & 1;
-      if (forked)
-        k_zero_closest_counters<<<1, 32, 0, s>>>(P.ctr);
-      else
-        k_zero_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
-      PathClosestMulti pc{P.ctr + kCtrQ0 + cur, sorted ? P.sray : P.nray, P.ro, P.hit, M.recs, M.any_alpha};
-      TravArgs TA{nullptr, 0, nullptr, 1e-6, 1e30, P.slow, P.ctr + kCtrSlow, P.ctr + kCtrWork, P.ctr + kCtrErr,
-                  nullptr, top};
-      launch_closest_multi(M, P, TA, pc, s);
-      if (forked) {  // the previous bounce's resolve (lrem, radiance) precedes this shade
-        cudaStreamWaitEvent(s, M.ev_join, 0);
-        k_zero_shade_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
-      }
-      k_shade_t<SceneTable, true><<<shade_blocks, shade_t, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b, A);
-      const bool fork = M.side && b < M.max_bounces;
-      cudaStream_t t = s;
-      if (fork) {
-        cudaEventRecord(M.ev_fork, s);
-        cudaStreamWaitEvent(M.side, M.ev_fork, 0);
-        t = M.side;
-      }
-      PathShadowMulti ps{P.ctr + kCtrShadow, P.qs, P.sh_o, P.sh_d, P.sh_c, M.recs, M.sid, M.any_alpha};
-      TravArgs TB{nullptr, 0, nullptr, 1e-6, 1e30, P.slow2, P.ctr + kCtrSlow2, P.ctr + kCtrWork2, P.ctr + kCtrErr,
-                  nullptr, top};
-      launch_shadow_multi(M, aux * 2, TB, ps, t);
-      Paths Pr = P;  // resolve walks the pre-sort queue, in path order
-      if (sorted) Pr.q[cur] = P.sort_tmp;
-      if (pass == 1)  // the primal replay resolves in its next shade and in k_seed_lrem
-        k_resolve_adjoint<<<aux, 128, (size_t)nmat * 24, t>>>(Pr, A, rec, cur, nmat);
-      if (fork) cudaEventRecord(M.ev_join, t);
-      forked = fork;
-      const bool was_sorted = sorted;
-      sorted = M.sort_rays && b < M.max_bounces && (b < 2 || (b == 2 && M.total_paths >= (1u << 21)));
-      if (sorted && was_sorted) {  // as in render_wave_multi
-        uint32_t* busy = P.sort_tmp;
-        P.sort_tmp = sort_rays_into(M, P, cur ^ 1, aux, s, P.q[cur]);
-        P.q[cur] = busy;
-      } else if (sorted) {
-        sort_rays(M, P, cur ^ 1, aux, s);
-      }
+  AdjointDev A{H.dl, H.lrem, H.hit, H.count, H.lit, H.dmat, H.denv, M.total_pixels, M.total_paths, 1};
+  Paths P = M.paths;
+  P.q[0] = H.queue;
+  bool sorted = false;  // as in render_wave_multi: the rays of bounces 1 and 2 are sorted
+  bool forked = false;  // as in render_wave_multi: shadow rays on M.side
+  k_camera_multi<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, M.recs, M.path_base, M.n, M.sid, M.S);
+  for (int b = 0; b <= M.max_bounces; b++) {
+    const int cur = b & 1;
+    if (forked)
+      k_zero_closest_counters<<<1, 32, 0, s>>>(P.ctr);
+    else
+      k_zero_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
+    PathClosestMulti pc{P.ctr + kCtrQ0 + cur, sorted ? P.sray : P.nray, P.ro, P.hit, M.recs, M.any_alpha};
+    TravArgs TA{nullptr, 0, nullptr, 1e-6, 1e30, P.slow, P.ctr + kCtrSlow, P.ctr + kCtrWork, P.ctr + kCtrErr,
+                nullptr, top};
+    launch_closest_multi(M, P, TA, pc, s);
+    if (forked) {  // the previous bounce's shadow rays precede this shade, which resolves them
+      cudaStreamWaitEvent(s, M.ev_join, 0);
+      k_zero_shade_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
     }
-    if (pass == 0) k_seed_lrem<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, A, M.total_paths);
+    // The next bounce's queue is kept as it is shaded: after its sort, if there is one.
+    const bool sort = M.sort_rays && b < M.max_bounces && (b < 2 || (b == 2 && M.total_paths >= (1u << 21)));
+    uint32_t* const kept = H.queue + (size_t)(b + 1) * M.total_paths;
+    P.q[cur ^ 1] = sort || b == M.max_bounces ? M.paths.q[0] : kept;
+    k_shade_t<SceneTable, true><<<shade_blocks, shade_t, 0, s>>>(P, SceneTable{M.recs, M.sid}, cur, b, A);
+    const bool fork = M.side && b < M.max_bounces;
+    cudaStream_t t = s;
+    if (fork) {
+      cudaEventRecord(M.ev_fork, s);
+      cudaStreamWaitEvent(M.side, M.ev_fork, 0);
+      t = M.side;
+    }
+    PathShadowMulti ps{P.ctr + kCtrShadow, P.qs, P.sh_o, P.sh_d, P.sh_c, M.recs, M.sid, M.any_alpha};
+    TravArgs TB{nullptr, 0, nullptr, 1e-6, 1e30, P.slow2, P.ctr + kCtrSlow2, P.ctr + kCtrWork2, P.ctr + kCtrErr,
+                nullptr, top};
+    launch_shadow_multi(M, aux * 2, TB, ps, t);
+    if (fork) cudaEventRecord(M.ev_join, t);
+    forked = fork;
+    sorted = sort;
+    if (sort) sort_rays(M, P, cur ^ 1, aux, s, kept);
+  }
+  k_seed_lrem<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, A, M.total_paths);
+  A.primal = 0;
+  P.q[0] = H.queue;
+  k_camera_multi<<<grid_for(M.total_paths, 256), 256, 0, s>>>(P, M.recs, M.path_base, M.n, M.sid, M.S);
+  for (int b = 0; b <= M.max_bounces; b++) {
+    P.q[b & 1] = H.queue + (size_t)b * M.total_paths;
+    k_shade_t<SceneTable, true><<<shade_blocks, shade_t, 0, s>>>(P, SceneTable{M.recs, M.sid}, b & 1, b, A);
   }
 }
 

@@ -1122,12 +1122,13 @@ lucent_status lucent_renderer_backward(lucent_renderer* r, uint32_t samples, uin
   lucent_status st = X.reserve(batch * WH);
   if (st) return st;
   const size_t cap = X.path_cap;
-  const size_t nmat = (size_t)scene_owner(r)->material_count * 6;
+  const size_t nmat = scene_owner(r)->material_count;
   const size_t texels = d_env ? (size_t)r->light.env_w * r->light.env_h : 0;
-  const size_t env_off = (nmat + 3) & ~(size_t)3;  // the env gradients: float4 per texel, 16-byte aligned
+  const size_t env_off = nmat * 8;  // 6 of 8 floats per material, then RGB and a pad per texel
   const size_t nenv = texels * 4;
-  // per path: lrem 1 + gcont 5 + genv 2 float4; per shadow slot: gslot 2 float4 (3 slots per path)
-  if ((st = r->adj_dl.reserve((size_t)WH * 16)) || (st = r->adj_path.reserve(cap * 16 * (1 + 5 + 2 + 6))) ||
+  // per path: the remaining radiance, and 4 + 4 + 1 bytes for each bounce
+  const size_t vertices = cap * (r->max_bounces + 1);
+  if ((st = r->adj_dl.reserve((size_t)WH * 16)) || (st = r->adj_path.reserve(cap * 16 + vertices * 9 + (r->max_bounces + 1) * 4)) ||
       (st = r->adj_grad.reserve((env_off + nenv) * 4 + 16)))
     return st;
   std::vector<float> dl((size_t)WH * 4);
@@ -1141,9 +1142,11 @@ lucent_status lucent_renderer_backward(lucent_renderer* r, uint32_t samples, uin
   if (e == cudaSuccess) e = cudaMemsetAsync(r->adj_grad.ptr, 0, (env_off + nenv) * 4, s);
   if (e != cudaSuccess) return cuda_fail(e, "backward setup");
   float4* base = (float4*)r->adj_path.ptr;
-  AdjointDevHost H{(const float4*)r->adj_dl.ptr, base, base + cap, base + 6 * cap, base + 12 * cap,
-                   (float*)r->adj_grad.ptr, nenv ? (float*)r->adj_grad.ptr + env_off : nullptr,
-                   (int)scene_owner(r)->material_count};
+  int* const hit = (int*)(base + cap);
+  uint32_t* const queue = (uint32_t*)hit + vertices;
+  uint32_t* const count = queue + vertices;
+  AdjointDevHost H{(const float4*)r->adj_dl.ptr, base, hit, queue, count, (uint8_t*)(count + r->max_bounces + 1),
+                   (float*)r->adj_grad.ptr, nenv ? (float*)r->adj_grad.ptr + env_off : nullptr};
   for (uint32_t done = 0; done < samples; done += batch) {
     const uint32_t S = std::min(batch, samples - done);
     MultiLaunch M{};
@@ -1160,7 +1163,7 @@ lucent_status lucent_renderer_backward(lucent_renderer* r, uint32_t samples, uin
     clear_now((uint32_t*)X.ctr.ptr + kCtrErr, 4);
     return fail(LUCENT_ERR_DEVICE, "backward raised device error word 0x%x", word);
   }
-  for (size_t i = 0; i < nmat; i++) d_materials[i] += g[i];
+  for (size_t i = 0; i < nmat * 6; i++) d_materials[i] += g[i / 6 * 8 + i % 6];
   for (size_t i = 0; i < texels; i++)
     for (int c = 0; c < 3; c++) d_env[3 * i + c] += g[env_off + 4 * i + c];
   return LUCENT_OK;

@@ -159,14 +159,18 @@ struct PhaseEvents {
 int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe = nullptr, bool accumulate = true);
 int accumulate_wave(const MultiLaunch& M, cudaStream_t s);
 
-// Device buffers of a path-replay backward pass (per path: lrem 1, gcont 5,
-// genv 2 float4; per shadow slot: gslot 2 float4; dl per pixel).
+// Device buffers of a path-replay backward pass: dl per pixel, the remaining
+// radiance per path, and for each bounce (0 .. max_bounces) its queue, the
+// queue's length and what its rays met: a triangle slot per queue position and
+// the unoccluded next-event rays per path.
 struct AdjointDevHost {
   const float4* dl;
-  float4 *lrem, *gcont, *gslot, *genv;
-  float* dmat;
+  float4* lrem;
+  int* hit;
+  uint32_t *queue, *count;
+  uint8_t* lit;
+  float* dmat;  // 8 floats (6 parameters, pad) per material, 16-byte aligned
   float* denv;  // environment texel gradients, 4 floats (RGB, pad) per texel, 16-byte aligned
-  int materials;  // of the scene: dmat holds 6 floats each
 };
 // Gradient of sum_px dl[px] . (mean of the wave's samples) with respect to
 // material parameters (6 per material) and environment texels, for a launch
