@@ -36,7 +36,7 @@
 namespace lucent {
 namespace envs {
 
-constexpr int kScanBlock = 1024;
+constexpr uint32_t kMaxCells = 1u << 20;
 
 // Weight of cell i: mean luminance of its texels times sin(theta) of its row.
 __global__ void k_weights(const float* __restrict__ rgb, uint32_t w, uint32_t h, uint32_t gw, uint32_t gh,
@@ -98,78 +98,163 @@ __device__ __forceinline__ float dd_to_float(double2 a) {
   return up ? (r > 0 ? nextafterf(f, INFINITY) : nextafterf(f, -INFINITY)) : f;
 }
 
-__device__ __forceinline__ double2 as_dd(double v) { return make_double2(v, 0.0); }
-__device__ __forceinline__ double2 as_dd(double2 v) { return v; }
+// Scans: each thread takes `per` elements in turn, a warp its lanes' sums by
+// shuffles, a block its warps'; the blocks' sums are scanned by one block
+// before a second pass emits the prefixes. A fixed order, so deterministic.
+//
+// Bound by binary64 arithmetic: a double-double addition is 20 operations, of
+// which an SM does two lanes a cycle. 32,768 cells as 32 blocks of 1024 threads
+// in log2(1024) whole-block steps took 57 us a pass and as much again for the
+// one block over the blocks' sums; small blocks of 64 threads, four elements or
+// more a thread, bring it to 3 additions an element on all SMs: 10, 15 and 15
+// us for the sums, the parts and the prefixes. A sampler build of 256 x 128,
+// 1024 x 512 and 1024 x 1024 cells: 712, 1428 and 2156 us before, 160, 445 and
+// 706 now.
+constexpr int kScanThreads = 64, kScanParts = 512, kPartThreads = 128;  // kScanParts / kPartThreads parts a thread
 
-// Block-wise inclusive scan (Hillis-Steele in double-double: a fixed order,
-// deterministic); 1024 threads a block.
-__device__ __forceinline__ double2 block_scan(double2 x, double2* sh) {
-  const int t = threadIdx.x;
-  sh[t] = x;
-  __syncthreads();
-  for (int o = 1; o < kScanBlock; o <<= 1) {
-    const double2 y = t >= o ? sh[t - o] : make_double2(0.0, 0.0);
-    __syncthreads();
-    if (t >= o) sh[t] = dd_add(sh[t], y);
-    __syncthreads();
+struct WeightAt {
+  const double* v;
+  __device__ double2 operator()(uint32_t i) const { return make_double2(v[i], 0.0); }
+};
+struct DdAt {
+  const double2* v;
+  __device__ double2 operator()(uint32_t i) const { return v[i]; }
+};
+// Light flags (scaled pmf < 1) in descending cell order (position r = n - 1 -
+// i), the order in which the reference pops its stacks.
+struct LightAt {
+  const double* x;
+  uint32_t n;
+  __device__ uint32_t operator()(uint32_t r) const { return x[n - 1 - r] < 1 ? 1u : 0u; }
+};
+__device__ __forceinline__ double2 add(double2 a, double2 b) { return dd_add(a, b); }
+__device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) { return a + b; }
+__device__ __forceinline__ double2 shfl_up(double2 v, int o) {
+  return make_double2(__shfl_up_sync(~0u, v.x, o), __shfl_up_sync(~0u, v.y, o));
+}
+__device__ __forceinline__ uint32_t shfl_up(uint32_t v, int o) { return __shfl_up_sync(~0u, v, o); }
+
+// Sum of x over the threads before this one; `all`: over the block.
+template <int kThreads, class V>
+__device__ __forceinline__ V block_before(V x, V& all) {
+  __shared__ V sums[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+  V s = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const V y = shfl_up(s, o);
+    if (lane >= o) s = add(y, s);
   }
-  return sh[t];
+  if (lane == 31) sums[warp] = s;
+  __syncthreads();
+  V before{};
+  all = V{};
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; w++) {
+    if (w == warp) before = all;
+    all = add(all, sums[w]);
+  }
+  const V lanes = shfl_up(s, 1);
+  return lane ? add(before, lanes) : before;
 }
 
-template <class T>
-__global__ void __launch_bounds__(kScanBlock) k_scan_blocks(const T* __restrict__ v, uint32_t n,
-                                                            double2* __restrict__ out, double2* __restrict__ part) {
-  __shared__ double2 sh[kScanBlock];
-  const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
-  const double2 s = block_scan(i < n ? as_dd(v[i]) : make_double2(0.0, 0.0), sh);
-  if (i < n) out[i] = s;
-  if (threadIdx.x == kScanBlock - 1) part[blockIdx.x] = s;
+// One of a launch's scans: n elements `at`, block sums at `part`.
+template <class At, class V>
+struct ScanJob {
+  At at;
+  uint32_t n;
+  V* part;
+  V* out;  // inclusive prefixes (k_scan_emit)
+};
+template <class At, class V>
+struct ScanJobs {
+  ScanJob<At, V> job[2];  // blockIdx.y
+};
+
+template <class At, class V>
+__device__ __forceinline__ V thread_sum(const ScanJob<At, V>& J, uint32_t i0, uint32_t per) {
+  V s{};
+  for (uint32_t k = 0; k < per && i0 + k < J.n; k++) s = add(s, J.at(i0 + k));
+  return s;
+}
+template <class At, class V>
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const __grid_constant__ ScanJobs<At, V> jobs, uint32_t per) {
+  const ScanJob<At, V>& J = jobs.job[blockIdx.y];
+  V all;
+  block_before<kScanThreads>(thread_sum(J, (blockIdx.x * kScanThreads + threadIdx.x) * per, per), all);
+  if (threadIdx.x == 0) J.part[blockIdx.x] = all;
 }
 
-// Exclusive scan of the (at most 1024) block totals in place, one block.
-__global__ void __launch_bounds__(kScanBlock) k_scan_parts(double2* __restrict__ part, uint32_t m) {
-  __shared__ double2 sh[kScanBlock];
-  const uint32_t t = threadIdx.x;
-  block_scan(t < m ? part[t] : make_double2(0.0, 0.0), sh);  // ends with a barrier
-  if (t < m) part[t] = t == 0 ? make_double2(0.0, 0.0) : sh[t - 1];
+// The m block sums of each job become the sums before each block; their total
+// goes to part[kScanParts].
+template <class V>
+__global__ void __launch_bounds__(kPartThreads) k_scan_parts(V* part0, V* part1, uint32_t m) {
+  V* const part = blockIdx.x ? part1 : part0;
+  constexpr uint32_t per = kScanParts / kPartThreads;
+  V v[per], s{}, all;
+#pragma unroll
+  for (uint32_t k = 0; k < per; k++) {
+    const uint32_t i = threadIdx.x * per + k;
+    v[k] = i < m ? part[i] : V{};
+    s = add(s, v[k]);
+  }
+  s = block_before<kPartThreads>(s, all);
+#pragma unroll
+  for (uint32_t k = 0; k < per; k++) {
+    const uint32_t i = threadIdx.x * per + k;
+    if (i < m) part[i] = s;
+    s = add(s, v[k]);
+  }
+  if (threadIdx.x == 0) part[kScanParts] = all;
 }
 
-__global__ void k_scan_add(double2* __restrict__ out, uint32_t n, const double2* __restrict__ part) {
-  const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
-  if (i < n && blockIdx.x > 0) out[i] = dd_add(out[i], part[blockIdx.x]);
+// Sum of everything before this thread's elements.
+template <class At, class V>
+__device__ __forceinline__ V thread_before(const ScanJob<At, V>& J, uint32_t i0, uint32_t per) {
+  V all;
+  const V before = block_before<kScanThreads>(thread_sum(J, i0, per), all);
+  return add(J.part[blockIdx.x], before);
+}
+template <class At, class V>
+__global__ void __launch_bounds__(kScanThreads) k_scan_emit(const __grid_constant__ ScanJobs<At, V> jobs, uint32_t per) {
+  const ScanJob<At, V>& J = jobs.job[blockIdx.y];
+  const uint32_t i0 = (blockIdx.x * kScanThreads + threadIdx.x) * per;
+  V s = thread_before(J, i0, per);
+  for (uint32_t k = 0; k < per && i0 + k < J.n; k++) {
+    s = add(s, J.at(i0 + k));
+    J.out[i0 + k] = s;
+  }
 }
 
-// x_i = pmf_i * n with pmf = w / total (1/n for a black map); light flags for
-// the index scan, taken in descending index order (position r = n - 1 - i),
-// the order in which the reference pops its stacks.
+// x_i = pmf_i * n with pmf = w / total (1/n for a black map).
 __global__ void k_classify(const double* __restrict__ weight, uint32_t n, const double2* __restrict__ total_p,
-                           double* __restrict__ pmf, double* __restrict__ x, double* __restrict__ light_rev) {
+                           double* __restrict__ pmf, double* __restrict__ x) {
   const double total = total_p->x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double p = total > 0 ? __ddiv_rn(weight[i], total) : __ddiv_rn(1.0, (double)n);
     const double xi = __dmul_rn(p, (double)n);
     pmf[i] = p;
     x[i] = xi;
-    light_rev[n - 1 - i] = xi < 1 ? 1.0 : 0.0;
   }
 }
 
 // Compacts lights and heavies (descending index) with their exact deficit
 // 1 - x / excess x - 1 as double-doubles.
-__global__ void k_split(const double* __restrict__ x, uint32_t n, const double2* __restrict__ light_incl,
-                        uint32_t* __restrict__ L, double2* __restrict__ deficit, uint32_t* __restrict__ H,
-                        double2* __restrict__ excess) {
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    const uint32_t i = n - 1 - r;
-    const bool light = x[i] < 1;
-    const uint32_t lights_before = (uint32_t)light_incl[r].x - (light ? 1u : 0u);
-    if (light) {
-      L[lights_before] = i;
-      deficit[lights_before] = dd_two_sum(1.0, -x[i]);
+__global__ void __launch_bounds__(kScanThreads) k_split(const __grid_constant__ ScanJob<LightAt, uint32_t> J,
+                                                        uint32_t per, uint32_t* __restrict__ L,
+                                                        double2* __restrict__ deficit, uint32_t* __restrict__ H,
+                                                        double2* __restrict__ excess) {
+  const uint32_t i0 = (blockIdx.x * kScanThreads + threadIdx.x) * per;
+  uint32_t lights = thread_before(J, i0, per);
+  for (uint32_t r = i0; r < i0 + per && r < J.n; r++) {
+    const uint32_t i = J.n - 1 - r;
+    const double x = J.at.x[i];
+    if (x < 1) {
+      L[lights] = i;
+      deficit[lights++] = dd_two_sum(1.0, -x);
     } else {
-      const uint32_t k = r - lights_before;
-      H[k] = i;
-      excess[k] = dd_two_sum(x[i], -1.0);
+      H[r - lights] = i;
+      excess[r - lights] = dd_two_sum(x, -1.0);
     }
   }
 }
@@ -223,15 +308,9 @@ __global__ void k_table(const float* __restrict__ prob, const uint32_t* __restri
   }
 }
 
-// Inclusive double-double scan of v[0..n) into out (n <= 1024 * 1024); part:
-// 1024 double-doubles.
-template <class T>
-static void scan(const T* v, uint32_t n, double2* out, double2* part, cudaStream_t s) {
-  const uint32_t blocks = (n + kScanBlock - 1) / kScanBlock;
-  k_scan_blocks<T><<<blocks, kScanBlock, 0, s>>>(v, n, out, part);
-  k_scan_parts<<<1, kScanBlock, 0, s>>>(part, blocks);
-  k_scan_add<<<blocks, kScanBlock, 0, s>>>(out, n, part);
-}
+// Elements a thread: at most kScanParts blocks.
+static uint32_t scan_per(uint32_t n) { return std::max(4u, (n + kScanThreads * kScanParts - 1) / (kScanThreads * kScanParts)); }
+static uint32_t scan_blocks(uint32_t n) { return (n + kScanThreads * scan_per(n) - 1) / (kScanThreads * scan_per(n)); }
 
 }  // namespace envs
 
@@ -246,20 +325,20 @@ lucent_status gpu_env_sampler(const float* rgb_d, uint32_t w, uint32_t h, uint32
   using namespace envs;
   env_grid(w, h, max_w, gw, gh);
   const uint32_t n = gw * gh;
-  if (n > (uint32_t)kScanBlock * kScanBlock)
-    return fail(LUCENT_ERR_UNSUPPORTED, "%u sampler cells; the device build takes at most %u", n,
-                (uint32_t)kScanBlock * kScanBlock);
+  if (n > kMaxCells)
+    return fail(LUCENT_ERR_UNSUPPORTED, "%u sampler cells; the device build takes at most %u", n, kMaxCells);
   std::vector<double> sin_row(gh);
   for (uint32_t cy = 0; cy < gh; cy++) sin_row[cy] = std::sin(M_PI * (cy + 0.5) / gh);
-  // Scratch, carved in 256-byte aligned pieces: sin rows, 4 arrays of n
-  // doubles, 5 of n double-doubles, 3 of n uint32, the scans' block totals
-  // and the error word.
+  // Scratch, carved in 256-byte aligned pieces: sin rows, 3 arrays of n
+  // doubles, 3 of n double-doubles, 3 of n uint32 and one of n floats, the
+  // scans' block sums with their totals, and the error word.
   const size_t dbl = 8 * (size_t)n, dd = 16 * (size_t)n;
   auto piece = [](size_t sz) { return (sz + 255) & ~(size_t)255; };
-  const size_t bytes = piece(8 * (size_t)gh) + 4 * piece(dbl) + 5 * piece(dd) + 3 * piece(4 * (size_t)n) +
-                       piece(16 * (size_t)kScanBlock) + piece(16);
-  DeviceBuffer buf;
-  lucent_status st = buf.reserve(bytes);
+  const size_t parts = piece(16 * (size_t)(kScanParts + 1)), lparts = piece(4 * (size_t)(kScanParts + 1));
+  const size_t bytes = piece(8 * (size_t)gh) + 3 * piece(dbl) + 3 * piece(dd) + 4 * piece(4 * (size_t)n) + 2 * parts +
+                       lparts + piece(16);
+  TempBuffer buf;
+  lucent_status st = buf.reserve(bytes, s);
   if (st) return st;
   char* b = (char*)buf.ptr;
   char* const end = b + bytes;
@@ -272,22 +351,21 @@ lucent_status gpu_env_sampler(const float* rgb_d, uint32_t w, uint32_t h, uint32
   double* weight = (double*)take(dbl);
   double* pmf = (double*)take(dbl);
   double* x = (double*)take(dbl);
-  double* light = (double*)take(dbl);
-  double2* wsum = (double2*)take(dd);
-  double2* light_incl = (double2*)take(dd);
   double2* deficit = (double2*)take(dd);
   double2* excess = (double2*)take(dd);
   double2* DC = (double2*)take(dd);  // D in [0, nl), C in [nl, n)
   uint32_t* L = (uint32_t*)take(4 * (size_t)n);
   uint32_t* H = (uint32_t*)take(4 * (size_t)n);
   uint32_t* alias = (uint32_t*)take(4 * (size_t)n);
-  double2* part = (double2*)take(16 * (size_t)kScanBlock);
+  float* prob = (float*)take(4 * (size_t)n);
+  double2* part = (double2*)take(parts);
+  double2* part2 = (double2*)take(parts);
+  uint32_t* lpart = (uint32_t*)take(lparts);
   unsigned* bad = (unsigned*)take(16);
   if (b > end) {  // the pieces above must add up to `bytes`
     buf.release();
     return fail(LUCENT_ERR_DEVICE, "environment sampler scratch layout");
   }
-  float* prob = (float*)wsum;  // wsum is dead once the total is read
   const int g = grid_for(n, 256);
   cudaError_t e = cudaMemcpyAsync(sin_d, sin_row.data(), 8 * (size_t)gh, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, 4, s);
@@ -296,14 +374,19 @@ lucent_status gpu_env_sampler(const float* rgb_d, uint32_t w, uint32_t h, uint32
     return cuda_fail(e, "environment sampler upload");
   }
   k_weights<<<g, 256, 0, s>>>(rgb_d, w, h, gw, gh, sin_d, weight, bad);
-  scan(weight, n, wsum, part, s);  // total = the last inclusive sum
-  k_classify<<<g, 256, 0, s>>>(weight, n, wsum + (n - 1), pmf, x, light);
-  scan(light, n, light_incl, part, s);
+  const uint32_t per = scan_per(n), blocks = scan_blocks(n);
+  const ScanJobs<WeightAt, double2> weights{{{{weight}, n, part, nullptr}, {}}};
+  k_scan_sums<<<blocks, kScanThreads, 0, s>>>(weights, per);
+  k_scan_parts<<<1, kPartThreads, 0, s>>>(part, part, blocks);
+  k_classify<<<g, 256, 0, s>>>(weight, n, part + kScanParts, pmf, x);
+  const ScanJobs<LightAt, uint32_t> lights{{{{x, n}, n, lpart, nullptr}, {}}};
+  k_scan_sums<<<blocks, kScanThreads, 0, s>>>(lights, per);
+  k_scan_parts<<<1, kPartThreads, 0, s>>>(lpart, lpart, blocks);
   uint32_t nl = 0;
   unsigned bad_h = 0;
-  double2 nl_d = {0, 0}, total_d = {0, 0};
-  e = cudaMemcpyAsync(&nl_d, light_incl + (n - 1), 16, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&total_d, wsum + (n - 1), 16, cudaMemcpyDeviceToHost, s);
+  double2 total_d = {0, 0};
+  e = cudaMemcpyAsync(&nl, lpart + kScanParts, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&total_d, part + kScanParts, 16, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&bad_h, bad, 4, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
@@ -315,11 +398,13 @@ lucent_status gpu_env_sampler(const float* rgb_d, uint32_t w, uint32_t h, uint32
     return fail(LUCENT_ERR_INVALID, "environment weights must be finite and >= 0");
   }
   total = total_d.x;
-  nl = (uint32_t)nl_d.x;
   const uint32_t nh = n - nl;
-  k_split<<<g, 256, 0, s>>>(x, n, light_incl, L, deficit, H, excess);
-  if (nl) scan(deficit, nl, DC, part, s);
-  if (nh) scan(excess, nh, DC + nl, part, s);
+  k_split<<<blocks, kScanThreads, 0, s>>>(lights.job[0], per, L, deficit, H, excess);
+  const uint32_t most = std::max(nl, nh), per2 = scan_per(most), blocks2 = scan_blocks(most);
+  const ScanJobs<DdAt, double2> sums{{{{deficit}, nl, part, DC}, {{excess}, nh, part2, DC + nl}}};
+  k_scan_sums<<<dim3(blocks2, 2), kScanThreads, 0, s>>>(sums, per2);
+  k_scan_parts<<<2, kPartThreads, 0, s>>>(part, part2, blocks2);
+  k_scan_emit<<<dim3(blocks2, 2), kScanThreads, 0, s>>>(sums, per2);
   k_serve<<<g, 256, 0, s>>>(L, nl, DC, H, nh, DC + nl, x, prob, alias);
   k_table<<<g, 256, 0, s>>>(prob, alias, pmf, n, table_d);
   e = cudaGetLastError();
