@@ -40,9 +40,16 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     return LUCENT_OK;
   }
 
-  // Scratch, one allocation. Big nodes hold more than kSub triangles, so a
-  // level has at most n / (kSub + 1) of them, each with one ragged chunk.
-  const uint32_t nrec = 2 * n - 1, big_cap = n / (kSub + 1) + 1, chunk_cap = n / kChunk + big_cap;
+  // Scratch, one allocation. Big nodes hold more than sub_n triangles, so a
+  // level has at most n / (sub_n + 1) of them, each with one ragged chunk.
+  // Small builds: all big levels in one cluster. Whole builds of a soup, by
+  // launches with subtrees of 1,024 and so: 2,503 triangles 435 and 321 us,
+  // 8,000 569 and 443, 16,000 663 and 617 but of a knot 672 and 683. Subtrees
+  // of 256 and 512 triangles: 2,503 321 and 322 us, 4,000 373 and 393, 12,000
+  // 548 and 519; of 128, 2,503 takes 346.
+  const bool clustered = n <= 12288;
+  const uint32_t sub_n = !clustered ? kSub : n <= 4096 ? 256 : 512;
+  const uint32_t nrec = 2 * n - 1, big_cap = n / (sub_n + 1) + 1, chunk_cap = n / kChunk + big_cap;
   const size_t words = (size_t)3 * bins * 7;
   struct Part {
     size_t bytes;
@@ -107,6 +114,7 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
   cx.big_cap = big_cap;
   cx.chunk_cap = chunk_cap;
   cx.rec_cap = nrec;
+  cx.sub = sub_n;
   cx.max_leaf = max_leaf;
   cx.nbins = bins;
 
@@ -118,13 +126,14 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
                                                                              (float4*)b_hi.ptr, (float*)b_cz.ptr);
   uint32_t got[kCtrBuild] = {0};
   int p = 0;
-  if (n > kSub) {
+  uint32_t small = 0;  // blocks of the subtree kernel
+  if (n > sub_n) {
     k_clear_bins<<<std::min<uint32_t>((uint32_t)(big_cap * words + 255) / 256, 152 * 8), 256, 0, s>>>(cx.bins, big_cap * words);
     // Two levels more than halving would take, then a few at a time until no
     // big node is left; a level of no nodes costs five empty launches.
     int levels = 3;
     while ((n >> (levels - 2)) > (uint32_t)kSub) levels++;
-    for (int total = 0;; levels = 3) {
+    for (int total = 0; !clustered; levels = 3) {
       if ((total += levels) > 8192) return done(fail(LUCENT_ERR_DEVICE, "BVH build did not converge"));
       for (int k = 0; k < levels; k++, p ^= 1) {
         k_big_bins<<<chunk_cap, 256, words * 4, s>>>(cx, p);
@@ -138,19 +147,26 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
       if (got[kErrW]) return done(fail(LUCENT_ERR_DEVICE, "BVH build raised device error 0x%x", got[kErrW]));
       if (got[kNBig + p] == 0) break;
     }
+    small = got[kNSmall];
+    if (clustered) {
+      k_big_levels<<<kCluster, 256, 8 * words * 4, s>>>(cx);
+      small = std::min(n, 2 * 152u);  // the device knows how many there are
+    }
   } else {
-    got[kNSmall] = 1;
+    small = 1;
   }
-  if (got[kNSmall] > n) return done(fail(LUCENT_ERR_DEVICE, "task list overflow"));
+  if (small > n) return done(fail(LUCENT_ERR_DEVICE, "task list overflow"));
   // Subtrees that all run at once take 16 warps each, as the launch lasts as
-  // long as one of them (2,503 triangles, whole build: 367 us against 416 with
-  // 8; 82,000: 651 against 703); more of them 8 (2,000,000: 3.80 ms against
-  // 3.94). Subtrees of 512 or 2,048 triangles measured slower at both ends.
-  const int threads = got[kNSmall] <= 3 * 152 ? kSubThreads : kSubThreads / 2;
-  const size_t smem = sub_bytes(bins, threads);
-  BB_CUDA(cudaFuncSetAttribute((const void*)k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  // long as one of them (82,000 triangles, whole build: 651 us against 703 with
+  // 8); more of them 8 (2,000,000: 3.80 ms against 3.94). Subtrees of 512 or
+  // 2,048 triangles measured slower after big levels by launches.
+  const int threads = small <= 3 * 152 ? kSubThreads : kSubThreads / 2;
+  const size_t smem = sub_bytes(sub_n, bins, threads);
+  // The most any build asks for, so that builds on several threads agree.
+  BB_CUDA(cudaFuncSetAttribute((const void*)k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sub_bytes(kSub, kMaxBins, kSubThreads)),
           "shared memory of the subtree kernel");
-  if (got[kNSmall]) k_subtree<<<got[kNSmall], threads, smem, s>>>(cx);
+  if (small) k_subtree<<<small, threads, smem, s>>>(cx);
   const int g = (int)((nrec + 127) / 128);
   uint32_t* inner = (uint32_t*)b_inner.ptr;
   uint32_t* height = (uint32_t*)b_height.ptr;
