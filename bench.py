@@ -200,8 +200,8 @@ def run_ours_closest(args, rank, world, local):
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": NCU_DRAM_BYTES_CLOSEST_LAUNCH,
                 "traffic_scope": "DRAM bytes of one launch over the 1e6 rays; ncu capture of this workload "
-                                 "summarised in profiles/closest_wide_soup65k_1Mrays.md",
-                "peak_source": which, "kernel": "k_closest_wide_t<ApiPolicy> (+ slow path)",
+                                 "summarised in profiles/near_box512_and_soup.md",
+                "peak_source": which, "kernel": "k_closest_near_t<ApiPolicy> (+ the rays it hands on)",
                 "bytes_per_ray": alg["bytes_per_ray"]}
     return {
         "metric": "closest-hit Mrays/s (intersectBVH, 65,536-triangle soup, 1e6 rays)",
@@ -230,8 +230,8 @@ CPU_BASELINE_SECONDS = 10.0
 # dram__bytes_read.sum + dram__bytes_write.sum of the closest-hit launches,
 # from ncu captures of the same workloads (the source is named in each line's
 # traffic_scope).
-NCU_DRAM_BYTES_PT_FRAME = 553_000_000
-NCU_DRAM_BYTES_CLOSEST_LAUNCH = 115_400_000
+NCU_DRAM_BYTES_PT_FRAME = 594_000_000
+NCU_DRAM_BYTES_CLOSEST_LAUNCH = 48_900_000
 PT_METRIC = ("closest-hit Mrays/s inside path tracing: box scene (81,956 triangles), 512x512, 16 spp, "
              "max depth 8 (also spp/s)")
 CONFIGS = {
@@ -347,8 +347,8 @@ def run_ours_pt(args, rank, world, local):
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": NCU_DRAM_BYTES_PT_FRAME,
                 "traffic_scope": "DRAM bytes of the frame's 9 closest-hit launches, like achieved; ncu capture of "
-                                 "this workload summarised in profiles/closest_pt_box512_16spp.md",
-                "peak_source": which, "kernel": "k_closest_wide_t<PathClosestMulti> (+ slow path)",
+                                 "this workload summarised in profiles/near_box512_and_soup.md",
+                "peak_source": which, "kernel": "k_closest_near_t<PathClosestOne> (+ the rays it hands on)",
                 "bytes_per_closest_ray": alg["bytes_per_closest_ray"],
                 "closest_ms_per_frame": round(ph["closest"], 3)}
     # Kernels launched in the timed frames, as the renderer counts them (reset + trace: camera, 7 per bounce,
@@ -618,7 +618,7 @@ def run_ours_knot(args, rank, world, local):
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": None,
                 "traffic_scope": "not captured for this workload",
-                "peak_source": which, "kernel": "k_closest_wide_t<PathClosestMulti> (+ slow path)",
+                "peak_source": which, "kernel": "k_closest_near_t<PathClosestOne> (+ the rays it hands on)",
                 "bytes_per_closest_ray": alg["bytes_per_closest_ray"],
                 "closest_ms_per_step": round(ph["closest"], 3)}
     r.dispose()

@@ -83,10 +83,13 @@ void lucent_bvh_destroy(lucent_bvh* bvh);
 lucent_status lucent_bvh_info(const lucent_bvh* bvh, uint32_t* node_count, uint32_t* tri_count);
 /* Traversal mode: 0 = f32 bounded-error path with binary64 fallback and the
  * top six BVH levels staged in shared memory, 1 = every decision in binary64,
- * 2 = mode 0 reading every node from global memory, 3 = mode 0's decisions
- * over a four-wide view of the tree (each inner step reads a node's four
- * grandchildren; built on first use, 128 bytes per node; the default). All
- * return identical results. lucent_bvh_intersect_noalloc always uses 0. */
+ * 2 = mode 0 reading every node from global memory, 3 = nearest first over a
+ * four-wide view of the tree, each hit checked against the reference's
+ * decisions and the rays that the check leaves open traced as in mode 0 (the
+ * default; 128 bytes per node and 4 per triangle, built on the first call,
+ * which then waits; a first call inside a stream capture, a tree that is not
+ * the builder's kind, or rays far from it take a four-wide view in mode 0's
+ * order). All return identical results. lucent_bvh_intersect_noalloc always uses 0. */
 #define LUCENT_TRAVERSE_FAST 0
 #define LUCENT_TRAVERSE_EXACT 1
 #define LUCENT_TRAVERSE_FAST_GLOBAL 2
@@ -364,11 +367,11 @@ lucent_status lucent_renderer_set_ray_sort(lucent_renderer* r, int32_t enabled);
  * memory (default on). Hits and images are the same either way; only where
  * the traversal reads those nodes changes. */
 lucent_status lucent_renderer_set_top_levels(lucent_renderer* r, int32_t enabled);
-/* Closest-hit rays over a four-wide view of the BVH (each inner step reads the
- * four grandchildren of a node; built at scene load, 128 bytes per binary
- * node; default on). Hits and images are the same either way: the
- * grandchildren's boxes lie inside their parents', so the reference's cull
- * decisions and visiting order are unchanged. */
+/* Closest-hit and shadow rays over four-wide views of the BVH (each inner step
+ * reads the four grandchildren of a node; built at scene load, 128 bytes per
+ * binary node each; default on): nearest first, and in the reference's order
+ * where that cannot show the reference's answer. Hits and images are the same
+ * either way. */
 lucent_status lucent_renderer_set_wide_bvh(lucent_renderer* r, int32_t enabled);
 /* Pipelined waves (default on): successive waves (of one trace or of
  * successive traces) alternate between two path-state buffers and are traced
@@ -466,10 +469,11 @@ typedef struct lucent_batch_options {
   uint32_t max_wave_paths;   /* path-state budget of one wave (about 430 bytes of device memory per path) */
   int32_t use_graph;         /* capture a full wave once as a CUDA graph and replay it */
   uint32_t trace_blocks;     /* grid of the persistent traversal kernels; 0 = all resident blocks */
-  uint32_t shade_blocks;     /* grid of the shade / resolve kernels; 0 = all resident blocks */
+  uint32_t shade_blocks;     /* grid of the shade kernels (blocks of 256 or 512 threads) and, in blocks
+                                of 128, of the sort and shadow kernels; 0 = all resident blocks */
   int32_t sort_rays;         /* sort the rays of bounces 1 and 2 (see lucent_renderer_set_ray_sort) */
   int32_t top_levels;        /* top BVH levels of the first 8 scenes in shared memory (lucent_renderer_set_top_levels) */
-  int32_t wide_bvh;          /* closest hit over the four-wide BVH views (lucent_renderer_set_wide_bvh) */
+  int32_t wide_bvh;          /* traversal of the four-wide BVH views (lucent_renderer_set_wide_bvh) */
   uint32_t scenes_per_wave;  /* waves hold consecutive groups of this many scenes, each group traced for all
                                 samples before the next (samples_per_wave / max_wave_paths then apply per
                                 group); 0 = every scene in every wave */

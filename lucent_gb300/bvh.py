@@ -71,7 +71,7 @@ class DeviceBVH:
 
     def set_mode(self, exact, top_levels=True, wide=True):
         """lucent_bvh_set_mode: all-binary64 traversal (exact), else the
-        binary32 path over the four-wide view of the tree (wide), or over the
+        binary32 path nearest first over a four-wide view (wide), or over the
         binary nodes with (top_levels) or without the shared-memory copy of
         the top BVH levels. Results are identical in every mode."""
         mode = 1 if exact else 3 if wide else 0 if top_levels else 2

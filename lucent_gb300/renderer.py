@@ -240,7 +240,7 @@ class Renderer:
         return col, dat
 
     def set_wide_bvh(self, enabled=True):
-        """Closest hit over the four-wide BVH view (lucent_renderer_set_wide_bvh)."""
+        """Nearest-first and four-wide traversal (lucent_renderer_set_wide_bvh)."""
         N.check(N.lib().lucent_renderer_set_wide_bvh(self._h, 1 if enabled else 0))
 
     def set_pipelining(self, enabled=True):
