@@ -41,7 +41,7 @@ constexpr int kChunk = 1024;  // triangles per block of a big level, 4 a thread
 // bins, three blocks an SM.
 constexpr int kSub = 1024;
 constexpr int kSubThreads = 512;  // at most: see k_subtree's launch
-constexpr int kCluster = 8;       // blocks of k_big_levels
+constexpr int kCluster = 8, kLevelThreads = 512;  // blocks of k_big_levels and their threads
 
 struct Prims {
   const float4* lo;  // (min.xyz, centroid.x)
@@ -502,6 +502,7 @@ __global__ void __launch_bounds__(256) k_prim_bounds(const float* __restrict__ p
 // order buffer, which also gathers the children's boxes. Grids cover the most
 // chunks and nodes a level can have; blocks beyond the level's own end at once.
 // ---------------------------------------------------------------------------
+template <int T>
 __device__ __forceinline__ void big_bins(const Ctx& cx, int p, uint32_t chunk, unsigned* sbin) {
   const Chunk ck = cx.chunk[p][chunk];
   const unsigned* bx = cx.box[p] + 12 * (size_t)ck.big;
@@ -510,12 +511,12 @@ __device__ __forceinline__ void big_bins(const Ctx& cx, int p, uint32_t chunk, u
   const Task t = cx.big[p][ck.big].t;
   const Split s = make_split(cbox, t.end - t.start, cx.nbins);
   const int words = 3 * cx.nbins * 7;
-  for (int k = threadIdx.x; k < words; k += 256) sbin[k] = bin_clear(k % 7);
+  for (int k = threadIdx.x; k < words; k += T) sbin[k] = bin_clear(k % 7);
   __syncthreads();
   const uint32_t* tri = cx.tri[t.src];
 #pragma unroll
-  for (int j = 0; j < kChunk / 256; j++) {
-    const uint32_t i = ck.begin + j * 256 + threadIdx.x;
+  for (int j = 0; j < kChunk / T; j++) {
+    const uint32_t i = ck.begin + j * T + threadIdx.x;
     const unsigned act = __ballot_sync(0xffffffffu, i < ck.end);
     if (i < ck.end) {
       const uint32_t k = tri[i];
@@ -524,7 +525,7 @@ __device__ __forceinline__ void big_bins(const Ctx& cx, int p, uint32_t chunk, u
   }
   __syncthreads();
   unsigned* to = cx.bins + (size_t)ck.big * words;
-  for (int k = threadIdx.x; k < words; k += 256) {
+  for (int k = threadIdx.x; k < words; k += T) {
     const int w = k % 7;
     if (sbin[k - w] == 0) continue;  // an empty bin
     if (w == 0) atomicAdd(to + k, sbin[k]);
@@ -536,7 +537,7 @@ __device__ __forceinline__ void big_bins(const Ctx& cx, int p, uint32_t chunk, u
 __global__ void __launch_bounds__(256) k_big_bins(Ctx cx, int p) {
   extern __shared__ unsigned sbin[];
   if (blockIdx.x == 0 && threadIdx.x == 0) cx.ctr[kNBig + (p ^ 1)] = cx.ctr[kNChunk + (p ^ 1)] = 0;
-  if (blockIdx.x < cx.ctr[kNChunk + p]) big_bins(cx, p, blockIdx.x, sbin);
+  if (blockIdx.x < cx.ctr[kNChunk + p]) big_bins<256>(cx, p, blockIdx.x, sbin);
 }
 
 // One warp per big node w: split, children, the node's record; its bins are left clear.
@@ -600,6 +601,7 @@ __global__ void __launch_bounds__(128) k_big_sah(Ctx cx, int p) {
 }
 
 // Which side each triangle of a chunk goes to (bits), and how many cross.
+template <int T>
 __device__ __forceinline__ void big_count(const Ctx& cx, int p, uint32_t chunk) {
   __shared__ uint32_t cross[2];
   const Chunk ck = cx.chunk[p][chunk];
@@ -610,8 +612,8 @@ __device__ __forceinline__ void big_count(const Ctx& cx, int p, uint32_t chunk) 
   const int lane = threadIdx.x & 31;
   const uint32_t* tri = cx.tri[B.t.src];
 #pragma unroll
-  for (int j = 0; j < kChunk / 256; j++) {
-    const uint32_t i = ck.begin + j * 256 + threadIdx.x;
+  for (int j = 0; j < kChunk / T; j++) {
+    const uint32_t i = ck.begin + j * T + threadIdx.x;
     bool left = false;
     if (i < ck.end) {
       const uint32_t k = tri[i];
@@ -622,7 +624,7 @@ __device__ __forceinline__ void big_count(const Ctx& cx, int p, uint32_t chunk) 
     const unsigned fr = __ballot_sync(0xffffffffu, i < ck.end && i < B.mid && !left);
     const unsigned bl = __ballot_sync(0xffffffffu, i < ck.end && i >= B.mid && left);
     if (lane == 0) {
-      cx.bits[(size_t)chunk * (kChunk / 32) + j * 8 + (threadIdx.x >> 5)] = m;
+      cx.bits[(size_t)chunk * (kChunk / 32) + j * (T / 32) + (threadIdx.x >> 5)] = m;
       if (fr) atomicAdd(&cross[0], __popc(fr));
       if (bl) atomicAdd(&cross[1], __popc(bl));
     }
@@ -631,7 +633,7 @@ __device__ __forceinline__ void big_count(const Ctx& cx, int p, uint32_t chunk) 
   if (threadIdx.x == 0) cx.count[chunk] = make_uint2(cross[0], cross[1]);
 }
 __global__ void __launch_bounds__(256) k_big_count(Ctx cx, int p) {
-  if (blockIdx.x < cx.ctr[kNChunk + p]) big_count(cx, p, blockIdx.x);
+  if (blockIdx.x < cx.ctr[kNChunk + p]) big_count<256>(cx, p, blockIdx.x);
 }
 
 // Block-wide setup of a partitioned chunk: the crossing counts before it and
@@ -639,6 +641,7 @@ __global__ void __launch_bounds__(256) k_big_count(Ctx cx, int p) {
 struct Cross {
   uint32_t fr0, bl0, m, m2;
 };
+template <int T>
 __device__ __forceinline__ Cross cross_setup(const Ctx& cx, const Big& B, const Chunk& ck, uint32_t chunk, unsigned* word,
                                              uint2* before) {
   __shared__ uint32_t sum[4];
@@ -646,7 +649,7 @@ __device__ __forceinline__ Cross cross_setup(const Ctx& cx, const Big& B, const 
   if (threadIdx.x < 4) sum[threadIdx.x] = 0;
   __syncthreads();
   uint32_t v[4] = {0, 0, 0, 0};  // before this chunk, and in all
-  for (uint32_t c = threadIdx.x; c < B.chunks; c += 256) {
+  for (uint32_t c = threadIdx.x; c < B.chunks; c += T) {
     const uint2 k = cx.count[B.chunk0 + c];
     v[2] += k.x;
     v[3] += k.y;
@@ -696,17 +699,18 @@ __device__ __forceinline__ Rank rank_of(const Cross& X, const Big& B, const Chun
           X.bl0 + before[j].y + __popc(m & ~in_front & lt)};
 }
 
+template <int T>
 __device__ __forceinline__ void big_place(const Ctx& cx, int p, uint32_t chunk) {
   __shared__ unsigned word[kChunk / 32];
   __shared__ uint2 before[kChunk / 32];
   const Chunk ck = cx.chunk[p][chunk];
   const Big& B = cx.big[p][ck.big];
   if (B.axis < 0) return;
-  const Cross X = cross_setup(cx, B, ck, chunk, word, before);
+  const Cross X = cross_setup<T>(cx, B, ck, chunk, word, before);
   if (X.m != X.m2 && threadIdx.x == 0) atomicOr(cx.ctr + kErrW, kErrQueue);  // impossible for a consistent binning
 #pragma unroll
-  for (int j = 0; j < kChunk / 256; j++) {
-    const uint32_t i = ck.begin + j * 256 + threadIdx.x;
+  for (int j = 0; j < kChunk / T; j++) {
+    const uint32_t i = ck.begin + j * T + threadIdx.x;
     if (i >= ck.end) continue;
     const Rank k = rank_of(X, B, ck, i, word, before);
     const uint32_t r = i - B.t.start;
@@ -716,9 +720,10 @@ __device__ __forceinline__ void big_place(const Ctx& cx, int p, uint32_t chunk) 
 }
 
 __global__ void __launch_bounds__(256) k_big_place(Ctx cx, int p) {
-  if (blockIdx.x < cx.ctr[kNChunk + p]) big_place(cx, p, blockIdx.x);
+  if (blockIdx.x < cx.ctr[kNChunk + p]) big_place<256>(cx, p, blockIdx.x);
 }
 
+template <int T>
 __device__ __forceinline__ void big_move(const Ctx& cx, int p, uint32_t chunk) {
   __shared__ unsigned word[kChunk / 32], sbox[2][12];
   __shared__ uint2 before[kChunk / 32];
@@ -729,15 +734,15 @@ __device__ __forceinline__ void big_move(const Ctx& cx, int p, uint32_t chunk) {
   const bool kids = B.kid[0] >= 0 || B.kid[1] >= 0;
   if (threadIdx.x < 24) sbox[threadIdx.x / 12][threadIdx.x % 12] = threadIdx.x % 6 < 3 ? 0xffffffffu : 0u;
   Cross X{0, 0, 0, 0};
-  if (B.axis >= 0) X = cross_setup(cx, B, ck, chunk, word, before);
+  if (B.axis >= 0) X = cross_setup<T>(cx, B, ck, chunk, word, before);
   else __syncthreads();
   const uint32_t start = B.t.start, n = B.t.end - start, L = B.mid - start;
   unsigned v[2][12];
   clear_box(v[0]);
   clear_box(v[1]);
 #pragma unroll
-  for (int j = 0; j < kChunk / 256; j++) {
-    const uint32_t i = ck.begin + j * 256 + threadIdx.x;
+  for (int j = 0; j < kChunk / T; j++) {
+    const uint32_t i = ck.begin + j * T + threadIdx.x;
     if (i >= ck.end) continue;
     const uint32_t t = tri[i], r = i - start;
     bool left = r < L;
@@ -773,15 +778,18 @@ __device__ __forceinline__ void big_move(const Ctx& cx, int p, uint32_t chunk) {
   }
 }
 __global__ void __launch_bounds__(256) k_big_move(Ctx cx, int p) {
-  if (blockIdx.x < cx.ctr[kNChunk + p]) big_move(cx, p, blockIdx.x);
+  if (blockIdx.x < cx.ctr[kNChunk + p]) big_move<256>(cx, p, blockIdx.x);
 }
 
 // All levels of a small build's big nodes by one cluster: the five steps of a
 // level wait for one another at the cluster's barrier instead of at launches,
 // and there are as many levels as the tree has, so subtrees can be small and
 // many. Bound by its dependent loads (25 us a level of 2,503 triangles, where
-// five launches took 30 to 45 and the empty levels 13 each).
-__global__ void __launch_bounds__(256) __cluster_dims__(kCluster, 1, 1) k_big_levels(Ctx cx) {
+// five launches took 30 to 45 and the empty levels 13 each). 512 threads a
+// block against 256: whole builds of 12,000 triangles of a soup and a knot 519
+// -> 490 and 571 -> 525 us, of 2,503 alike. A block a node, whose steps wait for the block alone, once
+// nodes have a chunk each: within 3 % either way.
+__global__ void __launch_bounds__(kLevelThreads) __cluster_dims__(kCluster, 1, 1) k_big_levels(Ctx cx) {
   extern __shared__ unsigned sbin[];
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const uint32_t rank = cluster.block_rank(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -797,27 +805,27 @@ __global__ void __launch_bounds__(256) __cluster_dims__(kCluster, 1, 1) k_big_le
     }
     if (rank == 0 && threadIdx.x == 0) cx.ctr[kNBig + (p ^ 1)] = cx.ctr[kNChunk + (p ^ 1)] = 0;
     for (uint32_t c = rank; c < chunks; c += kCluster) {
-      big_bins(cx, p, c, sbin);
+      big_bins<kLevelThreads>(cx, p, c, sbin);
       __syncthreads();
     }
     cluster.sync();
-    for (uint32_t w = rank * 8 + warp; w < nodes; w += kCluster * 8) {
+    for (uint32_t w = rank * (kLevelThreads / 32) + warp; w < nodes; w += kCluster * (kLevelThreads / 32)) {
       big_sah(cx, p, w, sbin + warp * 3 * cx.nbins * 7, lane);
       __syncwarp();
     }
     cluster.sync();
     for (uint32_t c = rank; c < chunks; c += kCluster) {
-      big_count(cx, p, c);
+      big_count<kLevelThreads>(cx, p, c);
       __syncthreads();
     }
     cluster.sync();
     for (uint32_t c = rank; c < chunks; c += kCluster) {
-      big_place(cx, p, c);
+      big_place<kLevelThreads>(cx, p, c);
       __syncthreads();
     }
     cluster.sync();
     for (uint32_t c = rank; c < chunks; c += kCluster) {
-      big_move(cx, p, c);
+      big_move<kLevelThreads>(cx, p, c);
       __syncthreads();
     }
     cluster.sync();

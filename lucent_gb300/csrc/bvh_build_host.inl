@@ -43,10 +43,10 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
   // Scratch, one allocation. Big nodes hold more than sub_n triangles, so a
   // level has at most n / (sub_n + 1) of them, each with one ragged chunk.
   // Small builds: all big levels in one cluster. Whole builds of a soup, by
-  // launches with subtrees of 1,024 and so: 2,503 triangles 435 and 321 us,
-  // 8,000 569 and 443, 16,000 663 and 617 but of a knot 672 and 683. Subtrees
-  // of 256 and 512 triangles: 2,503 321 and 322 us, 4,000 373 and 393, 12,000
-  // 548 and 519; of 128, 2,503 takes 346.
+  // launches with subtrees of 1,024 and so: 2,503 triangles 435 and 316 us,
+  // 8,000 569 and 427; 16,000, with blocks of 256 threads, 663 and 617 but of a
+  // knot 672 and 683. Subtrees of 256 and 512 triangles: 2,503 321 and 322 us,
+  // 4,000 373 and 393, 12,000 548 and 519; of 128, 2,503 takes 346.
   const bool clustered = n <= 12288;
   const uint32_t sub_n = !clustered ? kSub : n <= 4096 ? 256 : 512;
   const uint32_t nrec = 2 * n - 1, big_cap = n / (sub_n + 1) + 1, chunk_cap = n / kChunk + big_cap;
@@ -149,7 +149,7 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     }
     small = got[kNSmall];
     if (clustered) {
-      k_big_levels<<<kCluster, 256, 8 * words * 4, s>>>(cx);
+      k_big_levels<<<kCluster, kLevelThreads, kLevelThreads / 32 * words * 4, s>>>(cx);
       small = std::min(n, 2 * 152u);  // the device knows how many there are
     }
   } else {
