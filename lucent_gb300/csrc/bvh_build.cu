@@ -414,6 +414,7 @@ __device__ __forceinline__ int push_big(const Ctx& cx, int p, Task t, int lane) 
 }
 
 __global__ void k_clear_bins(unsigned* bins, size_t n) {
+  wait_for_previous();
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
     bins[k] = bin_clear((int)(k % 7));
 }
@@ -463,6 +464,7 @@ __device__ __forceinline__ void grow_box(unsigned* v, float4 lo, float4 hi, floa
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_prim_bounds(const float* __restrict__ pos, Ctx cx, float4* __restrict__ lo4,
                                                      float4* __restrict__ hi4, float* __restrict__ cz) {
+  wait_for_previous();
   __shared__ unsigned sbox[12];
   if (threadIdx.x < 12) sbox[threadIdx.x] = threadIdx.x % 6 < 3 ? 0xffffffffu : 0u;
   __syncthreads();
@@ -535,6 +537,7 @@ __device__ __forceinline__ void big_bins(const Ctx& cx, int p, uint32_t chunk, u
 }
 
 __global__ void __launch_bounds__(256) k_big_bins(Ctx cx, int p) {
+  wait_for_previous();
   extern __shared__ unsigned sbin[];
   if (blockIdx.x == 0 && threadIdx.x == 0) cx.ctr[kNBig + (p ^ 1)] = cx.ctr[kNChunk + (p ^ 1)] = 0;
   if (blockIdx.x < cx.ctr[kNChunk + p]) big_bins<256>(cx, p, blockIdx.x, sbin);
@@ -594,6 +597,7 @@ __device__ __forceinline__ void big_sah(const Ctx& cx, int p, uint32_t w, unsign
 }
 
 __global__ void __launch_bounds__(128) k_big_sah(Ctx cx, int p) {
+  wait_for_previous();
   extern __shared__ unsigned sbin[];
   const int warp = threadIdx.x >> 5;
   const uint32_t w = blockIdx.x * 4 + warp;
@@ -633,6 +637,7 @@ __device__ __forceinline__ void big_count(const Ctx& cx, int p, uint32_t chunk) 
   if (threadIdx.x == 0) cx.count[chunk] = make_uint2(cross[0], cross[1]);
 }
 __global__ void __launch_bounds__(256) k_big_count(Ctx cx, int p) {
+  wait_for_previous();
   if (blockIdx.x < cx.ctr[kNChunk + p]) big_count<256>(cx, p, blockIdx.x);
 }
 
@@ -720,6 +725,7 @@ __device__ __forceinline__ void big_place(const Ctx& cx, int p, uint32_t chunk) 
 }
 
 __global__ void __launch_bounds__(256) k_big_place(Ctx cx, int p) {
+  wait_for_previous();
   if (blockIdx.x < cx.ctr[kNChunk + p]) big_place<256>(cx, p, blockIdx.x);
 }
 
@@ -778,6 +784,7 @@ __device__ __forceinline__ void big_move(const Ctx& cx, int p, uint32_t chunk) {
   }
 }
 __global__ void __launch_bounds__(256) k_big_move(Ctx cx, int p) {
+  wait_for_previous();
   if (blockIdx.x < cx.ctr[kNChunk + p]) big_move<256>(cx, p, blockIdx.x);
 }
 
@@ -790,6 +797,7 @@ __global__ void __launch_bounds__(256) k_big_move(Ctx cx, int p) {
 // -> 490 and 571 -> 525 us, of 2,503 alike. A block a node, whose steps wait for the block alone, once
 // nodes have a chunk each: within 3 % either way.
 __global__ void __launch_bounds__(kLevelThreads) __cluster_dims__(kCluster, 1, 1) k_big_levels(Ctx cx) {
+  wait_for_previous();
   extern __shared__ unsigned sbin[];
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const uint32_t rank = cluster.block_rank(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1019,6 +1027,7 @@ __device__ __forceinline__ void subtree(const Ctx& cx, const Sub& S, const Task 
 }
 
 __global__ void __launch_bounds__(kSubThreads) k_subtree(Ctx cx) {
+  wait_for_previous();
   const uint32_t tasks = cx.ctr[kNSmall];  // may be more than the grid has blocks
 
   extern __shared__ float4 smem[];
@@ -1052,6 +1061,7 @@ __global__ void __launch_bounds__(kSubThreads) k_subtree(Ctx cx) {
 // ---------------------------------------------------------------------------
 __global__ void k_tree_counts(Ctx cx, uint32_t* __restrict__ arrived, uint32_t* inner, uint32_t* height,
                               uint32_t n_ids) {
+  wait_for_previous();
   uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= n_ids || __float_as_int(cx.recs[2 * (size_t)x + 1].w) <= 0) return;  // holes and inner nodes
   for (uint32_t up = cx.parent[x]; up != 0;) {  // the second child to arrive at a node goes on; ids fall on the way up

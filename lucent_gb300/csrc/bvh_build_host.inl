@@ -122,13 +122,14 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
   BB_CUDA(cudaMemsetAsync(cx.recs, 0xff, (size_t)nrec * 32, s), "clear nodes");
   BB_CUDA(cudaMemsetAsync(cx.parent, 0, (char*)b_height.ptr + b_height.bytes - (char*)b_parent.ptr, s), "clear tree");
   k_init<<<1, 32, 0, s>>>(cx);
-  k_prim_bounds<<<std::min<uint32_t>((n + 255) / 256, 152 * 8), 256, 0, s>>>(pos_d, cx, (float4*)b_lo.ptr,
-                                                                             (float4*)b_hi.ptr, (float*)b_cz.ptr);
+  launch_after(k_prim_bounds, std::min<uint32_t>((n + 255) / 256, 152 * 8), 256, 0, s, pos_d, cx, (float4*)b_lo.ptr,
+               (float4*)b_hi.ptr, (float*)b_cz.ptr);
   uint32_t got[kCtrBuild] = {0};
   int p = 0;
   uint32_t small = 0;  // blocks of the subtree kernel
   if (n > sub_n) {
-    k_clear_bins<<<std::min<uint32_t>((uint32_t)(big_cap * words + 255) / 256, 152 * 8), 256, 0, s>>>(cx.bins, big_cap * words);
+    launch_after(k_clear_bins, std::min<uint32_t>((uint32_t)(big_cap * words + 255) / 256, 152 * 8), 256, 0, s, cx.bins,
+                 big_cap * words);
     // Two levels more than halving would take, then a few at a time until no
     // big node is left; a level of no nodes costs five empty launches.
     int levels = 3;
@@ -136,11 +137,11 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     for (int total = 0; !clustered; levels = 3) {
       if ((total += levels) > 8192) return done(fail(LUCENT_ERR_DEVICE, "BVH build did not converge"));
       for (int k = 0; k < levels; k++, p ^= 1) {
-        k_big_bins<<<chunk_cap, 256, words * 4, s>>>(cx, p);
-        k_big_sah<<<(big_cap + 3) / 4, 128, 4 * words * 4, s>>>(cx, p);
-        k_big_count<<<chunk_cap, 256, 0, s>>>(cx, p);
-        k_big_place<<<chunk_cap, 256, 0, s>>>(cx, p);
-        k_big_move<<<chunk_cap, 256, 0, s>>>(cx, p);
+        launch_after(k_big_bins, chunk_cap, 256, words * 4, s, cx, p);
+        launch_after(k_big_sah, (big_cap + 3) / 4, 128, 4 * words * 4, s, cx, p);
+        launch_after(k_big_count, chunk_cap, 256, 0, s, cx, p);
+        launch_after(k_big_place, chunk_cap, 256, 0, s, cx, p);
+        launch_after(k_big_move, chunk_cap, 256, 0, s, cx, p);
       }
       BB_CUDA(cudaMemcpyAsync(got, cx.ctr, sizeof got, cudaMemcpyDeviceToHost, s), "read counters");
       BB_CUDA(cudaStreamSynchronize(s), "big levels");
@@ -149,7 +150,7 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
     }
     small = got[kNSmall];
     if (clustered) {
-      k_big_levels<<<kCluster, kLevelThreads, kLevelThreads / 32 * words * 4, s>>>(cx);
+      launch_after(k_big_levels, kCluster, kLevelThreads, kLevelThreads / 32 * words * 4, s, cx);
       small = std::min(n, 2 * 152u);  // the device knows how many there are
     }
   } else {
@@ -166,11 +167,11 @@ lucent_status gpu_build_bvh(const float* pos_d, uint32_t n, int max_leaf, int bi
   BB_CUDA(cudaFuncSetAttribute((const void*)k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sub_bytes(kSub, kMaxBins, kSubThreads)),
           "shared memory of the subtree kernel");
-  if (small) k_subtree<<<small, threads, smem, s>>>(cx);
+  if (small) launch_after(k_subtree, small, threads, smem, s, cx);
   const int g = (int)((nrec + 127) / 128);
   uint32_t* inner = (uint32_t*)b_inner.ptr;
   uint32_t* height = (uint32_t*)b_height.ptr;
-  k_tree_counts<<<g, 128, 0, s>>>(cx, (uint32_t*)b_arrived.ptr, inner, height, nrec);
+  launch_after(k_tree_counts, g, 128, 0, s, cx, (uint32_t*)b_arrived.ptr, inner, height, nrec);
   uint32_t root[2];
   float box[8];
   BB_CUDA(cudaMemcpyAsync(got, cx.ctr, sizeof got, cudaMemcpyDeviceToHost, s), "read counters");

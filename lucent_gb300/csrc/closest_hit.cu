@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(32) k_pick(TravArgs A, const __grid_constant__
 // arithmetic where its bound proves the roundings of all three, else from
 // binary64; prim becomes the triangle's source index. One thread per ray.
 __global__ void k_refine_api(ApiPolicy P) {
+  wait_for_previous();
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
     const int32_t code = P.prim[k];
     if (code > -3) continue;
@@ -352,8 +353,8 @@ void launch_closest(const Node* nodes, uint32_t node_count, const float4* tris, 
     if (wide) {
       A.queue = queue + n;
       A.queue_len = ctr + 4;
-      k_closest_wide_t<Listed><<<want < wide_blocks ? want : wide_blocks, ApiPolicy::kThreads, 0, s>>>(A, L);
-      k_closest_exact_t<Listed><<<grid_for(n < 4096 ? n : 4096, 128), 128, 0, s>>>(A, L);
+      launch_after(k_closest_wide_t<Listed>, want < wide_blocks ? want : wide_blocks, ApiPolicy::kThreads, 0, s, A, L);
+      launch_after(k_closest_exact_t<Listed>, grid_for(n < 4096 ? n : 4096, 128), 128, 0, s, A, L);
     } else {
       k_closest_fast_t<Listed, true><<<want < blocks ? want : blocks, ApiPolicy::kThreads, 0, s>>>(A, L);
     }
@@ -368,7 +369,7 @@ void launch_closest(const Node* nodes, uint32_t node_count, const float4* tris, 
     // Slow path over the rays the fast kernel queued (length read on the device).
     k_closest_exact_t<ApiPolicy><<<grid_for(n < 4096 ? n : 4096, 128), 128, 0, s>>>(A, P);
   }
-  k_refine_api<<<grid_for(n, 256), 256, 0, s>>>(P);
+  launch_after(k_refine_api, grid_for(n, 256), 256, 0, s, P);
 }
 
 void launch_wide_view(const Node* nodes, uint32_t node_count, Node* wide, cudaStream_t s) {

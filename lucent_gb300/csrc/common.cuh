@@ -105,4 +105,28 @@ enum : unsigned {
   kErrTree = 8u,        // a caller-supplied device tree failed its check (no-allocation entry point)
 };
 
+// First statement of every kernel that launch_after() may launch: waits until
+// the kernel before it has finished and its writes are visible.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Launches `kernel`, whose previous work on s is a kernel, before that one has
+// ended: what is left between the two is the wait above. For chains of short
+// kernels (4,099 rays: 78 -> 72 us a call; builds of 64,000 and 300,000
+// triangles 945 -> 837 us and 2.19 -> 2.04 ms). Kernels that let the next one's
+// blocks in while their own still run were slower where a second stream wants
+// the SMs (box frame 5.58 -> 5.88 ms).
+template <class... K, class... A>
+inline void launch_after(void (*kernel)(K...), dim3 grid, int block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &early;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
+}
+
 }  // namespace lucent

@@ -980,6 +980,7 @@ __global__ void k_zero_counters(uint32_t* ctr, int nxt) {
 // run on the side stream: the closest-hit counters before the closest hit,
 // the rest after the join.
 __global__ void k_zero_closest_counters(uint32_t* ctr) {
+  wait_for_previous();
   if (threadIdx.x == 0) {
     ctr[kCtrWork] = 0;
     ctr[kCtrSlow] = 0;
@@ -1095,6 +1096,7 @@ __global__ void k_sort_keys(Paths P, const SceneRec* __restrict__ recs, int n_cl
 // owns bins [w * 1024, (w + 1) * 1024), read 32 at a time (coalesced) and
 // scanned with shuffles; then the warp totals are scanned.
 __global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ hist) {
+  wait_for_previous();
   constexpr int kPerWarp = kSortBins / 32, kSteps = kPerWarp / 32;
   __shared__ uint32_t warp_total[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1133,6 +1135,7 @@ __global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ hist)
 // Copies each queued ray (read in queue order from the unsorted stream) to
 // its sorted position in the sorted stream, and the path to the sorted queue.
 __global__ void k_sort_scatter(Paths P, int nxt) {
+  wait_for_previous();
   const uint32_t n = P.ctr[kCtrQ0 + nxt];
   const uint32_t* q = P.q[nxt];
   const unsigned lane = threadIdx.x & 31;
@@ -1159,8 +1162,8 @@ static uint32_t* sort_rays(const MultiLaunch& M, Paths& P, int nxt, int blocks, 
   Ps.sort_tmp = dst;
   cudaMemsetAsync(P.sort_hist, 0, (size_t)kSortBins * 4, s);
   k_sort_keys<<<blocks, 256, 0, s>>>(Ps, M.recs, M.sort_classes > 0 ? M.sort_classes : M.n, nxt);
-  k_sort_scan<<<1, 1024, 0, s>>>(P.sort_hist);
-  k_sort_scatter<<<blocks, 256, 0, s>>>(Ps, nxt);
+  launch_after(k_sort_scan, 1, 1024, 0, s, P.sort_hist);
+  launch_after(k_sort_scatter, blocks, 256, 0, s, Ps, nxt);
   uint32_t* pre = P.q[nxt];
   P.q[nxt] = dst;
   return pre;
@@ -1214,13 +1217,14 @@ static void launch_closest_multi(const MultiLaunch& M, const Paths& P, const Tra
   if (M.near) {
     const int g = own > 0 ? own : G.near;
     if (M.n == 1)
-      k_closest_near_t<PathClosestOne><<<g, PathClosestOne::kNearThreads, 0, s>>>(one_scene(M, A), PathClosestOne{pc});
+      launch_after(k_closest_near_t<PathClosestOne>, g, PathClosestOne::kNearThreads, 0, s, one_scene(M, A), PathClosestOne{pc});
     else
-      k_closest_near_t<PathClosestMulti><<<g, PathClosestMulti::kNearThreads, 0, s>>>(A, pc);
+      launch_after(k_closest_near_t<PathClosestMulti>, g, PathClosestMulti::kNearThreads, 0, s, A, pc);
     TravArgs R = A;
     R.work = P.ctr + kCtrRestWork;
     using Listed = Queued<PathClosestMulti>;
-    k_closest_wide_t<Listed, true><<<own > 0 ? own : G.wide, PathClosestMulti::kThreads, 0, s>>>(R, Listed{pc, A.queue, A.queue_len});
+    launch_after(k_closest_wide_t<Listed, true>, own > 0 ? own : G.wide, PathClosestMulti::kThreads, 0, s, R,
+                 Listed{pc, A.queue, A.queue_len});
     return;
   }
   if (M.wide)
@@ -1242,7 +1246,7 @@ static void launch_shadow_multi(const MultiLaunch& M, int blocks, const TravArgs
     k_anyhit_wide_t<PathShadowMulti><<<blocks, 256, 0, s>>>(A, ps);
   else
     k_anyhit_fast_t<PathShadowMulti><<<blocks, 256, top_smem_bytes(A.top_scenes), s>>>(A, ps);
-  k_anyhit_exact_t<PathShadowMulti><<<64, 128, 0, s>>>(A, ps);
+  launch_after(k_anyhit_exact_t<PathShadowMulti>, 64, 128, 0, s, A, ps);
 }
 
 int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, bool accumulate) {
@@ -1265,7 +1269,7 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
   for (int b = 0; b <= M.max_bounces; b++) {
     const int cur = b & 1;
     if (forked)  // the side stream still reads the other counters
-      k_zero_closest_counters<<<1, 32, 0, s>>>(P.ctr);
+      launch_after(k_zero_closest_counters, 1, 32, 0, s, P.ctr);
     else
       k_zero_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
     nl++;
@@ -1366,7 +1370,7 @@ void render_backward(const MultiLaunch& M, const AdjointDevHost& H, cudaStream_t
   for (int b = 0; b <= M.max_bounces; b++) {
     const int cur = b & 1;
     if (forked)
-      k_zero_closest_counters<<<1, 32, 0, s>>>(P.ctr);
+      launch_after(k_zero_closest_counters, 1, 32, 0, s, P.ctr);
     else
       k_zero_counters<<<1, 32, 0, s>>>(P.ctr, cur ^ 1);
     PathClosestMulti pc{P.ctr + kCtrQ0 + cur, sorted ? P.sray : P.nray, P.ro, P.hit, M.recs, M.any_alpha};

@@ -259,6 +259,7 @@ __device__ __forceinline__ void closest_exact_ray(const TravArgs& A, const Pol& 
 
 template <class Pol>
 __global__ void k_closest_exact_t(TravArgs A, Pol P) {
+  wait_for_previous();
   const uint32_t limit = A.queue ? *A.queue_len : P.count();
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < limit; q += gridDim.x * blockDim.x)
     closest_exact_ray(A, P, A.queue ? A.queue[q] : q);
@@ -555,6 +556,7 @@ __device__ bool any_exact(const TravArgs& A, const Pol& P, const BvhView& bv, D3
 // Any-hit rays carry their own tMax: P.tmax32(k).
 template <class Pol>
 __global__ void k_anyhit_exact_t(TravArgs A, Pol P) {
+  wait_for_previous();
   const uint32_t limit = *A.queue_len;
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < limit; q += gridDim.x * blockDim.x) {
     const uint32_t k = A.queue[q];

@@ -237,6 +237,7 @@ LUCENT_DEV bool near_ray_ok(float3 o, float3 d, const NearView& v, float& grow) 
 // 1080p 4-spp frame over 2 M triangles (14.7 M rays) 25.5 -> 9.4 ms.
 template <class Pol>
 __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest_near_t(TravArgs A, const __grid_constant__ Pol P) {
+  wait_for_previous();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -438,6 +439,7 @@ __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest
 // for an accepted triangle only.
 template <class Pol>
 __global__ void __launch_bounds__(kAnyThreads, kAnyBlocks) k_anyhit_near_t(TravArgs A, const __grid_constant__ Pol P) {
+  wait_for_previous();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;

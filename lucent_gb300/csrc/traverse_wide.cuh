@@ -132,6 +132,7 @@ static __device__ __noinline__ Closest closest_exact(Closest s, float3 o, float3
 template <class Pol, bool Rest = false>
 __global__ void __launch_bounds__(Pol::kThreads, Pol::kMinBlocks)
     k_closest_wide_t(const __grid_constant__ TravArgs A, const __grid_constant__ Pol P) {
+  wait_for_previous();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
