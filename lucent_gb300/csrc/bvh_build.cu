@@ -1068,9 +1068,7 @@ __global__ void k_tree_counts(Ctx cx, uint32_t* __restrict__ arrived, uint32_t* 
     x = up - 1;
     const uint32_t l = (uint32_t)__float_as_int(cx.recs[2 * (size_t)x].w);
     up = cx.parent[x];
-    uint32_t before;  // orders this child's counts before, the other's after
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(arrived + x) : "memory");
-    if (before == 0) return;
+    if (arrive(arrived + x) == 0) return;
     const uint32_t n = __ldcg(inner + l) + __ldcg(inner + l + 1), h = max(__ldcg(height + l), __ldcg(height + l + 1));
     __stcg(inner + x, 1 + n);
     __stcg(height + x, 1 + h);

@@ -105,6 +105,14 @@ enum : unsigned {
   kErrTree = 8u,        // a caller-supplied device tree failed its check (no-allocation entry point)
 };
 
+// Counts this arrival at *p and returns those before it; what this thread wrote
+// is visible to the later ones, what the earlier ones wrote to it.
+__device__ __forceinline__ uint32_t arrive(uint32_t* p) {
+  uint32_t before;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(p) : "memory");
+  return before;
+}
+
 // First statement of every kernel that launch_after() may launch: waits until
 // the kernel before it has finished and its writes are visible.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
