@@ -166,7 +166,9 @@ struct lucent_bvh {
   // 64-entry stack take the all-binary64 path, which reproduces the overflow.
   uint32_t depth = 0;
   int mode = LUCENT_TRAVERSE_WIDE;
-  DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch, stage{nullptr, 0, true};
+  // From the pool: with everything else pooled, a cudaMalloc of the scratch maps
+  // a new 2 MiB block (100 us of a new tree's first query).
+  DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch{nullptr, 0, true}, stage{nullptr, 0, true};
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // the root's box
   NearTree near;       // nearest-first view (LUCENT_TRAVERSE_WIDE, where usable), built on first use
   bool near_tried = false;
