@@ -45,7 +45,8 @@ __device__ float leaf_growth(float4 a, float4 b, float4 c, float s, float& rise)
 }
 
 // Parents, and the checks that the traversal's argument needs: one parent per
-// node, child boxes inside their parent's, leaves the reference can hold.
+// node (k_near_leaves sees to it that there is one), child boxes inside their
+// parent's, leaves the reference can hold.
 __global__ void k_near_parents(const Node* __restrict__ nodes, uint32_t n_nodes, uint32_t* __restrict__ parent,
                                uint32_t* __restrict__ words) {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,6 +77,13 @@ __global__ void k_near_leaves(const Node* __restrict__ nodes, uint32_t n_nodes, 
   wait_for_previous();
   uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= n_nodes) return;
+  if (n > 0 && parent[n] == 0) {
+    // Outside the tree (children have higher indices than their parent, so all
+    // that has one hangs below the root or below such a node): none of its
+    // boxes bounds what the reference visits, but a leaf would claim its slots.
+    atomicOr(words + kNearBad, 1u);
+    return;
+  }
   const Node nd = load_node(nodes, n);
   const int cnt = node_count(nd), f = node_first(nd);
   if (cnt == 0) return;
