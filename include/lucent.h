@@ -86,10 +86,10 @@ lucent_status lucent_bvh_info(const lucent_bvh* bvh, uint32_t* node_count, uint3
  * 2 = mode 0 reading every node from global memory, 3 = nearest first over a
  * four-wide view of the tree, each hit checked against the reference's
  * decisions and the rays that the check leaves open traced as in mode 0 (the
- * default; 128 bytes per node and 4 per triangle, built on the first call,
- * which then waits; a first call inside a stream capture, a tree that is not
- * the builder's kind, or rays far from it take a four-wide view in mode 0's
- * order). All return identical results. lucent_bvh_intersect_noalloc always uses 0. */
+ * default; 128 bytes per node and 4 per triangle, built on the first call
+ * outside a stream capture, which waits for them; a call captured before that
+ * traverses as mode 0; a tree that is not the builder's kind, or rays far from
+ * it take a four-wide view in mode 0's order). All return identical results. lucent_bvh_intersect_noalloc always uses 0. */
 #define LUCENT_TRAVERSE_FAST 0
 #define LUCENT_TRAVERSE_EXACT 1
 #define LUCENT_TRAVERSE_FAST_GLOBAL 2
@@ -102,8 +102,9 @@ lucent_status lucent_bvh_set_mode(lucent_bvh* bvh, int32_t mode);
  * t_out, u_out, v_out may be NULL. */
 lucent_status lucent_bvh_intersect(lucent_bvh* bvh, const float* rays, uint32_t n, double t_min, double t_max,
                                    int32_t* prim_out, float* t_out, float* u_out, float* v_out, void* stream);
-/* Same with device pointers; asynchronous. Errors raised by the kernels are
- * reported by lucent_bvh_check(). */
+/* Same with device pointers; asynchronous, but for the first call with a
+ * tree, which waits for its views (lucent_bvh_set_mode). Errors raised by the
+ * kernels are reported by lucent_bvh_check(). */
 lucent_status lucent_bvh_intersect_device(lucent_bvh* bvh, const float* rays_d, uint32_t n, double t_min,
                                           double t_max, int32_t* prim_d, float* t_d, float* u_d, float* v_d,
                                           void* stream);

@@ -90,7 +90,8 @@ class DeviceBVH:
 
     def intersect_device(self, rays_ptr, n, prim_ptr, t_ptr=None, u_ptr=None, v_ptr=None, t_min=1e-5,
                          t_max=math.inf, stream=None):
-        """Asynchronous form on device pointers (ints); call check() to synchronise."""
+        """Asynchronous form on device pointers (ints; a tree's first call waits for its views); call check() to
+        synchronise."""
         N.check(N.lib().lucent_bvh_intersect_device(self._h, rays_ptr, n, t_min, t_max, prim_ptr, t_ptr, u_ptr,
                                                     v_ptr, stream))
 

@@ -173,6 +173,7 @@ struct lucent_bvh {
   NearTree near;       // nearest-first view (LUCENT_TRAVERSE_WIDE, where usable), built on first use
   bool near_tried = false;
   DeviceBuffer wide{nullptr, 0, true};  // four-wide view of `nodes` (LUCENT_TRAVERSE_WIDE otherwise), built on first use
+  bool views = false;  // what LUCENT_TRAVERSE_WIDE reads has been built, and is there for every stream
 };
 
 static void set_root(lucent_bvh* b, const float* nodes) {
@@ -404,6 +405,27 @@ static lucent_status prepare_scratch(lucent_bvh* b, uint32_t n, cudaStream_t s, 
   return LUCENT_OK;
 }
 
+// The views of LUCENT_TRAVERSE_WIDE, outside any capture; returns when they
+// are complete, as the next call may come on another stream.
+static lucent_status build_views(lucent_bvh* b, cudaStream_t s) {
+  lucent_status st;
+  if (!b->near_tried) {
+    if ((st = build_near_view((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, b->tri_count, b->lo,
+                              b->hi, b->near, s)))
+      return st;
+    b->near_tried = true;
+  }
+  if (!(b->near.usable && b->near.wide_range)) {
+    if ((st = b->wide.reserve((size_t)b->node_count * 4 * sizeof(Node)))) return st;
+    launch_wide_view((const Node*)b->nodes.ptr, b->node_count, (Node*)b->wide.ptr, s);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(e, "four-wide view");
+  }
+  b->views = true;
+  return LUCENT_OK;
+}
+
 lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, uint32_t n, double t_min,
                                           double t_max, int32_t* prim_d, float* t_d, float* u_d, float* v_d,
                                           void* stream) {
@@ -419,30 +441,19 @@ lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, ui
     cudaError_t e = cudaMemsetAsync(prim_d, 0xff, (size_t)n * 4, s);
     return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "memset");
   }
-  const Node* wide = nullptr;
-  if (b->mode == LUCENT_TRAVERSE_WIDE && !b->near_tried) {
-    // Building the view waits for its verdict, which a capture cannot: the
-    // captured call then takes the four-wide view.
+  if (b->mode == LUCENT_TRAVERSE_WIDE && !b->views) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(s, &cap);
-    if (cap == cudaStreamCaptureStatusNone) {
-      if ((st = build_near_view((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, b->tri_count,
-                                b->lo, b->hi, b->near, s)))
-        return st;
-      b->near_tried = true;
-    }
+    if (cudaError_t e = cudaStreamIsCapturing(s, &cap); e != cudaSuccess) return cuda_fail(e, "stream");
+    if (cap == cudaStreamCaptureStatusNone && (st = build_views(b, s))) return st;
   }
-  const bool near = b->mode == LUCENT_TRAVERSE_WIDE && b->near.usable;
-  if (b->mode == LUCENT_TRAVERSE_WIDE && !(near && b->near.wide_range)) {
-    if (!b->wide.ptr) {
-      if ((st = b->wide.reserve((size_t)b->node_count * 4 * sizeof(Node)))) return st;
-      launch_wide_view((const Node*)b->nodes.ptr, b->node_count, (Node*)b->wide.ptr, s);
-    }
-    wide = (const Node*)b->wide.ptr;
-  }
+  // Without them, in a capture, as mode 0: what a capture records has not run
+  // by the next call, so no view can be built in one.
+  const bool views = b->mode == LUCENT_TRAVERSE_WIDE && b->views;
+  const bool near = views && b->near.usable;
+  const Node* wide = views && !(near && b->near.wide_range) ? (const Node*)b->wide.ptr : nullptr;
+  const bool top = b->mode == LUCENT_TRAVERSE_FAST || (b->mode == LUCENT_TRAVERSE_WIDE && !b->views);
   launch_closest((const Node*)b->nodes.ptr, b->node_count, (const float4*)b->tris.ptr, rays_d, n, t_min, t_max, prim_d, t_d, u_d,
-                 v_d, queue, ctr, b->mode == LUCENT_TRAVERSE_EXACT || b->depth + 2 > kTsStack, b->mode == LUCENT_TRAVERSE_FAST, s,
-                 wide, near ? &b->near : nullptr);
+                 v_d, queue, ctr, b->mode == LUCENT_TRAVERSE_EXACT || b->depth + 2 > kTsStack, top, s, wide, near ? &b->near : nullptr);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "closest-hit launch");
 }
