@@ -54,22 +54,26 @@ uint64_t first_not_finite(const float* v, uint64_t n) {
   return n;
 }
 
-// The pool of the current device for the memory of single calls and of BVH
-// handles: cudaMalloc and cudaFree of a build's buffers cost as much as a small
+// The pool of a device for the memory of single calls and of BVH handles:
+// cudaMalloc and cudaFree of a build's buffers cost as much as a small
 // build (the last cudaFree of a 2 MiB block alone some 180 us). Stream-ordered,
 // so threads and streams share it safely; it holds at most 1 GiB between calls
 // (the driver takes back what is free beyond that), and gives what is free
 // back when an ordinary allocation fails or a renderer is trimmed. `stream`:
 // the pool's own, for allocations that outlive a call.
 struct Pool {
+  int device = 0;
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
+  std::mutex lock;
+  std::vector<void*> waiting;  // of closed handles, until the device can be waited for
+  void give_waiting_back();
 };
-static Pool device_pool() {
+static Pool* device_pool() {  // of the current device
   static std::mutex lock;
-  static Pool pools[64];
+  static Pool* const pools = new Pool[64];  // never destroyed: handles may outlive any static object
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return {};
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> hold(lock);
   Pool& P = pools[dev];
   if (!P.pool) {
@@ -77,31 +81,123 @@ static Pool device_pool() {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    Pool made;
-    if (cudaStreamCreateWithFlags(&made.stream, cudaStreamNonBlocking) != cudaSuccess) return {};
-    if (cudaMemPoolCreate(&made.pool, &props) != cudaSuccess) {
-      cudaStreamDestroy(made.stream);
-      return {};
+    cudaStream_t stream;
+    if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+    if (cudaMemPoolCreate(&P.pool, &props) != cudaSuccess) {
+      cudaStreamDestroy(stream);
+      P.pool = nullptr;
+      return nullptr;
     }
     uint64_t keep = 1ull << 30;
-    cudaMemPoolSetAttribute(made.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    P = made;
+    cudaMemPoolSetAttribute(P.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    P.device = dev;
+    P.stream = stream;
   }
-  return P;
+  return &P;
+}
+
+std::shared_mutex& capture_lock() {
+  static std::shared_mutex* const m = new std::shared_mutex;
+  return *m;
+}
+
+// Blocks that no event stands for are given back once their device has been
+// waited for, as cudaFree would; where that is refused, they stay for the next time.
+void Pool::give_waiting_back() {
+  std::lock_guard<std::mutex> hold(lock);
+  if (waiting.empty()) return;
+  std::unique_lock<std::shared_mutex> no_capture(capture_lock(), std::try_to_lock);
+  if (!no_capture) return;
+  int before = 0;
+  cudaError_t e = cudaGetDevice(&before);
+  if (e == cudaSuccess && before != device) e = cudaSetDevice(device);
+  if (e == cudaSuccess) {
+    e = cudaDeviceSynchronize();
+    if (before != device) cudaSetDevice(before);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  for (void* p : waiting) cudaFreeAsync(p, stream);
+  waiting.clear();
+}
+
+lucent_status StreamUses::begin(cudaStream_t s) {
+  unsigned long long id = 0;
+  if (cudaError_t e = cudaStreamGetId(s, &id); e != cudaSuccess) return cuda_fail(e, "stream");
+  for (size_t k = 0; k < uses.size(); k++)
+    if (uses[k].stream == id) {
+      std::swap(uses[k], uses.back());
+      return LUCENT_OK;
+    }
+  if (uses.size() < 4) {
+    cudaEvent_t event;
+    if (cudaError_t e = cudaEventCreateWithFlags(&event, cudaEventDisableTiming); e != cudaSuccess)
+      return cuda_fail(e, "event");
+    uses.push_back({id, event, false});
+  } else {
+    Use& u = uses.front();
+    if (u.open && cudaStreamWaitEvent(home->stream, u.event, 0) != cudaSuccess) {
+      cudaGetLastError();
+      unordered = true;
+    }
+    u.stream = id;
+    u.open = false;
+    std::swap(u, uses.back());
+  }
+  return LUCENT_OK;
+}
+
+lucent_status StreamUses::end(cudaStream_t s) {
+  uses.back().open = true;
+  const cudaError_t e = cudaEventRecord(uses.back().event, s);
+  if (e == cudaSuccess) return LUCENT_OK;
+  unordered = true;
+  return cuda_fail(e, "event");
+}
+
+void StreamUses::give_back(void* ptr, bool held) {
+  if (!held && !unordered) {
+    bool ok = true;
+    for (Use& u : uses) {
+      if (u.open) ok = cudaStreamWaitEvent(home->stream, u.event, 0) == cudaSuccess && ok;
+      u.open = false;
+    }
+    if (ok && cudaFreeAsync(ptr, home->stream) == cudaSuccess) return;
+    cudaGetLastError();
+    unordered = true;
+  }
+  kept.push_back(ptr);
+}
+
+void StreamUses::close() {
+  for (Use& u : uses) cudaEventDestroy(u.event);
+  uses.clear();
+  if (!home) return;
+  {
+    std::lock_guard<std::mutex> hold(home->lock);
+    home->waiting.insert(home->waiting.end(), kept.begin(), kept.end());
+  }
+  kept.clear();
+  home->give_waiting_back();
 }
 
 void trim_temporaries() {
-  if (cudaMemPool_t p = device_pool().pool) cudaMemPoolTrimTo(p, 0);
+  if (Pool* P = device_pool()) {
+    P->give_waiting_back();
+    cudaMemPoolTrimTo(P->pool, 0);
+  }
 }
 
-static lucent_status pool_alloc(void** ptr, size_t bytes, const Pool& P, cudaStream_t s) {
+static lucent_status pool_alloc(void** ptr, size_t bytes, const Pool* P, cudaStream_t s) {
   *ptr = nullptr;
-  if (!P.pool) return cuda_fail(cudaGetLastError(), "memory pool");
-  cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, P.pool, s);
+  if (!P) return cuda_fail(cudaGetLastError(), "memory pool");
+  cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, P->pool, s);
   if (e == cudaErrorMemoryAllocation) {  // once more without what the pool holds
     cudaGetLastError();
     trim_temporaries();
-    e = cudaMallocFromPoolAsync(ptr, bytes, P.pool, s);
+    e = cudaMallocFromPoolAsync(ptr, bytes, P->pool, s);
   }
   if (e == cudaSuccess) return LUCENT_OK;
   *ptr = nullptr;
@@ -123,10 +219,12 @@ lucent_status DeviceBuffer::reserve(size_t bytes) {
   if (bytes <= cap) return LUCENT_OK;
   release();
   const size_t want = bytes < 256 ? 256 : bytes;
-  if (pooled) {  // allocated on the pool's stream and waited for: usable on any stream
-    const Pool P = device_pool();
-    if (lucent_status st = pool_alloc(&ptr, want, P, P.stream)) return st;
-    if (cudaError_t e = cudaStreamSynchronize(P.stream); e != cudaSuccess) {
+  if (uses) {  // allocated on the pool's stream and waited for: usable on any stream
+    if (!uses->home) uses->home = device_pool();
+    const Pool* P = uses->home;
+    if (lucent_status st = pool_alloc(&ptr, want, P, P ? P->stream : nullptr)) return st;
+    if (cudaError_t e = cudaStreamSynchronize(P->stream); e != cudaSuccess) {
+      cudaFreeAsync(ptr, P->stream);
       ptr = nullptr;
       return cuda_fail(e, "pool allocation");
     }
@@ -148,14 +246,13 @@ lucent_status DeviceBuffer::reserve(size_t bytes) {
 }
 
 void DeviceBuffer::release() {
-  if (ptr && pooled) {
-    cudaDeviceSynchronize();  // as cudaFree does: no stream still uses it
-    if (const Pool P = device_pool(); P.stream) cudaFreeAsync(ptr, P.stream);
-  } else if (ptr) {
+  if (ptr && uses)
+    uses->give_back(ptr, held);
+  else if (ptr)
     cudaFree(ptr);
-  }
   ptr = nullptr;
   cap = 0;
+  held = false;
 }
 
 }  // namespace lucent
@@ -166,13 +263,14 @@ struct lucent_bvh {
   // 64-entry stack take the all-binary64 path, which reproduces the overflow.
   uint32_t depth = 0;
   int mode = LUCENT_TRAVERSE_WIDE;
+  StreamUses uses;
   // From the pool: with everything else pooled, a cudaMalloc of the scratch maps
   // a new 2 MiB block (100 us of a new tree's first query).
-  DeviceBuffer nodes{nullptr, 0, true}, tris{nullptr, 0, true}, scratch{nullptr, 0, true}, stage{nullptr, 0, true};
+  DeviceBuffer nodes{nullptr, 0, &uses}, tris{nullptr, 0, &uses}, scratch{nullptr, 0, &uses}, stage{nullptr, 0, &uses};
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // the root's box
-  NearTree near;       // nearest-first view (LUCENT_TRAVERSE_WIDE, where usable), built on first use
+  NearTree near{&uses};  // nearest-first view (LUCENT_TRAVERSE_WIDE, where usable), built on first use
   bool near_tried = false;
-  DeviceBuffer wide{nullptr, 0, true};  // four-wide view of `nodes` (LUCENT_TRAVERSE_WIDE otherwise), built on first use
+  DeviceBuffer wide{nullptr, 0, &uses};  // four-wide view of `nodes` (LUCENT_TRAVERSE_WIDE otherwise), built on first use
   bool views = false;  // what LUCENT_TRAVERSE_WIDE reads has been built, and is there for every stream
 };
 
@@ -248,7 +346,10 @@ lucent_status lucent_bvh_create(const float* nodes, uint32_t node_count, const u
     ref.release();
     pos.release();
     idx.release();
-    if (code) lucent_bvh_destroy(b);
+    if (code) {
+      b->uses.unordered = true;
+      lucent_bvh_destroy(b);
+    }
     return code;
   };
   if ((st = b->nodes.reserve((size_t)node_count * sizeof(Node)))) return cleanup(st);
@@ -288,6 +389,7 @@ static lucent_status build_common(const float* pos_d, uint32_t n, const lucent_b
   out.tri_host = tri_out;
   lucent_status st = gpu_build_bvh(pos_d, n, max_leaf, bins, s, out);
   if (st) {
+    if (b) b->uses.unordered = true;
     lucent_bvh_destroy(b);
     return st;
   }
@@ -351,6 +453,7 @@ void lucent_bvh_destroy(lucent_bvh* b) {
   b->stage.release();
   b->wide.release();
   b->near.release();
+  b->uses.close();
   delete b;
 }
 
@@ -426,14 +529,11 @@ static lucent_status build_views(lucent_bvh* b, cudaStream_t s) {
   return LUCENT_OK;
 }
 
-lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, uint32_t n, double t_min,
-                                          double t_max, int32_t* prim_d, float* t_d, float* u_d, float* v_d,
-                                          void* stream) {
-  clear_error();
-  if (!b || (n && (!rays_d || !prim_d))) return fail(LUCENT_ERR_INVALID, "null argument");
-  lucent_status st = check_tmin(t_min, t_max);
-  if (st) return st;
-  cudaStream_t s = (cudaStream_t)stream;
+// Queues one call's work on s.
+static lucent_status intersect_queue(lucent_bvh* b, const float* rays_d, uint32_t n, double t_min, double t_max,
+                                     int32_t* prim_d, float* t_d, float* u_d, float* v_d, cudaStream_t s,
+                                     bool capturing) {
+  lucent_status st;
   uint32_t *ctr, *queue;
   if ((st = prepare_scratch(b, n, s, &ctr, &queue))) return st;
   if (n == 0) return LUCENT_OK;
@@ -441,11 +541,7 @@ lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, ui
     cudaError_t e = cudaMemsetAsync(prim_d, 0xff, (size_t)n * 4, s);
     return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "memset");
   }
-  if (b->mode == LUCENT_TRAVERSE_WIDE && !b->views) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaError_t e = cudaStreamIsCapturing(s, &cap); e != cudaSuccess) return cuda_fail(e, "stream");
-    if (cap == cudaStreamCaptureStatusNone && (st = build_views(b, s))) return st;
-  }
+  if (b->mode == LUCENT_TRAVERSE_WIDE && !b->views && !capturing && (st = build_views(b, s))) return st;
   // Without them, in a capture, as mode 0: what a capture records has not run
   // by the next call, so no view can be built in one.
   const bool views = b->mode == LUCENT_TRAVERSE_WIDE && b->views;
@@ -456,6 +552,27 @@ lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, ui
                  v_d, queue, ctr, b->mode == LUCENT_TRAVERSE_EXACT || b->depth + 2 > kTsStack, top, s, wide, near ? &b->near : nullptr);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? LUCENT_OK : cuda_fail(e, "closest-hit launch");
+}
+
+lucent_status lucent_bvh_intersect_device(lucent_bvh* b, const float* rays_d, uint32_t n, double t_min,
+                                          double t_max, int32_t* prim_d, float* t_d, float* u_d, float* v_d,
+                                          void* stream) {
+  clear_error();
+  if (!b || (n && (!rays_d || !prim_d))) return fail(LUCENT_ERR_INVALID, "null argument");
+  lucent_status st = check_tmin(t_min, t_max);
+  if (st) return st;
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaError_t e = cudaStreamIsCapturing(s, &cap); e != cudaSuccess) return cuda_fail(e, "stream");
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  if (!capturing && (st = b->uses.begin(s))) return st;
+  st = intersect_queue(b, rays_d, n, t_min, t_max, prim_d, t_d, u_d, v_d, s, capturing);
+  if (capturing) {  // the graph holds these from now on
+    for (DeviceBuffer* m : {&b->nodes, &b->tris, &b->scratch, &b->wide, &b->near.records, &b->near.leaf_of}) m->held = true;
+    return st;
+  }
+  const lucent_status end = b->uses.end(s);
+  return st ? st : end;
 }
 
 static lucent_status device_error(unsigned word) {
@@ -504,7 +621,10 @@ lucent_status lucent_bvh_intersect(lucent_bvh* b, const float* rays, uint32_t n,
   if (e == cudaSuccess && t_out) e = cudaMemcpyAsync(t_out, t_d, ob, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && u_out) e = cudaMemcpyAsync(u_out, u_d, ob, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && v_out) e = cudaMemcpyAsync(v_out, v_d, ob, cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return cuda_fail(e, "download hits");
+  if (e != cudaSuccess) {
+    b->uses.unordered = true;
+    return cuda_fail(e, "download hits");
+  }
   if (b->tri_count == 0 && t_out)
     for (uint32_t i = 0; i < n; i++) t_out[i] = INFINITY;
   return lucent_bvh_check(b, stream);
@@ -546,7 +666,10 @@ lucent_status lucent_bvh_intersect_f64(lucent_bvh* b, const double* rays, uint32
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(hits, hits_d, hb, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_fail(e, "f64 closest-hit");
+    if (e != cudaSuccess) {
+      b->uses.unordered = true;
+      return cuda_fail(e, "f64 closest-hit");
+    }
     unsigned word = 0;
     for (uint32_t i = 0; i < n; i++) {
       prim_out[i] = hits[i].prim;
@@ -575,7 +698,10 @@ lucent_status lucent_bvh_intersect_f64(lucent_bvh* b, const double* rays, uint32
   if (e == cudaSuccess) e = cudaMemcpyAsync(t_out, t_d, ob, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(u_out, u_d, ob, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(v_out, v_d, ob, cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return cuda_fail(e, "f64 closest-hit");
+  if (e != cudaSuccess) {
+    b->uses.unordered = true;
+    return cuda_fail(e, "f64 closest-hit");
+  }
   return lucent_bvh_check(b, stream);
 }
 

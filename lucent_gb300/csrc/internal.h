@@ -45,7 +45,8 @@ void launch_closest_d(const Node* nodes, uint32_t node_count, const float4* tris
 // distance. Not usable (and empty) for trees the argument does not
 // cover. `tris`: slot order, 3 float4 each; lo, hi: the root's box.
 struct NearTree {
-  DeviceBuffer records{nullptr, 0, true}, leaf_of{nullptr, 0, true};
+  explicit NearTree(StreamUses* uses = nullptr) : records{nullptr, 0, uses}, leaf_of{nullptr, 0, uses} {}
+  DeviceBuffer records, leaf_of;
   float4 bound = {0.f, 0.f, 0.f, 0.f};  // centre, radius
   float2 far = {0.f, 0.f};              // from this distance on, growth per unit of distance
   bool wide_range = false;              // the radius is 64 diagonals or more

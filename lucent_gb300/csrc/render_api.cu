@@ -200,10 +200,13 @@ struct WaveGraph {
       drop();
       if (!cap && (e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)) != cudaSuccess)
         return cuda_fail(e, "capture stream");
-      if ((e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-        return cuda_fail(e, "begin capture");
-      launches = render_wave_multi(M, cap, nullptr, accumulate);
-      e = cudaStreamEndCapture(cap, &graph);
+      {
+        std::shared_lock<std::shared_mutex> capturing(capture_lock());
+        if ((e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
+          return cuda_fail(e, "begin capture");
+        launches = render_wave_multi(M, cap, nullptr, accumulate);
+        e = cudaStreamEndCapture(cap, &graph);
+      }
       if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
       if (e != cudaSuccess) {
         drop();
