@@ -256,7 +256,9 @@ typedef struct lucent_render_stats {
 
 lucent_status lucent_renderer_create(uint32_t width, uint32_t height, lucent_renderer** out);
 void lucent_renderer_destroy(lucent_renderer* r);
-/* loadScene(scene, bvh?) (renderer.ts:279-312). */
+/* loadScene(scene, bvh?) (renderer.ts:279-312). A load that fails while the
+ * scene is built or copied (not: a description that is refused) leaves the
+ * renderer without one. */
 lucent_status lucent_renderer_load_scene(lucent_renderer* r, const lucent_scene_desc* scene);
 lucent_status lucent_renderer_upload_lighting(lucent_renderer* r, const lucent_lighting* lighting);
 /* buildEnvSampler(img, maxWidth) (src/scene/environment.ts:52-85, with

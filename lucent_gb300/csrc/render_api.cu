@@ -791,6 +791,9 @@ lucent_status lucent_renderer_load_scene(lucent_renderer* r, const lucent_scene_
   if (d->uvs && (st = upload(uvs, d->uvs, (size_t)n * 24))) return cleanup(st);
   if (d->tri_light && (st = upload(lgt, d->tri_light, (size_t)n * 4))) return cleanup(st);
   if (d->tri_alpha && (st = upload(alp, d->tri_alpha, (size_t)n))) return cleanup(st);
+  // From here on the last scene's memory is overwritten piece by piece: after a
+  // failure there is no scene, rather than one's tree with the other's views.
+  r->has_scene = false;
   uint32_t nc, depth;
   float root[6];
   if (d->bvh_nodes) {

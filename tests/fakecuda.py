@@ -10,6 +10,7 @@ import types
 import numpy as np
 
 from lucent_gb300 import _native as N
+from lucent_gb300 import _native_render as R
 from lucent_gb300 import build as B
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -116,3 +117,28 @@ def intersect(b, n, s=None):
     mem = [np.zeros(max(1, n) * w, np.float32) for w in (6, 1, 1, 1, 1)]
     return L.lucent_bvh_intersect_device(b.h, mem[0].ctypes.data, n, 0.0, float("inf"), *(m.ctypes.data for m in mem[1:]),
                                          s)
+
+
+def renderer(w=8, h=8):
+    L = library()
+    r = C.c_void_p()
+    assert L.lucent_renderer_create(w, h, C.byref(r)) == 0, L.lucent_last_error()
+    env = np.ones((4, 8, 3), np.float32)
+    light = R.LightingDesc(env_width=8, env_height=4, env_rgb=N.ptr(env, C.c_float), env_rotation_cos=1.0,
+                           env_intensity=1.0)
+    assert L.lucent_renderer_upload_lighting(r, C.byref(light)) == 0, L.lucent_last_error()
+    return r
+
+
+def load_scene(r, pos, nodes=None, **more):
+    """Loads triangles with their tree (halved in order unless given) and a grey material; the call's status."""
+    L = library()
+    n = len(pos)
+    nodes = tree(pos) if nodes is None else nodes
+    idx, mat, grey = np.arange(n, dtype=np.uint32), np.zeros(n, np.int32), np.zeros(40, np.float32)
+    grey[:3], grey[16:20] = 0.5, -1
+    d = R.SceneDesc(tri_count=n, positions=N.ptr(pos, C.c_float), normals=N.ptr(pos, C.c_float),
+                    tri_material=N.ptr(mat, C.c_int32), bvh_nodes=N.ptr(nodes, C.c_float),
+                    bvh_node_count=nodes.size // 8, bvh_tri_indices=N.ptr(idx, C.c_uint32),
+                    materials=N.ptr(grey, C.c_float), material_count=1, ground_material=-1, **more)
+    return L.lucent_renderer_load_scene(r, C.byref(d))
