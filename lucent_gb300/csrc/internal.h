@@ -43,7 +43,7 @@ void launch_closest_d(const Node* nodes, uint32_t node_count, const float4* tris
 // each slot's leaf, the centre of the tree with the radius within which ray
 // origins may lie, and how the box growth for farther origins rises with their
 // distance. Not usable (and empty) for trees the argument does not
-// cover. `tris`: slot order, 3 float4 each; lo, hi: the root's box.
+// cover, and where there is no memory for it. `tris`: slot order, 3 float4 each; lo, hi: the root's box.
 struct NearTree {
   explicit NearTree(StreamUses* uses = nullptr) : records{nullptr, 0, uses}, leaf_of{nullptr, 0, uses} {}
   DeviceBuffer records, leaf_of;

@@ -182,12 +182,16 @@ lucent_status build_near_view(const Node* nodes, uint32_t n_nodes, const float4*
   const float mag = fmaxf(fmaxf(fabsf(c[0]), fabsf(c[1])), fabsf(c[2]));
   if (!(mag < 1e3f * diag)) return LUCENT_OK;
   lucent_status st;
-  if ((st = out.records.reserve((size_t)n_nodes * kWide * sizeof(Node))) ||
-      (st = out.leaf_of.reserve((size_t)n_tris * 4)))
-    return st;
   TempBuffer tmp;
   const size_t cull = (size_t)n_nodes * sizeof(Node), idx = (size_t)n_nodes * 4;
-  if ((st = tmp.reserve(cull + 3 * idx + 64, s))) return st;
+  if ((st = out.records.reserve((size_t)n_nodes * kWide * sizeof(Node))) ||
+      (st = out.leaf_of.reserve((size_t)n_tris * 4)) || (st = tmp.reserve(cull + 3 * idx + 64, s))) {
+    out.release();
+    if (st != LUCENT_ERR_OOM) return st;
+    cudaGetLastError();  // no room for it: not usable, and nothing else is wrong
+    clear_error();
+    return LUCENT_OK;
+  }
   char* b = (char*)tmp.ptr;
   uint32_t* parent = (uint32_t*)(b + cull);
   uint32_t* arrived = parent + n_nodes;

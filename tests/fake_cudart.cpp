@@ -42,7 +42,7 @@ std::string text;
 CUstream_st legacy[2] = {{0, 1, false}, {1, 2, false}};
 unsigned long long next_id = 3;
 size_t fail_from = ~(size_t)0, fail_to = 0;
-int fail_times = 0;
+int fail_times = 0, fail_after = 0;
 thread_local int device = 0;
 thread_local cudaError_t last = cudaSuccess;
 struct Config {
@@ -71,7 +71,7 @@ bool capturing(int dev) {
 }
 cudaError_t allocate(void** p, size_t bytes, cudaMemPool_t pool, int dev) {
   *p = nullptr;
-  if (fail_times > 0 && bytes >= fail_from && bytes <= fail_to) {
+  if (fail_times > 0 && bytes >= fail_from && bytes <= fail_to && fail_after-- <= 0) {
     fail_times--;
     note("refuse %zu", bytes);
     return done(cudaErrorMemoryAllocation);
@@ -94,7 +94,9 @@ extern "C" {
 // What tests steer and read.
 const char* fake_log() { return text.c_str(); }
 void fake_clear() { text.clear(); }
-void fake_fail(size_t from, size_t to, int times) { fail_from = from, fail_to = to, fail_times = times; }
+void fake_fail(size_t from, size_t to, int times, int after) {  // allocations of `from` to `to` bytes
+  fail_from = from, fail_to = to, fail_times = times, fail_after = after;
+}
 size_t fake_live(int pooled) {
   std::lock_guard<std::recursive_mutex> hold(lock);
   size_t n = 0;

@@ -28,7 +28,7 @@ def library():
     L = C.CDLL(out)
     N._declare(L)
     L.fake_log.restype = C.c_char_p
-    L.fake_fail.argtypes = [C.c_size_t, C.c_size_t, C.c_int]
+    L.fake_fail.argtypes = [C.c_size_t, C.c_size_t, C.c_int, C.c_int]
     L.fake_fail.restype = L.fake_clear.restype = None
     L.fake_live.restype = C.c_size_t
     L.fake_id.argtypes = [C.c_void_p]
@@ -50,6 +50,11 @@ def clear():
 def calls(*words):
     """The log's lines that hold all of the words."""
     return [x for x in log() if all(w in x for w in words)]
+
+
+def fail(low, high, times=1, after=0):
+    """Refuses `times` allocations of low to high bytes, once `after` of them were made; fail(0, 0, 0): none."""
+    library().fake_fail(low, high, times, after)
 
 
 def stream():

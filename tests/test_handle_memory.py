@@ -18,7 +18,7 @@ def _fake():
     L = F.library()
     F.clear()
     yield
-    L.fake_fail(0, 0, 0)
+    F.fail(0, 0, 0)
     L.cudaSetDevice(0)
 
 
@@ -126,16 +126,16 @@ def test_what_a_graph_holds_stays():
 
 
 def test_allocation_after_the_pool_is_trimmed():
-    L.fake_fail(1, 1 << 40, 1)
+    F.fail(1, 1 << 40)
     b = F.create()
     text = F.log()
     refused = next(k for k, x in enumerate(text) if x.startswith("refuse"))
     assert text[refused + 1] == "trim device 0" and text[refused + 2].startswith("alloc")
-    L.fake_fail(1, 1 << 40, 100)
+    F.fail(1, 1 << 40, 100)
     h = C.c_void_p()
     pos = F.triangles(5)
     assert L.lucent_bvh_build_device(pos.ctypes.data, 5, None, C.byref(h), None) == 3  # out of memory
-    L.fake_fail(0, 0, 0)
+    F.fail(0, 0, 0)
     assert F.intersect(b, 10) == 0
     L.lucent_bvh_destroy(b.h)
     assert L.fake_live(1) == 0
