@@ -471,9 +471,11 @@ typedef struct lucent_batch_options {
   uint32_t samples_per_wave; /* samples of every pixel per wave; 0 = as many as max_wave_paths allows */
   uint32_t max_wave_paths;   /* path-state budget of one wave (about 430 bytes of device memory per path) */
   int32_t use_graph;         /* capture a full wave once as a CUDA graph and replay it */
-  uint32_t trace_blocks;     /* grid of the persistent traversal kernels; 0 = all resident blocks */
-  uint32_t shade_blocks;     /* grid of the shade kernels (blocks of 256 or 512 threads) and, in blocks
-                                of 128, of the sort and shadow kernels; 0 = all resident blocks */
+  uint32_t trace_blocks;     /* grid of the persistent closest-hit kernels in blocks of 256 threads; 0 = all
+                                resident blocks */
+  uint32_t shade_blocks;     /* grid of the shade kernels in blocks of 128 threads; the sort kernels take
+                                twice and the shadow kernels four times as many threads (no more than are
+                                resident); 0 = all resident blocks */
   int32_t sort_rays;         /* sort the rays of bounces 1 and 2 (see lucent_renderer_set_ray_sort) */
   int32_t top_levels;        /* top BVH levels of the first 8 scenes in shared memory (lucent_renderer_set_top_levels) */
   int32_t wide_bvh;          /* traversal of the four-wide BVH views (lucent_renderer_set_wide_bvh) */

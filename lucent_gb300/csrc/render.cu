@@ -447,6 +447,11 @@ static __device__ __forceinline__ float4 hit_values(const float4* __restrict__ g
 // 128 registers a thread, no spills in the forward kernel.
 constexpr int kShadeThreads = 512;  // at most
 static int shade_threads(uint32_t paths) { return paths >= (1u << 21) ? kShadeThreads : kShadeThreads / 2; }
+// MultiLaunch::shade_blocks counts 128 threads a block, whatever blocks the
+// kernel has: as many threads a block count as before they grew.
+static int shade_grid(const MultiLaunch& M, int threads, int resident) {
+  return M.shade_blocks > 0 ? std::max(1, (int)((int64_t)M.shade_blocks * 128 / threads)) : resident;
+}
 template <class Src, bool ADJ = false, bool TEX = false>
 __global__ void __launch_bounds__(kShadeThreads, 1) k_shade_t(Paths P, const __grid_constant__ Src src, int cur, int bounce,
                                                     const __grid_constant__ AdjointDev A = AdjointDev{}) {
@@ -1215,7 +1220,8 @@ static void launch_closest_multi(const MultiLaunch& M, const Paths& P, const Tra
   const TraversalGrids& G = traversal_grids();
   const int own = M.trace_blocks;
   if (M.near) {
-    const int g = own > 0 ? own : G.near;
+    // trace_blocks counts 256 threads a block, as the ordered kernels have.
+    const int g = own > 0 ? (int)std::min<int64_t>(G.near, (int64_t)own * 256 / PathClosestMulti::kNearThreads) : G.near;
     if (M.n == 1)
       launch_after(k_closest_near_t<PathClosestOne>, g, PathClosestOne::kNearThreads, 0, s, one_scene(M, A), PathClosestOne{pc});
     else
@@ -1238,10 +1244,13 @@ static void launch_closest_multi(const MultiLaunch& M, const Paths& P, const Tra
 static void launch_shadow_multi(const MultiLaunch& M, int blocks, const TravArgs& A, const PathShadowMulti& ps,
                                 cudaStream_t s) {
   const TraversalGrids& G = traversal_grids();
+  // shade_blocks sets this grid too: two blocks of 256 for each (`blocks` of the
+  // ordered kernels), so four of 128, no more than run at once (they are persistent).
+  const int own = M.shade_blocks > 0 ? (int)std::min<int64_t>(G.any, (int64_t)M.shade_blocks * 4) : G.any;
   if (M.near && M.n == 1)
-    k_anyhit_near_t<PathShadowOne><<<G.any, kAnyThreads, 0, s>>>(one_scene(M, A), PathShadowOne{ps});
+    k_anyhit_near_t<PathShadowOne><<<own, kAnyThreads, 0, s>>>(one_scene(M, A), PathShadowOne{ps});
   else if (M.near)
-    k_anyhit_near_t<PathShadowMulti><<<G.any, kAnyThreads, 0, s>>>(A, ps);
+    k_anyhit_near_t<PathShadowMulti><<<own, kAnyThreads, 0, s>>>(A, ps);
   else if (M.wide)
     k_anyhit_wide_t<PathShadowMulti><<<blocks, 256, 0, s>>>(A, ps);
   else
@@ -1261,7 +1270,7 @@ int render_wave_multi(const MultiLaunch& M, cudaStream_t s, PhaseEvents* pe, boo
   static const int max_shade[2] = {persistent_blocks((const void*)k_shade_t<SceneTable>, kShadeThreads / 2),
                                    persistent_blocks((const void*)k_shade_t<SceneTable>, kShadeThreads)};
   const int shade_t = shade_threads(M.total_paths);
-  const int shade_blocks = M.shade_blocks > 0 ? M.shade_blocks : max_shade[shade_t == kShadeThreads];
+  const int shade_blocks = shade_grid(M, shade_t, max_shade[shade_t == kShadeThreads]);
   const int aux = M.shade_blocks > 0 ? M.shade_blocks : aux_blocks();
   const int top = M.top_levels ? (M.n < kTopMaxScenes ? M.n : kTopMaxScenes) : 0;
   bool sorted = false;  // the rays of this bounce are in the sorted stream

@@ -382,8 +382,9 @@ class Batch:
     each renderer alone would give. Options (lucent_batch_options):
     samples_per_wave (0 = as many as max_wave_paths allows), max_wave_paths,
     use_graph (replay a captured wave), trace_blocks / shade_blocks (grid
-    sizes, 0 = all resident blocks), sort_rays, top_levels, wide_bvh (as
-    the renderer's set_ray_sort / set_top_levels / set_wide_bvh),
+    sizes in blocks of 256 / 128 threads, 0 = all resident blocks),
+    sort_rays, top_levels, wide_bvh (as the renderer's set_ray_sort /
+    set_top_levels / set_wide_bvh),
     scenes_per_wave (waves hold groups of this many consecutive scenes,
     each traced for all samples before the next; 0 = all scenes), streams
     (the renderers in that many parts, traced side by side on their own
@@ -430,8 +431,8 @@ class Batch:
         return "n%d_px%d_tri%d_b%d" % (len(self.renderers), px, tris, mb)
 
     # Second tuning stage: one option at a time from the best wave configuration
-    # (ray sorting, the shared-memory top BVH levels, the grid of the shade /
-    # resolve / any-hit kernels); none of them changes an image.
+    # (ray sorting, the shared-memory top BVH levels, the grid of the shade,
+    # sort and any-hit kernels); none of them changes an image.
     REFINE = ({"sort_rays": False}, {"top_levels": False}, {"shade_blocks": 152 * 3}, {"shade_blocks": 152 * 8},
               {"streams": 2})
 
