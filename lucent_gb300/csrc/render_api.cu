@@ -1123,20 +1123,29 @@ lucent_status lucent_renderer_backward(lucent_renderer* r, uint32_t samples, uin
   cudaStream_t s = (cudaStream_t)stream;
   const uint32_t WH = r->W * r->H;
   const uint32_t max_paths = 1u << 23;
-  const uint32_t batch = std::max(1u, std::min(samples, max_paths / std::max(1u, WH)));
+  uint32_t batch = std::max(1u, std::min(samples, max_paths / std::max(1u, WH)));
   WaveSet& X = r->set[0];
   lucent_status st = X.reserve(batch * WH);
   if (st) return st;
-  const size_t cap = X.path_cap;
   const size_t nmat = scene_owner(r)->material_count;
   const size_t texels = d_env ? (size_t)r->light.env_w * r->light.env_h : 0;
   const size_t env_off = nmat * 8;  // 6 of 8 floats per material, then RGB and a pad per texel
   const size_t nenv = texels * 4;
-  // per path: the remaining radiance, and 4 + 4 + 1 bytes for each bounce
-  const size_t vertices = cap * (r->max_bounces + 1);
-  if ((st = r->adj_dl.reserve((size_t)WH * 16)) || (st = r->adj_path.reserve(cap * 16 + vertices * 9 + (r->max_bounces + 1) * 4)) ||
-      (st = r->adj_grad.reserve((env_off + nenv) * 4 + 16)))
-    return st;
+  if ((st = r->adj_dl.reserve((size_t)WH * 16)) || (st = r->adj_grad.reserve((env_off + nenv) * 4 + 16))) return st;
+  // per path: the remaining radiance, and 4 + 4 + 1 bytes for each bounce. With
+  // many bounces that is more than a wave's path state (601 bytes at 64), so
+  // where it does not fit, waves of fewer samples.
+  size_t cap, vertices;
+  while (true) {
+    cap = (size_t)batch * WH;
+    vertices = cap * (r->max_bounces + 1);
+    st = r->adj_path.reserve(cap * 16 + vertices * 9 + (r->max_bounces + 1) * 4);
+    if (!st) break;
+    if (st != LUCENT_ERR_OOM || batch == 1) return st;
+    cudaGetLastError();
+    clear_error();
+    batch = (batch + 1) / 2;
+  }
   std::vector<float> dl((size_t)WH * 4);
   const float inv = 1.f / (float)samples;
   for (size_t i = 0; i < dl.size(); i++) {
