@@ -79,6 +79,11 @@ lucent_status lucent_bvh_download(const lucent_bvh* bvh, float* nodes_out, uint3
 lucent_status lucent_bvh_create(const float* nodes, uint32_t node_count, const uint32_t* tri_indices,
                                 uint32_t tri_count, const float* positions, lucent_bvh** out);
 void lucent_bvh_destroy(lucent_bvh* bvh);
+/* Gives back the device memory that builds and closed handles leave for the
+ * next ones (at most 1 GiB a device, the current one's), after waiting for the
+ * device. The library does so itself where an allocation of its own fails; for
+ * programs whose other allocations need the room. */
+lucent_status lucent_trim(void);
 /* Node and triangle counts of an uploaded BVH. */
 lucent_status lucent_bvh_info(const lucent_bvh* bvh, uint32_t* node_count, uint32_t* tri_count);
 /* Traversal mode: 0 = f32 bounded-error path with binary64 fallback and the
@@ -422,7 +427,8 @@ lucent_status lucent_renderer_backward(lucent_renderer* r, uint32_t samples, uin
 /* Frees the path-state buffers (about 315 bytes per path of the largest
  * wave traced so far); the next trace allocates them again. For hosts that
  * keep many renderers alive but trace one at a time. No reference
- * counterpart (WebGL owns the reference's render targets). */
+ * counterpart (WebGL owns the reference's render targets). Includes
+ * lucent_trim. */
 lucent_status lucent_renderer_trim(lucent_renderer* r);
 
 /* runDenoiser (renderer.ts:788-830; variance.frag, atrous.frag,

@@ -53,6 +53,7 @@ def _declare(L):
     _sig(L, "lucent_bvh_download", [VP, F32P, U32P])
     _sig(L, "lucent_bvh_create", [F32P, C.c_uint32, U32P, C.c_uint32, F32P, P(VP)])
     _sig(L, "lucent_bvh_destroy", [VP], None)
+    _sig(L, "lucent_trim", [])
     _sig(L, "lucent_bvh_info", [VP, U32P, U32P])
     _sig(L, "lucent_bvh_set_mode", [VP, C.c_int32])
     _sig(L, "lucent_bvh_intersect", [VP, F32P, C.c_uint32, C.c_double, C.c_double, I32P, F32P, F32P, F32P, VP])

@@ -185,6 +185,11 @@ def build_device(positions_ptr, tri_count, max_leaf_size=4, bins=12, stream=None
     return _wrap_handle(h, nc.value, tc.value)
 
 
+def trim():
+    """Gives back the device memory that builds and closed trees leave for the next ones (lucent_trim)."""
+    N.check(N.lib().lucent_trim())
+
+
 def download(dev: DeviceBVH):
     """Reference-layout (nodes, triIndices) of a device BVH."""
     nodes = np.zeros(dev.node_count * NODE_STRIDE, np.float32)

@@ -49,6 +49,26 @@ def test_closed_in_flight():
         assert torch.equal(prim, want[k][0]) and torch.equal(t, want[k][1])
 
 
+def test_trim_returns_what_builds_leave():
+    pos, r = _soup(9, 500_000, 1_000)
+    kept = B.build_device(pos.data_ptr(), len(pos))
+    want = _query(kept, r, torch.cuda.current_stream())[0]
+    B.trim()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        B.build_device(pos.data_ptr(), len(pos)).close()
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    B.trim()
+    after = torch.cuda.mem_get_info()[0]
+    assert held < before - (64 << 20)  # 168 bytes a triangle of scratch and more of the tree
+    assert after >= before - (8 << 20)
+    assert torch.equal(_query(kept, r, torch.cuda.current_stream())[0], want)
+    kept.check()
+    B.build_device(pos.data_ptr(), len(pos)).close()
+
+
 def test_threads():
     bad = []
 

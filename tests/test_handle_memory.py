@@ -125,6 +125,21 @@ def test_what_a_graph_holds_stays():
     assert text.index("sync device 0") < [k for k, x in enumerate(text) if x.startswith("give back")][2]
 
 
+def test_trimmed_without_a_renderer():
+    b, s, other = F.create(), F.stream(), F.stream()
+    assert F.intersect(b, 10, s) == 0
+    F.begin_capture(s)
+    assert F.intersect(b, 10, s) == 0
+    F.end_capture(s)
+    F.begin_capture(other)
+    L.lucent_bvh_destroy(b.h)
+    assert L.lucent_trim() != 0  # a capture is under way: nothing can be waited for
+    F.end_capture(other)
+    F.clear()
+    assert L.lucent_trim() == 0
+    assert L.fake_live(1) == 0 and F.log()[0] == "sync device 0" and F.log()[-1] == "trim device 0"
+
+
 def test_allocation_after_the_pool_is_trimmed():
     F.fail(1, 1 << 40)
     b = F.create()
