@@ -101,6 +101,12 @@ lucent_status lucent_bvh_info(const lucent_bvh* bvh, uint32_t* node_count, uint3
 #define LUCENT_TRAVERSE_WIDE 3
 lucent_status lucent_bvh_set_mode(lucent_bvh* bvh, int32_t mode);
 
+/* What the last call in mode 3 did, once it is over: whether the tree is
+ * traversed nearest first (0 also before the first call), how far from the
+ * tree's centre ray origins may lie for that, and how many of the call's rays
+ * were handed on to the ordered kernels. Any may be NULL. */
+lucent_status lucent_bvh_near_info(lucent_bvh* bvh, int32_t* usable, float* reach, uint32_t* handed_on);
+
 /* n rays, 6 floats each (origin xyz, direction xyz), host buffers. t_min and
  * t_max as in intersectBVH(bvh, positions, ray, tMin = 1e-5, tMax = Infinity).
  * prim_out[i] = source triangle index or -1 on a miss; t_out is +inf on a miss.

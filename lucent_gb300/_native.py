@@ -56,6 +56,7 @@ def _declare(L):
     _sig(L, "lucent_trim", [])
     _sig(L, "lucent_bvh_info", [VP, U32P, U32P])
     _sig(L, "lucent_bvh_set_mode", [VP, C.c_int32])
+    _sig(L, "lucent_bvh_near_info", [VP, I32P, F32P, U32P])
     _sig(L, "lucent_bvh_intersect", [VP, F32P, C.c_uint32, C.c_double, C.c_double, I32P, F32P, F32P, F32P, VP])
     _sig(L, "lucent_bvh_intersect_device", [VP, VP, C.c_uint32, C.c_double, C.c_double, VP, VP, VP, VP, VP])
     _sig(L, "lucent_bvh_check", [VP, VP])

@@ -77,6 +77,13 @@ class DeviceBVH:
         mode = 1 if exact else 3 if wide else 0 if top_levels else 2
         N.check(N.lib().lucent_bvh_set_mode(self._h, mode))
 
+    def near_info(self):
+        """Of the last call in the default mode, once it is over: whether the tree is traversed nearest first, from how
+        far off rays may come for that, how many were handed on to the ordered kernels (lucent_bvh_near_info)."""
+        usable, reach, handed = C.c_int32(), C.c_float(), C.c_uint32()
+        N.check(N.lib().lucent_bvh_near_info(self._h, C.byref(usable), C.byref(reach), C.byref(handed)))
+        return bool(usable.value), float(reach.value), int(handed.value)
+
     def intersect(self, rays, t_min=1e-5, t_max=math.inf, stream=None):
         """Closest hits of float32 rays [n, 6] -> (prim int32 (-1 miss), t, u, v) float32."""
         r = np.ascontiguousarray(rays, np.float32).reshape(-1, 6)

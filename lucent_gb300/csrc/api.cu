@@ -502,6 +502,22 @@ lucent_status lucent_bvh_set_mode(lucent_bvh* b, int32_t mode) {
   return LUCENT_OK;
 }
 
+lucent_status lucent_bvh_near_info(lucent_bvh* b, int32_t* usable, float* reach, uint32_t* handed_on) {
+  clear_error();
+  if (!b) return fail(LUCENT_ERR_INVALID, "null bvh");
+  const bool near = b->views && b->near.usable;
+  if (usable) *usable = near;
+  if (reach) *reach = near ? b->near.bound.w : 0.f;
+  if (handed_on) {
+    *handed_on = 0;
+    if (near && b->scratch.ptr) {  // the queue's length, the second counter word (launch_closest)
+      cudaError_t e = cudaMemcpy(handed_on, (uint32_t*)b->scratch.ptr + 1, 4, cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) return cuda_fail(e, "read counters");
+    }
+  }
+  return LUCENT_OK;
+}
+
 static lucent_status check_tmin(double t_min, double t_max) {
   if (!(t_min >= 0) || std::isnan(t_max)) return fail(LUCENT_ERR_INVALID, "t_min must be >= 0 and t_max not NaN");
   return LUCENT_OK;
