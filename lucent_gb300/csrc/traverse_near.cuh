@@ -44,12 +44,13 @@
 // bound for |d| <= 2 and origins within two diagonals of the tree's centre; for
 // farther ones it rises linearly with the distance, and the ray's boxes are
 // grown by the largest such rise of any triangle (NearTree::far), as long as
-// that is small against a leaf. Other rays go to the ordered kernel. A tree
+// that is small against a leaf. Other rays go to the ordered kernel, but for
+// those that pass the root's boxes by. A tree
 // with many leaves whose growth is not small against the scene (scenes in units
 // far above 1, where 1e-12 is no bound at all), with boxes that are not nested
-// or do not hold their triangles or slots out of visiting order
-// (caller-supplied trees), or with leaves of over 255 triangles is not
-// traversed this way (NearTree::usable).
+// or do not hold their triangles, nodes that the root never reaches or slots
+// out of visiting order (caller-supplied trees), or with leaves of over 255
+// triangles is not traversed this way (NearTree::usable).
 //
 // A record: (min.xyz, reference), (max.xyz, unused); the reference is the
 // binary index of an inner node or kNearLeaf | first slot << 8 | count. As in
@@ -245,12 +246,14 @@ static __device__ __noinline__ bool near_misses_all(float3 o, float3 d, const No
 // nearest. With few rays for the grid, a warp takes only as many as spread
 // them over all warps: fewer lanes in a warp diverge less, and a launch of few
 // rays lasts as long as its slowest warp.
-// Bound by divergence, instruction issue and node latency (ncu, bounce 1: some
-// 10 of 32 lanes active, issue slots 55 to 65 % busy, L1 45 to 52 %, DRAM 10 %).
-// Against the ordered wide kernel: 4,099 rays into 20,480 triangles 284 -> 89
-// us a call, 10^6 rays into the 65,536-triangle soup 3.48 -> 1.82 ms, closest
-// hit of the box frame (11.8 M rays, 82 k triangles) 4.19 -> 2.40 ms, of a
-// 1080p 4-spp frame over 2 M triangles (14.7 M rays) 25.5 -> 9.4 ms.
+// Bound by instruction issue on coherent waves (ncu, box frame, bounce 1: 18.0
+// of 32 lanes active, issue slots 70 % busy, L1 64 %, DRAM 4 %), by L1 and
+// divergence on incoherent rays (the soup: 13.0 lanes, L1 90 %, DRAM 0.4 %),
+// by the longest ray's chain in small launches.
+// Against the ordered wide kernel: 4,099 rays into 20,480 triangles 276 -> 69
+// us a call, 10^6 rays into the 65,536-triangle soup 3.47 -> 1.80 ms, closest
+// hit of the box frame (11.8 M rays, 82 k triangles) 4.19 -> 2.35 ms, of a
+// 1080p 4-spp frame over 2 M triangles (14.7 M rays) 25.5 -> 9.0 ms.
 template <class Pol>
 __global__ void __launch_bounds__(Pol::kNearThreads, Pol::kNearBlocks) k_closest_near_t(TravArgs A, const __grid_constant__ Pol P) {
   wait_for_previous();
