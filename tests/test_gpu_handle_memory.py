@@ -49,6 +49,31 @@ def test_closed_in_flight():
         assert torch.equal(prim, want[k][0]) and torch.equal(t, want[k][1])
 
 
+def test_replayed_after_the_scratch_grew():
+    pos, r = _soup(7, 30_000, 300_000)
+    dev = B.build_device(pos.data_ptr(), len(pos))
+    few = r[:5_000].clone()
+    want = _query(dev, few, torch.cuda.current_stream())
+    dev.check()
+    s = torch.cuda.Stream()
+    o = [torch.zeros_like(x) for x in want]
+    s.wait_stream(torch.cuda.current_stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        dev.intersect_device(few.data_ptr(), len(few), *(x.data_ptr() for x in o), stream=s.cuda_stream)
+    _query(dev, r, torch.cuda.current_stream())  # needs more scratch than the graph's call
+    dev.check()
+    other = B.build_device(pos.data_ptr(), len(pos))  # what was given back is taken again
+    for x in o:
+        x.fill_(-9)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(o[0], want[0]) and torch.equal(o[1], want[1])
+    other.close()
+    dev.close()
+    B.trim()
+
+
 def test_trim_returns_what_builds_leave():
     pos, r = _soup(9, 500_000, 1_000)
     kept = B.build_device(pos.data_ptr(), len(pos))
