@@ -186,20 +186,22 @@ void StreamUses::close() {
   home->give_waiting_back();
 }
 
-void trim_temporaries() {
-  if (Pool* P = device_pool()) {
-    P->give_waiting_back();
-    cudaMemPoolTrimTo(P->pool, 0);
-  }
+static void trim_pool(Pool& P) {
+  P.give_waiting_back();
+  cudaMemPoolTrimTo(P.pool, 0);
 }
 
-static lucent_status pool_alloc(void** ptr, size_t bytes, const Pool* P, cudaStream_t s) {
+void trim_temporaries() {
+  if (Pool* P = device_pool()) trim_pool(*P);
+}
+
+static lucent_status pool_alloc(void** ptr, size_t bytes, Pool* P, cudaStream_t s) {
   *ptr = nullptr;
   if (!P) return cuda_fail(cudaGetLastError(), "memory pool");
   cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, P->pool, s);
   if (e == cudaErrorMemoryAllocation) {  // once more without what the pool holds
     cudaGetLastError();
-    trim_temporaries();
+    trim_pool(*P);
     e = cudaMallocFromPoolAsync(ptr, bytes, P->pool, s);
   }
   if (e == cudaSuccess) return LUCENT_OK;
@@ -224,7 +226,7 @@ lucent_status DeviceBuffer::reserve(size_t bytes) {
   const size_t want = bytes < 256 ? 256 : bytes;
   if (uses) {  // allocated on the pool's stream and waited for: usable on any stream
     if (!uses->home) uses->home = device_pool();
-    const Pool* P = uses->home;
+    Pool* const P = uses->home;
     if (lucent_status st = pool_alloc(&ptr, want, P, P ? P->stream : nullptr)) return st;
     if (cudaError_t e = cudaStreamSynchronize(P->stream); e != cudaSuccess) {
       cudaFreeAsync(ptr, P->stream);

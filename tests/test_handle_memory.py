@@ -52,6 +52,17 @@ def test_closed_while_another_device_is_current():
     assert L.cudaGetLastError() == 0
 
 
+def test_grown_while_another_device_is_current():
+    b = _on_device(1)
+    L.lucent_bvh_set_mode(b.h, 0)  # no views: scratch alone
+    F.clear()
+    F.fail(1, 1 << 40)  # the first attempt: its own device's pool is trimmed for the second
+    F.intersect(b, 1_000)
+    assert F.calls("trim device 1") and F.calls("alloc", "device 1 pool") and not F.calls("device 0")
+    L.lucent_bvh_destroy(b.h)
+    assert L.fake_live(1) == 0
+
+
 def test_closed_on_another_thread():
     b = _on_device(1)
     F.clear()
